@@ -315,59 +315,112 @@ __global__ void k_mix_iprep(DevCtl *ctl, SimSegs seg, const float4 *__restrict__
     }
 }
 
-/* One j of a near-pair pass for i-body p (raw i: hi_i, lo_i; re-centred
- * i: xi..zi; threshold thk): adds the FP32 term to (tx, ty, tz), or, for a
- * near pair, the term from the exact hi/lo difference, or, for a possible
- * overlap, the FP64 term folded into the (hi, lo) sums with the event
- * recorded.  xj..m are j's re-centred position and mass from the tile;
- * hj, lj its raw hi/lo (read only for a near pair, through get_raw). */
-template <typename RAW>
-__device__ __forceinline__ void near_pass_j(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
-                                            const unsigned *__restrict__ perm, double inv_ms, ll i, ll q,
-                                            const float4 &hi_i, const float4 &lo_i, float xi, float yi, float zi,
-                                            float thk, float xj, float yj, float zj, float m, RAW get_raw, float &tx,
-                                            float &ty, float &tz, float &fhx, float &flx, float &fhy, float &fly,
-                                            float &fhz, float &flz)
+/* squared distance that stands for a pair taken out of a packed sum: the term
+ * m r^-3 d underflows to zero */
+#define FAR_R2 1.0e36f
+
+/* A tile's contribution to one body as unevaluated (hi, lo) sums. */
+struct TileSum {
+    float hx, lx, hy, ly, hz, lz;
+};
+
+/* A near pair (sorted positions p, q): the term from the exact hi/lo
+ * difference added to the (hi, lo) sums, or, for a possible overlap, the FP64
+ * term folded in with the event recorded. */
+__device__ __forceinline__ void near_pair(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
+                                          const unsigned *__restrict__ perm, ll p, ll q, const float4 &hi_i,
+                                          const float4 &lo_i, const float4 &hj, const float4 &lj, TileSum &t)
 {
-    float dx = xj - xi, dy = yj - yi, dz = zj - zi;
-    float r2 = dx * dx + dy * dy + dz * dz;
-    if (r2 < thk) {
-        /* near pair: difference of the hi/lo positions (error ~2^-24 |dx|) */
-        float4 hj, lj;
-        get_raw(q, hj, lj);
-        dx = (hj.x - hi_i.x) + (lj.x - lo_i.x);
-        dy = (hj.y - hi_i.y) + (lj.y - lo_i.y);
-        dz = (hj.z - hi_i.z) + (lj.z - lo_i.z);
-        r2 = dx * dx + dy * dy + dz * dz;
-        const float rs = lo_i.w + lj.w;
-        /* an overlap, or a pair within 2^-10 of the overlap distance, is
-         * decided in FP64 */
-        if (!(r2 > rs * rs * (1.0f + 0x1p-10f) && rs >= 0.f) || (lo_i.w < 0.f) || (lj.w < 0.f)) {
-            double qx, qy, qz;
-            candidate_pair(A, ctl, ev_keys, ev_cap, i, (ll)perm[q], inv_ms, qx, qy, qz);
-            fold64(fhx, flx, qx);
-            fold64(fhy, fly, qy);
-            fold64(fhz, flz, qz);
-            return;
-        }
-        /* A near pair can carry most of the body's force, so its term is
-         * made as exact as FP32 allows: one Newton step on the SFU's
-         * reciprocal square root (relative error 2^-22.9 -> ~2^-24), and
-         * the term goes straight into the (hi, lo) sums rather than through
-         * the tile's FP32 sum, whose roundings would be ulps of this term */
-        float inv = rsqrt_sfu(r2);
-        inv = inv * (1.5f - 0.5f * r2 * inv * inv);
-        const float s = m * inv * inv * inv;
-        two_sum_add(fhx, flx, s * dx);
-        two_sum_add(fhy, fly, s * dy);
-        two_sum_add(fhz, flz, s * dz);
+    /* difference of the hi/lo positions (error ~2^-24 |dx|) */
+    const float dx = (hj.x - hi_i.x) + (lj.x - lo_i.x);
+    const float dy = (hj.y - hi_i.y) + (lj.y - lo_i.y);
+    const float dz = (hj.z - hi_i.z) + (lj.z - lo_i.z);
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float rs = lo_i.w + lj.w;
+    /* an overlap, or a pair within 2^-10 of the overlap distance, is decided
+     * in FP64 */
+    if (!(r2 > rs * rs * (1.0f + 0x1p-10f) && rs >= 0.f) || (lo_i.w < 0.f) || (lj.w < 0.f)) {
+        double ms = ctl->m_scale;
+        if (!(ms > 0.0)) ms = 1.0;
+        double qx, qy, qz;
+        candidate_pair(A, ctl, ev_keys, ev_cap, (ll)perm[p], (ll)perm[q], 1.0 / ms, qx, qy, qz);
+        fold64(t.hx, t.lx, qx);
+        fold64(t.hy, t.ly, qy);
+        fold64(t.hz, t.lz, qz);
         return;
     }
-    const float inv = rsqrt_sfu(r2);
-    const float s = m * inv * inv * inv;
-    tx += s * dx;
-    ty += s * dy;
-    tz += s * dz;
+    /* A near pair can carry most of the body's force, so its term is made as
+     * exact as FP32 allows: one Newton step on the SFU's reciprocal square
+     * root (relative error 2^-22.9 -> ~2^-24), and the term goes straight
+     * into the (hi, lo) sums rather than through the tile's FP32 sum, whose
+     * roundings would be ulps of this term */
+    float inv = rsqrt_sfu(r2);
+    inv = inv * (1.5f - 0.5f * r2 * inv * inv);
+    const float s = hj.w * inv * inv * inv;
+    two_sum_add(t.hx, t.lx, s * dx);
+    two_sum_add(t.hy, t.ly, s * dy);
+    two_sum_add(t.hz, t.lz, s * dz);
+}
+
+/* The careful pass over one j tile (jpv j pairs in sA, sB from position jt)
+ * for body p, which met a near pair in it (its own body, in its own tile):
+ * the fast pass again, four j at a time, with each near pair taken out of
+ * the packed sum (moved so far away that its term is zero) and added exactly
+ * instead.  Bound by instruction issue, as the fast pass is: 25 instructions
+ * per j pair where a scalar walk spent 56.  Out of line because the tile
+ * loop's registers decide the kernel's speed: with the pass inlined, the
+ * 96-register shape spilled 120 bytes and ran 7.11 ms on the 131,072-body
+ * Plummer + disk, out of line 6.50 ms (the scalar walk inlined: 6.70 ms).
+ * Sharing the flagged bodies' tiles among the warp's lanes measured slower
+ * wherever most lanes are flagged (1.10 against 1.00 ms at 50,001 bodies). */
+__device__ __noinline__ TileSum careful_tile(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
+                                             const unsigned *__restrict__ perm, const float4 *__restrict__ jhi,
+                                             const float4 *__restrict__ jlo, const float4 *sA, const float4 *sB,
+                                             int jpv, ll jt, ll p, float nx, float ny, float nz, float thk)
+{
+    TileSum mine = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const float4 hi_i = jhi[p], lo_i = jlo[p];
+    float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+#pragma unroll 1
+    for (int pp = 0; pp < jpv; pp += 2) {
+        float2 dx[2], dy[2], dz[2], r2[2], mj[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const float4 a = sA[pp + u], b = sB[pp + u];
+            dx[u] = __fadd2_rn(make_float2(a.x, a.y), make_float2(nx, nx));
+            dy[u] = __fadd2_rn(make_float2(a.z, a.w), make_float2(ny, ny));
+            dz[u] = __fadd2_rn(make_float2(b.x, b.y), make_float2(nz, nz));
+            mj[u] = make_float2(b.z, b.w);
+            r2[u] = __fmul2_rn(dx[u], dx[u]);
+            r2[u] = __ffma2_rn(dy[u], dy[u], r2[u]);
+            r2[u] = __ffma2_rn(dz[u], dz[u], r2[u]);
+        }
+        unsigned hit = (r2[0].x < thk ? 1u : 0u) | (r2[0].y < thk ? 2u : 0u) | (r2[1].x < thk ? 4u : 0u) |
+                       (r2[1].y < thk ? 8u : 0u);
+        if (hit) {
+            if (hit & 1u) r2[0].x = FAR_R2;
+            if (hit & 2u) r2[0].y = FAR_R2;
+            if (hit & 4u) r2[1].x = FAR_R2;
+            if (hit & 8u) r2[1].y = FAR_R2;
+            do {
+                const ll q = jt + 2 * pp + __ffs(hit) - 1;
+                hit &= hit - 1u;
+                if (q != p) near_pair(A, ctl, ev_keys, ev_cap, perm, p, q, hi_i, lo_i, jhi[q], jlo[q], mine);
+            } while (hit);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const float2 inv = make_float2(rsqrt_sfu(r2[u].x), rsqrt_sfu(r2[u].y));
+            const float2 s = __fmul2_rn(__fmul2_rn(mj[u], inv), __fmul2_rn(inv, inv));
+            ax = __ffma2_rn(s, dx[u], ax);
+            ay = __ffma2_rn(s, dy[u], ay);
+            az = __ffma2_rn(s, dz[u], az);
+        }
+    }
+    two_sum_add(mine.hx, mine.lx, ax.x + ax.y);
+    two_sum_add(mine.hy, mine.ly, ay.x + ay.y);
+    two_sum_add(mine.hz, mine.lz, az.x + az.y);
+    return mine;
 }
 
 /* ---- bulk copies into shared memory ----------------------------------------
@@ -426,7 +479,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(ull *bar, unsigned parity)
  * event keys. */
 template <int BLOCK, int K, int JT, int UNROLL, int MINB, bool SF, bool DB, bool BULK>
 __global__ void __launch_bounds__(BLOCK, MINB)
-k_pair_mixed(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi, const float4 *__restrict__ jlo,
+k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi, const float4 *__restrict__ jlo,
              const float4 *__restrict__ tile_c, const float4 *__restrict__ iprep, const unsigned *__restrict__ perm,
              double *__restrict__ part, ull *ev_keys, ll ev_cap)
 {
@@ -457,12 +510,6 @@ k_pair_mixed(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ 
     if (ctl->error) return;
     const int C = ctl->splits;
     const ll W = ctl->work_total;
-    double ms = ctl->m_scale;
-    if (!(ms > 0.0)) ms = 1.0;
-    const double inv_ms = 1.0 / ms;
-    const float rmax = __uint_as_float(ctl->rmax_bits);
-    const float xmax = __uint_as_float(ctl->xmax_bits);
-    const double kappa = (double)ctl->near_kappa;
     const int tid = threadIdx.x;
     /* BULK: bit b of ph is the parity of mbar[b]'s next phase, bit b of pend
      * says a copy into raw buffer b is in flight (both the same in every
@@ -677,46 +724,38 @@ k_pair_mixed(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ 
                     az[k] = __ffma2_rn(s, dz, az[k]);
                 }
             };
-            /* a full tile keeps a constant trip count for the unroller */
+            /* a full tile keeps a constant trip count for the unroller; a short
+             * one runs on to a multiple of four pairs (the rest of the tile
+             * holds sentinels, whose terms are zero) */
             if (jpv == JP) {
 #pragma unroll UNROLL
                 for (int pp = 0; pp < JP; pp++) pair_step(pp);
             } else {
-                for (int pp = 0; pp < jpv; pp++) pair_step(pp);
+#pragma unroll 1
+                for (int pp = 0; pp < jpv; pp += 4) {
+                    pair_step(pp);
+                    pair_step(pp + 1);
+                    pair_step(pp + 2);
+                    pair_step(pp + 3);
+                }
             }
 #pragma unroll
             for (int k = 0; k < K; k++) {
                 const float thk = THR(k);
+                float tx = ax[k].x + ax[k].y, ty = ay[k].x + ay[k].y, tz = az[k].x + az[k].y;
                 if (mn[k] < thk) {
-                    /* slow path: this tile holds a near or overlapping pair for i */
-                    const ll p = ibase + (ll)k * BLOCK + tid;
-                    const ll i = perm[p];
-                    const float4 hi_i = jhi[p], lo_i = jlo[p];
-                    float tx = 0.f, ty = 0.f, tz = 0.f;
-                    const float xi = -nx[k].x, yi = -ny[k].x, zi = -nz[k].x;
-                    for (int pp = 0; pp < jpv; pp++) {
-                        const float4 a = sA[pp], b = sB[pp];
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const ll q = jt + 2 * pp + e;
-                            if (q >= je || q == p) continue;
-                            near_pass_j(A, ctl, ev_keys, ev_cap, perm, inv_ms, i, q, hi_i, lo_i, xi, yi, zi, thk,
-                                        e ? a.y : a.x, e ? a.w : a.z, e ? b.y : b.x, e ? b.w : b.z,
-                                        [&](ll qq, float4 &hj, float4 &lj) {
-                                            hj = jhi[qq];
-                                            lj = jlo[qq];
-                                        },
-                                        tx, ty, tz, FOLD(0, k), FOLD(1, k), FOLD(2, k), FOLD(3, k), FOLD(4, k),
-                                        FOLD(5, k));
-                        }
-                    }
-                    ax[k] = make_float2(tx, 0.f);
-                    ay[k] = make_float2(ty, 0.f);
-                    az[k] = make_float2(tz, 0.f);
+                    const TileSum t = careful_tile(A, ctl, ev_keys, ev_cap, perm, jhi, jlo, sA, sB, jpv, jt,
+                                                   ibase + (ll)k * BLOCK + tid, nx[k].x, ny[k].x, nz[k].x, thk);
+                    tx = t.hx;
+                    ty = t.hy;
+                    tz = t.hz;
+                    FOLD(1, k) += t.lx;
+                    FOLD(3, k) += t.ly;
+                    FOLD(5, k) += t.lz;
                 }
-                two_sum_add(FOLD(0, k), FOLD(1, k), ax[k].x + ax[k].y);
-                two_sum_add(FOLD(2, k), FOLD(3, k), ay[k].x + ay[k].y);
-                two_sum_add(FOLD(4, k), FOLD(5, k), az[k].x + az[k].y);
+                two_sum_add(FOLD(0, k), FOLD(1, k), tx);
+                two_sum_add(FOLD(2, k), FOLD(3, k), ty);
+                two_sum_add(FOLD(4, k), FOLD(5, k), tz);
             }
             if (BULK) {
                 /* tile buffer buf ^ 1 was last read by the previous tile,
