@@ -100,7 +100,7 @@ def parse():
     ap.add_argument("--p64-split-max", type=int, default=None,
                     help="plain FP64: largest capacity for the split pair pass (library default 65536)")
     ap.add_argument("--sort-interval", type=int, default=None,
-                    help="mixed: cycles between Morton sorts of the i-tiles (library default 4)")
+                    help="mixed: cycles between spatial sorts of the i-tiles (library default 4)")
     ap.add_argument("--drift-cycles", type=int, default=0,
                     help="after the timed run, step a fresh copy of the workload this many cycles and report the "
                          "relative energy and momentum drift (untimed)")

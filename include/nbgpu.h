@@ -240,7 +240,7 @@ int nbg_get_body_in(nbg_ctx *ctx, int64_t sim, int64_t id, nbg_soa *host, int32_
  * body.go:49-52,152-155), the NextId counter (body.go:316-329), the cycle
  * index that keys the fragment generator, its seed, the host adds staged
  * for the next Cycle, the collections' sizes, the precision form, kernel
- * shape and options, and in the mixed form the bodies' current Morton order.
+ * shape and options, and in the mixed form the bodies' current Hilbert order.
  *
  * nbg_save_state: *size receives the snapshot's bytes; with buf NULL that is
  * all it does (a size query).  A cap below the size returns NBG_E_OVERFLOW.
@@ -380,7 +380,7 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
 #define NBG_OPT_BARNES_HUT 8
 /* mixed Barnes-Hut walk: registers capped for 3, 4 or 5 CTAs per SM (0..2) */
 #define NBG_OPT_BH_SHAPE 9
-/* mixed: cycles between Morton sorts of the i-tiles (1..1000, default 4).
+/* mixed: cycles between sorts of the i-tiles (1..1000, default 4).
    Bodies move far less than a tile per cycle, so an older order still gives
    compact tiles.  Compaction carries the order along (kept bodies keep their
    places, arrivals follow); loads and host edits sort again at the next

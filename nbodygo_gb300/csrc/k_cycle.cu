@@ -1204,7 +1204,7 @@ __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_compact(BodyArrays A, BodyAr
     }
 }
 
-/* The mixed path's Morton order carried through compaction: the kept bodies
+/* The mixed path's Hilbert order carried through compaction: the kept bodies
  * keep their sorted sequence under their new indices, and each sim's arrivals
  * (fragments, host adds) follow its kept bodies.  A sim's sorted positions
  * cover the same range as its indices, so the stable compaction over

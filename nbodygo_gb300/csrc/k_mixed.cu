@@ -5,7 +5,7 @@
  * and the same collision set as Collided (body.go:192-208), with the pair
  * terms in FP32:
  *
- *  - bodies are visited in Morton order (k_sort.cu), so each 512-body i-tile
+ *  - bodies are visited in Hilbert order (k_sort.cu), so each 512-body i-tile
  *    is compact in space;
  *  - positions are held as hi/lo float pairs (x = hi + lo to ~2^-48 |x|);
  *    each work item re-centres positions on its i-tile's origin c with

@@ -289,7 +289,7 @@ static ll part_need(const nbg_ctx *ctx, ll cap)
     return NBG_PART_DOUBLES(cap, (ll)ctx->cb.slots * NBG_MIX_CHUNKS_PER_CTA, itile);
 }
 
-/* The mixed path's Morton order no longer matches the bodies: the arrays
+/* The mixed path's Hilbert order no longer matches the bodies: the arrays
  * were replaced, or bodies were edited or moved from the host. */
 static int drop_order(nbg_ctx *ctx)
 {
@@ -1338,7 +1338,7 @@ int nbg_get_body_in(nbg_ctx *ctx, int64_t sim, int64_t id, nbg_soa *h, int32_t *
  *     the behaviour), each field n values, padded to 8 bytes;
  *   the staged host adds in the same layout (grouped by collection, arrival
  *     order within one);
- *   mixed form: the Morton order of the bodies (uint32 per body) when one is
+ *   mixed form: the Hilbert order of the bodies (uint32 per body) when one is
  *     current, so the FP32 pair sums group the same bodies.
  * Values are stored in the machine's byte order (little-endian on x86-64 and
  * aarch64); the header records the field count and per-body bytes. */
@@ -1587,7 +1587,7 @@ static void launch_cycle(nbg_ctx *ctx, int precision, long ev_base)
         nbg_launch_pair_fp64(cb, ctx->ctl, st);
         if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 2), st);
     }
-    /* the mixed direct path keeps its Morton order through compaction */
+    /* the mixed direct path keeps its Hilbert order through compaction */
     nbg_launch_after_pair(cb, ctx->ctl, st, !cb.bh && precision == NBG_PRECISION_MIXED);
     if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 3), st);
     /* begin, fragment count + scan, 10 after the pair kernel, and the pair
@@ -1834,7 +1834,7 @@ int nbg_force_pass(nbg_ctx *ctx)
         int z = 0;
         CK(cudaMemcpyAsync(&ctx->ctl->error, &z, sizeof z, cudaMemcpyHostToDevice, ctx->st));
         /* a retry follows a buffer k_begin found short (partial-sum or
-         * j-partial slots) or the octree's (Barnes-Hut, which keeps no Morton
+         * j-partial slots) or the octree's (Barnes-Hut, which keeps no spatial
          * order): no kernel after k_begin ran, so the order stands */
         nbg_launch_begin(ctx->cb, ctx->ctl, ctx->st);
         if (ctx->cb.bh) {

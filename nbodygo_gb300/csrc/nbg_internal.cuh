@@ -35,7 +35,7 @@ typedef unsigned long long ull;
 #define NBG_EVT_SUB_JI 2u  /* subsume(j absorbs i) */
 
 #define NBG_MAX_BODIES ((ll)1 << 30) /* event keys pack i and j in 30 bits */
-#define NBG_MAX_SIMS 2048            /* Morton keys of several sims carry the sim in 11 bits */
+#define NBG_MAX_SIMS 2048            /* Hilbert keys of several sims carry the sim in 11 bits */
 
 #define NBG_NF64 20
 struct BodyArrays {
@@ -93,7 +93,7 @@ struct DevCtl {
     ull bh_rmax;
     unsigned bh_next; /* the walk's next 32-body group (one per warp) */
     unsigned pad2;
-    /* Morton order of the mixed path (perm): valid while no body changed
+    /* Hilbert order of the mixed path (perm): valid while no body changed
      * index; re-sorted when invalid or sort_interval cycles after the last
      * sort (0: NBG_SORT_INTERVAL_DEFAULT).  sort_now is this cycle's decision. */
     int sort_valid;
@@ -133,7 +133,7 @@ struct SimSegs {
     ll *hadd_start;  /* [nsims+1] */
     ll *keep_start;  /* [nsims+1] */
     ll *new_off;     /* [nsims+1] layout after Cycle */
-    unsigned *xmax_bits; /* [nsims] mixed: |x| max of sim s (Morton grid) */
+    unsigned *xmax_bits; /* [nsims] mixed: |x| max of sim s (Hilbert grid) */
 };
 
 /* bytes of the SimSegs arrays for nsims sims (one allocation, carved by
@@ -339,6 +339,44 @@ __host__ __device__ __forceinline__ int nbg_work_chunk(ll u, int C, ll W)
  * Slots needed: tiles + C - 1, tiles <= cap / itile + sims. */
 #define NBG_PART_DOUBLES(cap, chunks, itile) \
     (3 * ((ll)(cap) + (ll)(itile) * ((ll)(chunks) + NBG_MAX_SIMS + 2)))
+
+/* 10 bits spread three apart */
+__host__ __device__ __forceinline__ unsigned nbg_spread10(unsigned v)
+{
+    v &= 0x3ffu;
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    v = (v | (v << 2)) & 0x09249249u;
+    return v;
+}
+
+/* Index of cell (x, y, z) of a 2^bits cube along the Hilbert curve (bits <=
+ * 10), by Skilling's transpose method (Programming the Hilbert curve, AIP
+ * Conf. Proc. 707, 2004): the inverse undo of the rotations from the top bit
+ * down, Gray encoding, then the three words' bits interleaved. */
+__host__ __device__ __forceinline__ unsigned nbg_hilbert(unsigned x, unsigned y, unsigned z, int bits)
+{
+    unsigned X[3] = {x, y, z};
+    for (unsigned q = 1u << (bits - 1); q > 1u; q >>= 1) {
+        const unsigned p = q - 1u;
+        for (int i = 0; i < 3; i++) {
+            if (X[i] & q) {
+                X[0] ^= p;
+            } else {
+                const unsigned t = (X[0] ^ X[i]) & p;
+                X[0] ^= t;
+                X[i] ^= t;
+            }
+        }
+    }
+    X[1] ^= X[0];
+    X[2] ^= X[1];
+    unsigned t = 0;
+    for (unsigned q = 1u << (bits - 1); q > 1u; q >>= 1)
+        if (X[2] & q) t ^= q - 1u;
+    return (nbg_spread10(X[0] ^ t) << 2) | (nbg_spread10(X[1] ^ t) << 1) | nbg_spread10(X[2] ^ t);
+}
 
 #define NBG_SCAN_BLOCK 1024
 #define NBG_SCAN_ITEMS 4

@@ -8,7 +8,7 @@
  * the CUDA allocator, or code that runs where an allocation would
  * disturb a memory budget fixed in advance.  nbg_forces_mixed_noalloc serves
  * them.  The caller passes device pointers for the inputs and outputs; every
- * intermediate buffer the force pass needs (sorted packed positions, Morton
+ * intermediate buffer the force pass needs (sorted packed positions, spatial
  * sort keys, tile origins, partial sums, the control block) lives in one
  * file-scope __device__ array of NBG_NOALLOC_BYTES bytes.  Every GPU that
  * loads the library holds that array until the process exits, which is why
