@@ -378,7 +378,8 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
  * (body_collection.go:298-300).  With several collections each gets its own
  * tree, the one a context holding it alone would build. */
 #define NBG_OPT_BARNES_HUT 8
-/* mixed Barnes-Hut walk: registers capped for 3, 4 or 5 CTAs per SM (0..2) */
+/* mixed Barnes-Hut walk: registers capped for 4, 5 or 6 128-thread CTAs per
+   SM (0..2) */
 #define NBG_OPT_BH_SHAPE 9
 /* mixed: cycles between sorts of the i-tiles (1..1000, default 4).
    Bodies move far less than a tile per cycle, so an older order still gives

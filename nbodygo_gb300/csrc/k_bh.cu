@@ -72,6 +72,17 @@
 #define BH_SCAN_BLOCK 1024
 #define BH_SCAN_ITEMS 4
 #define BH_SCAN_TILE (BH_SCAN_BLOCK * BH_SCAN_ITEMS)
+#define BHW_BLOCK 128 /* the mixed walk's CTAs */
+#define BHW_TEAM (BHW_BLOCK / 32)
+/* Collections of at least this many tree bodies have a warp to each group of
+ * 32 bodies; in smaller ones, whose groups would leave warps idle, a CTA's
+ * four warps share a group's walk.  Tree pass, a warp to a group against four:
+ * 30,011 Plummer bodies 1.33 / 1.07 ms, 131,072 2.38 / 2.89 ms, 400,000
+ * 5.8 / 7.5 ms (the four repeat the top of the tree).  Decided for each
+ * collection by its own size, so its sums are those it has alone. */
+#ifndef BHW_SOLO_MIN
+#define BHW_SOLO_MIN 60000
+#endif
 #define BH_F_LEAF 1u
 #define BH_F_NAN_CM 2u
 #define FULL_MASK 0xffffffffu
@@ -189,29 +200,40 @@ __global__ void __launch_bounds__(32) k_bh_segs(DevCtl *ctl, SimSegs seg, BhTree
     const int ns = seg.nsims, lane = threadIdx.x;
     const int per = (ns + 31) / 32;
     const int s0 = lane * per, s1 = s0 + per < ns ? s0 + per : ns;
-    ll c = 0, g = 0;
+    /* units of the mixed walk: a group, or a CTA's warps' worth of them */
+    auto units = [&](int s) {
+        const ll gr = (t.scount[s] + 31) / 32;
+        return t.scount[s] >= BHW_SOLO_MIN ? (gr + BHW_TEAM - 1) / BHW_TEAM : gr;
+    };
+    ll c = 0, g = 0, u = 0;
     for (int s = s0; s < s1; s++) {
         c += t.scount[s];
         g += (t.scount[s] + 31) / 32;
+        u += units(s);
     }
-    ll xc = c, xg = g;
+    ll xc = c, xg = g, xu = u;
     for (int o = 1; o < 32; o <<= 1) {
         const ll yc = __shfl_up_sync(FULL_MASK, xc, o), yg = __shfl_up_sync(FULL_MASK, xg, o);
+        const ll yu = __shfl_up_sync(FULL_MASK, xu, o);
         if (lane >= o) {
             xc += yc;
             xg += yg;
+            xu += yu;
         }
     }
-    ll oc = xc - c, og = xg - g;
+    ll oc = xc - c, og = xg - g, ou = xu - u;
     for (int s = s0; s < s1; s++) {
         t.stree[s] = oc;
         t.sgrp[s] = og;
+        t.sunit[s] = ou;
         oc += t.scount[s];
         og += (t.scount[s] + 31) / 32;
+        ou += units(s);
     }
     if (lane == 31) {
         t.stree[ns] = xc;
         t.sgrp[ns] = xg;
+        t.sunit[ns] = xu;
         ctl->bh_count = xc;
     }
 }
@@ -726,14 +748,75 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_force(BodyArrays A, DevCtl *ctl
  * hi/lo float pairs (so dx = (cm_hi - x_hi) + (cm_lo - x_lo) keeps ~2^-24 of
  * |dx|), masses relative to the root's, the opening test as
  * r^2 > (2 half / theta)^2 on the softened r^2, and the reciprocal square
- * root of the SFU.  The 32 bodies of a warp (neighbours in key order) walk
- * one node sequence together: a lane that accepts a node waits until the
- * warp leaves that node's subtree (its skip pointer), and the warp descends
- * when any lane opens, so every node load is a broadcast and no lane
- * diverges.  A node with no mass below it is skipped by every lane.  Each
- * lane sums its terms in FP32 and, every 64 nodes, the warp folds them into
- * (hi, lo) FP32 pairs: the GB300 FP64 pipe is 1/64 of the FP32 rate, and a
- * few FP64 folds per node kept it saturated. */
+ * root of the SFU.
+ *
+ * A group of 32 bodies (neighbours in key order, one per lane) walks the tree
+ * together.  The warp keeps a stack of nodes, each with the lanes that have
+ * not accepted an ancestor of it, and visits 32 of them at once, one per
+ * lane: most nodes lie so far from the group's box (or so close) that all
+ * its bodies accept (or open) them, which one bound decides; accepted nodes
+ * are listed in shared memory and summed 32 or more at a time, every lane
+ * its own body, two nodes per packed instruction.  Only the nodes in between
+ * (1,100 of the 7,900 that a group of a 131,072-body Plummer sphere accepts)
+ * take each body's own test, with the same expression and rounding as a walk
+ * of that body alone, so every body sums the terms it would alone.  Sums are
+ * FP32, folded into (hi, lo) pairs after every list: the GB300 FP64 pipe is
+ * 1/64 of the FP32 rate.
+ *
+ * A walk that took one node at a time for the whole warp was bound by the
+ * latency of its node loads (issue slots 25 % busy).  The walk of a 131,072-
+ * body Plummer sphere went from 5.0 to 1.56 ms, of 10^6 uniform bodies from
+ * 20.3 to 7.3 ms.  What bounds it now is issue and, with a group to a warp,
+ * groups of uneven cost: 263,000 instructions a group before the lists were
+ * split into far and near ones, 60 % of them in the sums. */
+/* Where the walk finds a node: the children of a node take consecutive
+ * slots, so a visit that opens it goes on with one address and a count.
+ * Slots 0 .. nsims - 1 are the roots'; the others are handed out a warp of
+ * nodes at a time (which children lie where does not matter to the sums, only
+ * the order among siblings does, and that is theirs). */
+__global__ void __launch_bounds__(BH_BLOCK) k_bh_children(DevCtl *ctl, SimSegs seg, BhTree t)
+{
+    if (ctl->error) return;
+    const ll total = ctl->bh_nodes;
+    const int lane = threadIdx.x & 31;
+    for (ll base = (ll)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
+         base += (ll)gridDim.x * blockDim.x) {
+        const ll id = base + lane;
+        int nc = 0, child[8];
+        if (id < total && !(t.flags[id] & BH_F_LEAF)) {
+            const int stop = t.skip[id];
+            int c = (int)id + 1;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                child[q] = c;
+                if (c < stop) {
+                    nc++;
+                    c = t.skip[c];
+                }
+            }
+        }
+        int x = nc;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(FULL_MASK, x, o);
+            if (lane >= o) x += y;
+        }
+        unsigned at = 0;
+        if (lane == 31) at = atomicAdd(&ctl->bh_slots, (unsigned)x);
+        at = __shfl_sync(FULL_MASK, at, 31);
+        if (id < total) {
+            const int first = (int)at + seg.nsims + x - nc;
+            t.cbase[id] = first;
+            t.ccount[id] = (unsigned char)nc;
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (q < nc) t.slot[child[q]] = first + q;
+        }
+    }
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < seg.nsims; s += gridDim.x * blockDim.x)
+        if (t.sroot[s] < t.sroot[s + 1]) t.slot[t.sroot[s]] = s;
+}
+
+/* every node's record for the walk, in its slot */
 __global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(DevCtl *ctl, SimSegs seg, BhTree t)
 {
     if (ctl->error) return;
@@ -757,9 +840,10 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(DevCtl *ctl, SimSegs
             const double o = 2 * t.half[id] / BH_THETA;
             b.w = (float)(o * o);
         }
-        t.fa[id] = a;
-        t.fb[id] = b;
-        t.fc[id] = make_int4(t.skip[id], t.start[id], t.end[id], (int)t.flags[id]);
+        const int slot = t.slot[id];
+        t.fa[slot] = a;
+        t.fb[slot] = b;
+        t.fc[slot] = make_int4(t.cbase[id], (int)t.ccount[id] | ((int)t.flags[id] << 8), t.start[id], t.end[id]);
     }
 }
 
@@ -805,104 +889,430 @@ __device__ __noinline__ int bucket_terms(const BodyArrays &A, const unsigned *va
     return cnt;
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(BH_BLOCK, MINB) k_bh_force_mixed(BodyArrays A, DevCtl *ctl, SimSegs seg,
-                                                                const unsigned *vals, BhTree t)
+/* one warp's working set in shared memory */
+/* runs of sibling nodes still to visit.  Full stacks take nodes one by one:
+ * 384 single nodes in place of runs of up to eight made the walk twice as
+ * long, 1,024 still 10 % longer than 2,048. */
+#ifndef BHW_STACK
+#define BHW_STACK 256
+#endif
+#define BHW_SPARE 32 /* of them kept for taking one node at a time: one a level, 21 levels */
+#define BHW_FAR 64    /* far nodes waiting to be summed */
+#define BHW_MIX 32    /* nodes that need each body's own test, waiting */
+/* a node counts as far when its centre of mass is this many half extents of
+ * the group's box away: re-centred on the box, its coordinates then carry no
+ * more than 1.5 times the rounding of the bodies' distances to it */
+#ifndef BHW_FAR_RATIO
+#define BHW_FAR_RATIO 3.0f
+#endif
+struct alignas(16) BhWarp {
+    uint2 stack[BHW_STACK]; /* (first slot, the lanes that have not accepted an ancestor) */
+    /* far nodes, relative to the box */
+    float fx[BHW_FAR + 4], fy[BHW_FAR + 4], fz[BHW_FAR + 4], fm[BHW_FAR + 4];
+    unsigned fmask[BHW_FAR + 4];
+    /* nodes the bodies may disagree on, and accepted ones close by */
+    float hx[BHW_MIX + 4], hy[BHW_MIX + 4], hz[BHW_MIX + 4], m[BHW_MIX + 4];
+    float lx[BHW_MIX + 4], ly[BHW_MIX + 4], lz[BHW_MIX + 4], open2[BHW_MIX + 4];
+    unsigned mask[BHW_MIX + 4];
+    int cb[BHW_MIX], nc[BHW_MIX];
+    unsigned char run[BHW_STACK]; /* nodes of each run */
+};
+enum { BHW_DROP = 0, BHW_OPEN = 1, BHW_ACCEPT = 2, BHW_MIXED = 3, BHW_BUCKET = 4 };
+
+__device__ __forceinline__ float warp_minf(float v)
 {
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(FULL_MASK, v, o));
+    return v;
+}
+
+/* exclusive prefix of v (0..15) over the lanes and the warp's total */
+__device__ __forceinline__ int warp_prefix4(int v, unsigned lt, int &total)
+{
+    int x = 0;
+    total = 0;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        const unsigned m = __ballot_sync(FULL_MASK, (v >> b) & 1);
+        x += __popc(m & lt) << b;
+        total += __popc(m) << b;
+    }
+    return x;
+}
+
+/* FP32 partial sums and the (hi, lo) pairs they are folded into */
+struct BhSum {
+    float2 ax, ay, az;
+    float hx, lx, hy, ly, hz, lz;
+    __device__ __forceinline__ void term(const float2 &m, const float2 &r2, const float2 &dx, const float2 &dy,
+                                         const float2 &dz)
+    {
+        const float2 inv = make_float2(bh_rsqrt(r2.x), bh_rsqrt(r2.y));
+        const float2 wt = __fmul2_rn(__fmul2_rn(m, inv), __fmul2_rn(inv, inv));
+        ax = __ffma2_rn(wt, dx, ax);
+        ay = __ffma2_rn(wt, dy, ay);
+        az = __ffma2_rn(wt, dz, az);
+    }
+    __device__ __forceinline__ void fold()
+    {
+        fold2(hx, lx, ax.x + ax.y);
+        fold2(hy, ly, ay.x + ay.y);
+        fold2(hz, lz, az.x + az.y);
+        ax = ay = az = make_float2(0.f, 0.f);
+    }
+};
+
+template <int MINB>
+__global__ void __launch_bounds__(BHW_BLOCK, MINB) k_bh_force_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl,
+                                                                 SimSegs seg, const unsigned *vals,
+                                                                 const __grid_constant__ BhTree t)
+{
+    __shared__ BhWarp ws[BHW_TEAM];
+    __shared__ float red[BHW_TEAM - 1][6][32];
+    __shared__ int s_unit;
     if (ctl->error) return;
     if (ctl->bh_nodes <= 0) return;
-    const ll groups = t.sgrp[seg.nsims];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    BhWarp &w = ws[wi];
+    const unsigned lt = (1u << lane) - 1u;
+    const ll units = t.sunit[seg.nsims];
     const float soft2 = (float)(BH_SOFTENING * BH_SOFTENING);
-    unsigned long long terms = 0;
-    for (int grp; (grp = bh_next_group(ctl, groups)) >= 0;) {
-        int r;
-        ll p0, p1;
-        bh_group(t, seg.nsims, grp, r, p0, p1);
-        const ll p = p0 + (threadIdx.x & 31);
-        const int root = (int)t.sroot[r], total = (int)t.sroot[r + 1];
-        const double mroot = t.mass[root];
+    const float2 s2 = make_float2(soft2, soft2);
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    unsigned long long all_terms = 0;
+    for (;;) {
+        if (threadIdx.x == 0) s_unit = (int)atomicAdd(&ctl->bh_next, 1u);
+        __syncthreads();
+        const int unit = s_unit;
+        __syncthreads();
+        if ((ll)unit >= units) break;
+        const int r = nbg_sim_of(t.sunit, seg.nsims, unit);
+        const ll n_r = t.scount[r];
+        const bool solo = n_r >= BHW_SOLO_MIN;
+        const ll g = solo ? BHW_TEAM * (unit - t.sunit[r]) + wi : unit - t.sunit[r];
+        const ll p0 = t.stree[r] + 32 * g, p1 = p0 + 32 < t.stree[r + 1] ? p0 + 32 : t.stree[r + 1];
+        const ll p = p0 + lane;
         unsigned k = 0;
         bool have = p < p1;
         if (have) {
             k = vals[p];
             have = !(A.flags[k] & NBG_F_IS_SUN); /* k_bh_sun */
         }
-        float xh = 0.f, yh = 0.f, zh = 0.f, xl = 0.f, yl = 0.f, zl = 0.f;
-        if (have) {
-            const double x = A.x[k], y = A.y[k], z = A.z[k];
-            xh = (float)x;
-            yh = (float)y;
-            zh = (float)z;
-            xl = (float)(x - (double)xh);
-            yl = (float)(y - (double)yh);
-            zl = (float)(z - (double)zh);
-        }
-        int wait = have ? 0 : 0x7fffffff;
-        float ax = 0.f, ay = 0.f, az = 0.f;
-        /* every 64 nodes the warp folds the FP32 partial sums into (hi, lo)
-         * FP32 pairs (TwoSum): all lanes together, and no FP64 in the walk */
-        float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f, hz = 0.f, lz = 0.f;
-        int nacc = 0, steps = 0;
-        if (!__any_sync(FULL_MASK, have)) continue;
-        /* The next node is the first child when any lane opens this one, and
-         * otherwise this node's skip pointer: every lane that waits at this
-         * node accepted an ancestor, whose subtree ends at or after this
-         * node's.  So the next address is known right after the vote, and its
-         * loads are in flight while the lanes add their terms. */
-        int id = root;
-        float4 a = t.fa[root], b = t.fb[root];
-        int4 c = t.fc[root];
-        while (id < total) {
-            const int sk = c.x;
-            const unsigned fl = (unsigned)c.w;
-            const bool leaf = (fl & BH_F_LEAF) != 0;
-            const bool live = a.w != 0.f; /* nothing with mass below: skipped by every lane */
-            const bool active = live && id >= wait;
-            const float dx = (a.x - xh) + (b.x - xl);
-            const float dy = (a.y - yh) + (b.y - yl);
-            const float dz = (a.z - zh) + (b.z - zl);
-            const float r2 = dx * dx + dy * dy + dz * dz + soft2;
-            const bool accept = leaf || (!(fl & BH_F_NAN_CM) && r2 > b.w);
-            const int next = __any_sync(FULL_MASK, active && !accept) ? id + 1 : sk;
-            const int s = c.y, e = c.z;
-            const float mw = a.w;
-            if (next < total) {
-                a = t.fa[next];
-                b = t.fb[next];
-                c = t.fc[next];
+        const unsigned every = __ballot_sync(FULL_MASK, have);
+        if (!every) continue; /* solo warps meet at the next unit; a team's agree */
+        float2 xh, yh, zh, xl, yl, zl; /* (-hi, -hi) and (-lo, -lo) of the lane's body */
+        float2 xr, yr, zr;             /* minus its offset from the box's centre */
+        float gx, gy, gz, ex, ey, ez, far2;
+        {
+            float vh[3] = {0.f, 0.f, 0.f}, vl[3] = {0.f, 0.f, 0.f};
+            if (have) {
+                const double x = A.x[k], y = A.y[k], z = A.z[k];
+                vh[0] = (float)x;
+                vh[1] = (float)y;
+                vh[2] = (float)z;
+                vl[0] = (float)(x - (double)vh[0]);
+                vl[1] = (float)(y - (double)vh[1]);
+                vl[2] = (float)(z - (double)vh[2]);
             }
-            if (active && accept) {
-                if (leaf && e - s > 1) {
-                    nacc += bucket_terms(A, vals, s, e, k, xh, yh, zh, xl, yl, zl, soft2, mroot, ax, ay, az);
-                } else if (!(leaf && (ll)s == p)) { /* a one-body leaf holds sorted position s */
-                    const float inv = bh_rsqrt(r2);
-                    const float w = mw * inv * inv * inv;
-                    ax += w * dx;
-                    ay += w * dy;
-                    az += w * dz;
-                    nacc++;
+            /* the group's box: centre g, half extents e, widened past the
+             * rounding of the positions and of the distances to it */
+            float g3[3], e3[3], o3[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float lo = warp_minf(have ? vh[c] : 3e38f), hi = -warp_minf(have ? -vh[c] : 3e38f);
+                g3[c] = 0.5f * lo + 0.5f * hi;
+                e3[c] = fmaxf(hi - g3[c], g3[c] - lo) + 0x1p-20f * fmaxf(fabsf(lo), fabsf(hi));
+                o3[c] = (vh[c] - g3[c]) + vl[c];
+            }
+            gx = g3[0], gy = g3[1], gz = g3[2];
+            ex = e3[0], ey = e3[1], ez = e3[2];
+            far2 = (BHW_FAR_RATIO * BHW_FAR_RATIO) * (ex * ex + ey * ey + ez * ez);
+            xh = make_float2(-vh[0], -vh[0]);
+            yh = make_float2(-vh[1], -vh[1]);
+            zh = make_float2(-vh[2], -vh[2]);
+            xl = make_float2(-vl[0], -vl[0]);
+            yl = make_float2(-vl[1], -vl[1]);
+            zl = make_float2(-vl[2], -vl[2]);
+            xr = make_float2(-o3[0], -o3[0]);
+            yr = make_float2(-o3[1], -o3[1]);
+            zr = make_float2(-o3[2], -o3[2]);
+        }
+        BhSum b;
+        b.ax = b.ay = b.az = make_float2(0.f, 0.f);
+        b.hx = b.lx = b.hy = b.ly = b.hz = b.lz = 0.f;
+        unsigned terms = 0;
+        int cf = 0, cm = 0; /* nodes in the two lists */
+        int top = 1;
+        /* until the walk is dealt out, every warp of a team walks the same
+         * top of the tree, and only the first keeps its terms */
+        bool dealt = solo;
+        if (lane == 0) {
+            w.stack[0] = make_uint2((unsigned)r, every);
+            w.run[0] = 1;
+        }
+        __syncwarp();
+        /* the far list's terms, two per packed instruction */
+        auto flush = [&]() {
+            if (lane < 3) {
+                const int at = cf + lane; /* up to a multiple of four with nothing */
+                w.fx[at] = w.fy[at] = w.fz[at] = w.fm[at] = 0.f;
+                w.fmask[at] = every;
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int q = 0; q < cf; q += 4) {
+                const float4 X = *(const float4 *)&w.fx[q], Y = *(const float4 *)&w.fy[q];
+                const float4 Z = *(const float4 *)&w.fz[q];
+                float4 M = *(const float4 *)&w.fm[q];
+                const uint4 K = *(const uint4 *)&w.fmask[q];
+                if ((K.x & K.y & K.z & K.w) != every) {
+                    M.x = (K.x >> lane) & 1u ? M.x : 0.f;
+                    M.y = (K.y >> lane) & 1u ? M.y : 0.f;
+                    M.z = (K.z >> lane) & 1u ? M.z : 0.f;
+                    M.w = (K.w >> lane) & 1u ? M.w : 0.f;
                 }
-                wait = sk;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const float2 dx = __fadd2_rn(h ? make_float2(X.z, X.w) : make_float2(X.x, X.y), xr);
+                    const float2 dy = __fadd2_rn(h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y), yr);
+                    const float2 dz = __fadd2_rn(h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y), zr);
+                    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, s2)));
+                    b.term(h ? make_float2(M.z, M.w) : make_float2(M.x, M.y), r2, dx, dy, dz);
+                }
             }
-            if (++steps == 64) {
-                fold2(hx, lx, ax);
-                fold2(hy, ly, ay);
-                fold2(hz, lz, az);
-                ax = ay = az = 0.f;
-                steps = 0;
+            b.fold();
+            cf = 0;
+            __syncwarp();
+        };
+        /* the second list: each body's own test, with the precise distance;
+         * the children of the nodes that some body opens go on the stack */
+        auto settle = [&]() {
+            if (lane < 3) {
+                const int at = cm + lane;
+                w.hx[at] = w.hy[at] = w.hz[at] = w.m[at] = w.lx[at] = w.ly[at] = w.lz[at] = w.open2[at] = 0.f;
+                w.mask[at] = 0u;
             }
-            id = next;
+            __syncwarp();
+            unsigned open = 0, tm = 0;
+#pragma unroll 1
+            for (int q = 0; q < cm; q += 2) {
+                const float2 X = *(const float2 *)&w.hx[q], Y = *(const float2 *)&w.hy[q], Z = *(const float2 *)&w.hz[q];
+                const float2 U = *(const float2 *)&w.lx[q], V = *(const float2 *)&w.ly[q], W = *(const float2 *)&w.lz[q];
+                const float2 M = *(const float2 *)&w.m[q], O = *(const float2 *)&w.open2[q];
+                const uint2 K = *(const uint2 *)&w.mask[q];
+                const float2 dx = __fadd2_rn(__fadd2_rn(X, xh), __fadd2_rn(U, xl));
+                const float2 dy = __fadd2_rn(__fadd2_rn(Y, yh), __fadd2_rn(V, yl));
+                const float2 dz = __fadd2_rn(__fadd2_rn(Z, zh), __fadd2_rn(W, zl));
+                /* rounded as the acceptance rule states it: each square, the
+                 * sums left to right, the softening last */
+                const float2 r2 = __fadd2_rn(
+                    __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz)), s2);
+                const bool k0 = (K.x >> lane) & 1u, k1 = (K.y >> lane) & 1u;
+                const bool a0 = k0 && r2.x > O.x, a1 = k1 && r2.y > O.y;
+                const unsigned o0 = __ballot_sync(FULL_MASK, k0 && !a0), o1 = __ballot_sync(FULL_MASK, k1 && !a1);
+                if (lane == q) open = o0;
+                if (lane == q + 1) open = o1;
+                tm += (unsigned)a0 + (unsigned)a1;
+                b.term(make_float2(a0 ? M.x : 0.f, a1 ? M.y : 0.f), r2, dx, dy, dz);
+            }
+            b.fold();
+            if (dealt || wi == 0) terms += tm;
+            const unsigned om = __ballot_sync(FULL_MASK, open != 0u); /* lanes below cm only */
+            if (open) {
+                const int at = top + __popc(om & lt);
+                w.stack[at] = make_uint2((unsigned)w.cb[lane], open);
+                w.run[at] = (unsigned char)w.nc[lane];
+            }
+            top += __popc(om);
+            cm = 0;
+            __syncwarp();
+        };
+        for (;;) {
+            if (cm > 0 && (top == 0 || !dealt || top + cm + 32 > BHW_STACK - BHW_SPARE)) settle();
+            if (!dealt && (top == 0 || top >= 32)) {
+                /* the team's warps take every BHW_TEAM-th run */
+                int n = 0;
+                for (int s0 = 0; s0 < top; s0 += 32 * BHW_TEAM) {
+                    const int i = s0 + lane * BHW_TEAM + wi;
+                    const uint2 en = i < top ? w.stack[i] : make_uint2(0u, 0u);
+                    const unsigned char rn = i < top ? w.run[i] : 0;
+                    __syncwarp();
+                    if (i < top) {
+                        w.stack[n + lane] = en;
+                        w.run[n + lane] = rn;
+                    }
+                    n += __popc(__ballot_sync(FULL_MASK, i < top));
+                    __syncwarp();
+                }
+                top = n;
+                dealt = true;
+            }
+            if (top == 0) break; /* the second list is empty here too */
+            /* The next 32 nodes at once, of the topmost runs: lane i reads run
+             * i from the top; `mark` has a bit at each run's first node.  Each
+             * node leaves at most one run, so a nearly full stack takes fewer,
+             * down to one at a time: a descent that adds a run a level. */
+            int take = BHW_STACK - BHW_SPARE - top - cm;
+            take = take > 32 ? 32 : take < 1 ? 1 : take;
+            int cls = BHW_DROP, nc = 0, s = 0, e = 0, cb = 0;
+            unsigned mask = 0;
+            float4 na = zero4, nb = zero4;
+            int4 nd = make_int4(0, 0, 0, 0);
+            {
+                uint2 en = make_uint2(0u, 0u);
+                int rn = 0;
+                if (lane < top) {
+                    en = w.stack[top - 1 - lane];
+                    rn = w.run[top - 1 - lane];
+                }
+                int tot;
+                const int x = warp_prefix4(rn, lt, tot);
+                if (take > tot) take = tot;
+                const unsigned mark = __reduce_or_sync(FULL_MASK, rn > 0 && x < take ? 1u << x : 0u);
+                const unsigned m = mark & (0xffffffffu >> (31 - lane));
+                const int from = __popc(m) - 1, off = lane - (31 - __clz(m));
+                const unsigned slot = __shfl_sync(FULL_MASK, en.x, from) + (unsigned)off;
+                mask = __shfl_sync(FULL_MASK, en.y, from);
+                if (lane < take) {
+                    na = t.fa[slot];
+                    nb = t.fb[slot];
+                    nd = t.fc[slot];
+                }
+                /* the one run taken in part keeps the rest */
+                if (x < take && x + rn > take) {
+                    w.stack[top - 1 - lane] = make_uint2(en.x + (unsigned)(take - x), en.y);
+                    w.run[top - 1 - lane] = (unsigned char)(x + rn - take);
+                }
+                top -= __popc(__ballot_sync(FULL_MASK, rn > 0 && x + rn <= take));
+            }
+            if (cf >= 32) flush(); /* while those loads are in flight */
+            bool isfar = false;
+            if (lane < take) {
+                cb = nd.x;
+                nc = nd.y & 0xff;
+                s = nd.z;
+                e = nd.w;
+                const unsigned fl = (unsigned)nd.y >> 8;
+                const float ux = na.x - gx, uy = na.y - gy, uz = na.z - gz;
+                isfar = ux * ux + uy * uy + uz * uz > far2;
+                if (na.w == 0.f) {
+                    cls = BHW_DROP; /* nothing with mass below: skipped by every body */
+                } else if (fl & BH_F_LEAF) {
+                    cls = e - s > 1 ? BHW_BUCKET : BHW_ACCEPT;
+                    /* a one-body leaf holds sorted position s: not for itself */
+                    if (cls == BHW_ACCEPT && s >= p0 && s < p0 + 32) mask &= ~(1u << (int)(s - p0));
+                } else if (fl & BH_F_NAN_CM) {
+                    cls = BHW_OPEN;
+                } else {
+                    /* nearest and farthest the box can be from the centre of
+                     * mass, with room for every rounding of the bodies' own
+                     * tests: outside both bounds the bodies agree */
+                    const float mx = ex + 0x1p-20f * fabsf(na.x), my = ey + 0x1p-20f * fabsf(na.y);
+                    const float mz = ez + 0x1p-20f * fabsf(na.z);
+                    const float nx = fmaxf(fabsf(ux) - mx, 0.f), ny = fmaxf(fabsf(uy) - my, 0.f);
+                    const float nz = fmaxf(fabsf(uz) - mz, 0.f);
+                    const float fx = fabsf(ux) + mx, fy = fabsf(uy) + my, fz = fabsf(uz) + mz;
+                    const float rn = nx * nx + ny * ny + nz * nz, rf = fx * fx + fy * fy + fz * fz + soft2;
+                    cls = rn * (1.0f - 0x1p-18f) > nb.w ? BHW_ACCEPT
+                          : rf * (1.0f + 0x1p-18f) < nb.w ? BHW_OPEN : BHW_MIXED;
+                }
+                if (cls == BHW_ACCEPT && !isfar) { /* precise distances, no test, no children */
+                    cls = BHW_MIXED;
+                    nb.w = -1.f;
+                    nc = 0;
+                }
+            }
+            __syncwarp();
+            /* opened by every body: its children, for the same bodies */
+            {
+                const unsigned om = __ballot_sync(FULL_MASK, cls == BHW_OPEN);
+                if (cls == BHW_OPEN) {
+                    const int at = top + __popc(om & lt);
+                    w.stack[at] = make_uint2((unsigned)cb, mask);
+                    w.run[at] = (unsigned char)nc;
+                }
+                top += __popc(om);
+            }
+            /* accepted by every body, far away: listed */
+            const unsigned am = __ballot_sync(FULL_MASK, cls == BHW_ACCEPT && (dealt || wi == 0));
+            if ((am >> lane) & 1u) {
+                const int at = cf + __popc(am & lt);
+                w.fx[at] = (na.x - gx) + nb.x;
+                w.fy[at] = (na.y - gy) + nb.y;
+                w.fz[at] = (na.z - gz) + nb.z;
+                w.fm[at] = na.w;
+                w.fmask[at] = mask;
+                terms += __popc(mask);
+            }
+            cf += __popc(am);
+            /* each body decides for itself, later */
+            const unsigned mm = __ballot_sync(FULL_MASK, cls == BHW_MIXED);
+            if (mm) {
+                if (cm + __popc(mm) > BHW_MIX) settle();
+                if (cls == BHW_MIXED) {
+                    const int at = cm + __popc(mm & lt);
+                    w.hx[at] = na.x;
+                    w.hy[at] = na.y;
+                    w.hz[at] = na.z;
+                    w.m[at] = dealt || wi == 0 ? na.w : 0.f;
+                    w.lx[at] = nb.x;
+                    w.ly[at] = nb.y;
+                    w.lz[at] = nb.z;
+                    w.open2[at] = nb.w;
+                    w.mask[at] = mask;
+                    w.cb[at] = cb;
+                    w.nc[at] = nc;
+                }
+                cm += __popc(mm);
+            }
+            /* a leaf at the deepest level holding several bodies */
+            for (unsigned bm = __ballot_sync(FULL_MASK, cls == BHW_BUCKET && (dealt || wi == 0)); bm; bm &= bm - 1u) {
+                const int src = __ffs(bm) - 1;
+                const unsigned mk = __shfl_sync(FULL_MASK, mask, src);
+                const int bs = __shfl_sync(FULL_MASK, s, src), be = __shfl_sync(FULL_MASK, e, src);
+                if ((mk >> lane) & 1u) {
+                    float tx = 0.f, ty = 0.f, tz = 0.f;
+                    terms += bucket_terms(A, vals, bs, be, k, -xh.x, -yh.x, -zh.x, -xl.x, -yl.x, -zl.x, soft2,
+                                          t.mass[t.sroot[r]], tx, ty, tz);
+                    b.ax.x += tx;
+                    b.ay.x += ty;
+                    b.az.x += tz;
+                }
+                __syncwarp();
+            }
+            __syncwarp();
         }
-        if (have) {
-            terms += nacc;
-            const double gm = NBG_G * A.m[k] * mroot;
-            A.fx[k] = gm * (((double)hx + (double)lx) + (double)ax);
-            A.fy[k] = gm * (((double)hy + (double)ly) + (double)ay);
-            A.fz[k] = gm * (((double)hz + (double)lz) + (double)az);
+        flush();
+        if (!solo) {
+            /* the team's sums, in warp order */
+            if (wi > 0) {
+                red[wi - 1][0][lane] = b.hx;
+                red[wi - 1][1][lane] = b.lx;
+                red[wi - 1][2][lane] = b.hy;
+                red[wi - 1][3][lane] = b.ly;
+                red[wi - 1][4][lane] = b.hz;
+                red[wi - 1][5][lane] = b.lz;
+            }
+            __syncthreads();
+            if (wi == 0)
+                for (int q = 0; q < BHW_TEAM - 1; q++) {
+                    fold2(b.hx, b.lx, red[q][0][lane]);
+                    fold2(b.hy, b.ly, red[q][2][lane]);
+                    fold2(b.hz, b.lz, red[q][4][lane]);
+                    b.lx += red[q][1][lane];
+                    b.ly += red[q][3][lane];
+                    b.lz += red[q][5][lane];
+                }
         }
+        if (have && (solo || wi == 0)) {
+            const double gm = NBG_G * A.m[k] * t.mass[t.sroot[r]];
+            A.fx[k] = gm * ((double)b.hx + (double)b.lx);
+            A.fy[k] = gm * ((double)b.hy + (double)b.ly);
+            A.fz[k] = gm * ((double)b.hz + (double)b.lz);
+        }
+        all_terms += terms;
     }
-    for (int o = 16; o > 0; o >>= 1) terms += __shfl_xor_sync(FULL_MASK, terms, o);
-    if ((threadIdx.x & 31) == 0 && terms) atomicAdd((unsigned long long *)&ctl->acc_bh_terms, terms);
+    for (int o = 16; o > 0; o >>= 1) all_terms += __shfl_xor_sync(FULL_MASK, all_terms, o);
+    if (lane == 0 && all_terms) atomicAdd((unsigned long long *)&ctl->acc_bh_terms, all_terms);
 }
 
 /* a sun sums every tree body directly (directForce, octree.go:310-325): each
@@ -1075,15 +1485,19 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
     ALLOC(t.first, node_cap);
     ALLOC(t.level, node_cap);
     ALLOC(t.flags, node_cap);
-    ALLOC(t.fa, node_cap);
-    ALLOC(t.fb, node_cap);
-    ALLOC(t.fc, node_cap);
+    ALLOC(t.fa, node_cap + NBG_MAX_SIMS); /* a slot per collection's root, used or not */
+    ALLOC(t.fb, node_cap + NBG_MAX_SIMS);
+    ALLOC(t.fc, node_cap + NBG_MAX_SIMS);
     ALLOC(t.fd, node_cap);
+    ALLOC(t.cbase, node_cap);
+    ALLOC(t.ccount, node_cap);
+    ALLOC(t.slot, node_cap);
     ALLOC(t.sbox, 6 * (ll)NBG_MAX_SIMS);
     ALLOC(t.scount, NBG_MAX_SIMS + 1);
     ALLOC(t.stree, NBG_MAX_SIMS + 1);
     ALLOC(t.sroot, NBG_MAX_SIMS + 1);
     ALLOC(t.sgrp, NBG_MAX_SIMS + 1);
+    ALLOC(t.sunit, NBG_MAX_SIMS + 1);
 #undef ALLOC
     if (!ok) {
         nbg_bh_free(t);
@@ -1097,8 +1511,8 @@ void nbg_bh_free(BhTree &t)
 {
     void *ps[] = {t.key[0], t.key[1], t.val[0], t.val[1], t.hist, t.base, t.blk, t.mass, t.mx, t.my,
                   t.mz, t.cmx, t.cmy, t.cmz, t.cx, t.cy, t.cz, t.half, t.skip, t.start,
-                  t.end, t.first, t.level, t.flags, t.fa, t.fb, t.fc, t.fd,
-                  t.sbox, t.scount, t.stree, t.sroot, t.sgrp};
+                  t.end, t.first, t.level, t.flags, t.fa, t.fb, t.fc, t.fd, t.cbase, t.ccount, t.slot,
+                  t.sbox, t.scount, t.stree, t.sroot, t.sgrp, t.sunit};
     for (void *p : ps) cudaFree(p);
     memset(&t, 0, sizeof t);
 }
@@ -1143,16 +1557,18 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
     for (int level = BH_LEVELS; level >= 0; level--)
         k_bh_mass<<<ng, BH_BLOCK, 0, st>>>(cb.a, ctl, t.val[0], t, level);
     if (mixed) {
+        k_bh_children<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
         k_bh_prep_mixed<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
-        /* CTAs per SM the walk's registers are capped for: the walk is bound
-         * by the latency of its node loads, so occupancy is what counts */
-        /* one wave of resident CTAs; their warps share the group queue */
-        const int minb = cb.bh_shape == 1 ? 4 : cb.bh_shape == 2 ? 5 : 3;
-        const int gw = g < cb.sms * minb ? g : cb.sms * minb;
+        /* one wave of resident CTAs, which share the queue of units; 4 CTAs
+         * per SM (121 registers, no spill) measured fastest, 2.38 ms for the
+         * tree pass of 131,072 Plummer bodies against 2.52 with 5 or 6 */
+        const int minb = cb.bh_shape == 1 ? 5 : cb.bh_shape == 2 ? 6 : 4;
+        const ll wgroups = cap / 32 + 1 + seg.nsims;
+        const int gw = (int)(wgroups < (ll)cb.sms * minb ? wgroups : (ll)cb.sms * minb);
         switch (cb.bh_shape) {
-        case 1: k_bh_force_mixed<4><<<gw, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
-        case 2: k_bh_force_mixed<5><<<gw, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
-        default: k_bh_force_mixed<3><<<gw, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
+        case 1: k_bh_force_mixed<5><<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
+        case 2: k_bh_force_mixed<6><<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
+        default: k_bh_force_mixed<4><<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
         }
     } else {
         k_bh_force<<<g, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t);
@@ -1166,5 +1582,5 @@ int nbg_bh_launches(const CycleBufs &cb, bool mixed)
     const int passes = cb.seg.nsims > 1 ? 10 : 8;
     /* reset, bounds, segs, keys; the sort; count, top, scan, roots, nodes;
      * masses; (prep,) walk; suns; collisions */
-    return 4 + 3 * passes + 5 + (BH_LEVELS + 1) + (mixed ? 2 : 1) + 2;
+    return 4 + 3 * passes + 5 + (BH_LEVELS + 1) + (mixed ? 3 : 1) + 2;
 }

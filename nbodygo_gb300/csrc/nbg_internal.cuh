@@ -92,7 +92,7 @@ struct DevCtl {
     ll bh_nodes;
     ull bh_rmax;
     unsigned bh_next; /* the walk's next 32-body group (one per warp) */
-    unsigned pad2;
+    unsigned bh_slots; /* mixed walk: child slots handed out */
     /* Hilbert order of the mixed path (perm): valid while no body changed
      * index; re-sorted when invalid or sort_interval cycles after the last
      * sort (0: NBG_SORT_INTERVAL_DEFAULT).  sort_now is this cycle's decision. */
@@ -184,19 +184,22 @@ struct BhTree {
     ll *base;           /* nodes starting at each sorted position, then their scan */
     ll *blk;            /* per-block sums of that scan */
     double *mass, *mx, *my, *mz, *cmx, *cmy, *cmz, *cx, *cy, *cz, *half;
-    float4 *fa, *fb;    /* mixed walk: (cm hi xyz, mass / root mass), (cm lo xyz, opening r^2) */
-    int4 *fc;           /* mixed walk: (skip, start, end, flags) */
+    float4 *fa, *fb;    /* mixed walk, by slot: (cm hi xyz, mass / root mass), (cm lo xyz, opening r^2) */
+    int4 *fc;           /* mixed walk, by slot: (first child's slot, children | flags << 8, start, end) */
     float4 *fd;         /* collision query: the node's cube (centre xyz, half) in FP32 */
     int *skip, *start, *end, *first;
+    int *cbase;            /* mixed walk: slot of the first of the node's children */
+    unsigned char *ccount; /* and how many there are */
+    int *slot;             /* the node's own slot */
     unsigned char *level, *flags;
     /* one tree per collection, all in one depth-first node array: per
      * collection s its bounding box (sbox[6 s ..]: lo xyz, hi xyz as
      * order-preserving integers), tree bodies (scount), first sorted
      * position (stree, [nsims + 1]), root node (sroot, [nsims + 1]: the nodes
-     * of s are [sroot[s], sroot[s + 1])) and first 32-body walk group (sgrp,
-     * [nsims + 1]) */
+     * of s are [sroot[s], sroot[s + 1])), first 32-body walk group (sgrp,
+     * [nsims + 1]) and first unit of the mixed walk (sunit, [nsims + 1]) */
     ull *sbox;
-    ll *scount, *stree, *sroot, *sgrp;
+    ll *scount, *stree, *sroot, *sgrp, *sunit;
     ll node_cap;
 };
 
@@ -255,7 +258,7 @@ struct CycleBufs {
     double *p64_terms, *p64_acc;
     ll p64_jc;
     int bh;             /* forces from the Barnes-Hut octree */
-    int bh_shape;       /* register cap of the mixed walk: 0, 1, 2 = 3, 4, 5 CTAs per SM */
+    int bh_shape;       /* register cap of the mixed walk: 0, 1, 2 = 4, 5, 6 CTAs per SM */
     int sms;            /* streaming multiprocessors of the device */
     BhTree t;
 };
