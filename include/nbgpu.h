@@ -388,11 +388,9 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
    cycle.  The order affects FP32 rounding, never the event set.  1 sorts
    every cycle. */
 #define NBG_OPT_SORT_INTERVAL 10
-/* plain form, one collection: up to this capacity (default 65536) the pair
-   terms of all (i, j) are computed at once and each body adds its own in j
-   order; above it one thread walks each body's j.  Identical results; the
-   first keeps the FP64 pipes busy when there are few bodies, at the cost of
-   a 48 MB-per-thousand-bodies term buffer. */
+/* accepted for programs that set it (0..2^30); it chose between two pair
+   passes of the plain form with the same results, and one pass now serves
+   every size without a term buffer */
 #define NBG_OPT_P64_SPLIT_MAX 11
 /* wall-clock limit of one nbg_step call in milliseconds (0 = none): the call
    launches no further cycle once it has passed, and returns NBG_E_TIMEOUT */

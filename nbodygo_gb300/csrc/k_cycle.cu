@@ -13,6 +13,7 @@
 #error "k_cycle.cu must be compiled with --fmad=false -DNBG_NO_FMAD"
 #endif
 
+#include "nbg_exact.h"
 #include "nbg_internal.cuh"
 #include "nbg_math.h"
 #include "nbg_shared.h"
@@ -272,233 +273,238 @@ __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_scan_blocks(DevCtl *ctl, Sim
 /* K1: plain FP64 force + collision detection                              */
 /* ------------------------------------------------------------------------ */
 
-#define P64_BLOCK 64
-
-/* Detection rule of Compute's second pass (body.go:172-186) for a pair with
- * Collided(i, j) true. Returns the event type or -1. */
-/*
- * One thread per body i.  For each j in array order (tiles of P64_BLOCK staged
- * in shared memory) it evaluates exactly the reference's expressions
- * (calcForceFrom, body.go:214-225): the sum runs over j in ascending order,
- * so the result is bit-identical to the sequential loop.  The same dist
- * decides Collided (body.go:192-208); hits are appended to the event list.
- */
-__global__ void __launch_bounds__(P64_BLOCK) k_pair_fp64(BodyArrays A, DevCtl *ctl, SimSegs seg, ull *ev_keys,
-                                                          ll ev_cap)
+/* One pair of calcForceFrom and Collided (body.go:192-225) with the ordinary
+ * operators, for whatever the straight path does not take: bodies that may
+ * touch (their comparison and their event), that are not there, massless or
+ * the same one, and the operands nbg_exact.h refuses. */
+__device__ __noinline__ static void p64_pair_plain(DevCtl *ctl, ull *ev_keys, ll ev_cap, ll i, ll j, unsigned fi,
+                                                   unsigned fj, double dx, double dy, double dz, double gmi, double mj,
+                                                   double ri, double rj, double &ex, double &ey, double &ez)
 {
-    __shared__ double sx[P64_BLOCK], sy[P64_BLOCK], sz[P64_BLOCK], sm[P64_BLOCK], sr[P64_BLOCK];
-    __shared__ unsigned sf[P64_BLOCK];
-    if (ctl->error) return;
-    const ll ntiles = seg.tile_off[seg.nsims];
-    for (ll T = blockIdx.x; T < ntiles; T += gridDim.x) {
-        /* tile T of sim s: i in [s0 + 64 t, ...), j over the sim [s0, s1) */
-        const int sim = nbg_sim_of(seg.tile_off, seg.nsims, T);
-        const ll s0 = seg.off[sim], n = seg.off[sim + 1];
-        const ll i = s0 + (T - seg.tile_off[sim]) * P64_BLOCK + threadIdx.x;
-        const bool valid = i < n;
-        double xi = 0, yi = 0, zi = 0, mi = 0, ri = 0;
-        unsigned fi = 0;
-        if (valid) {
-            xi = A.x[i];
-            yi = A.y[i];
-            zi = A.z[i];
-            mi = A.m[i];
-            ri = A.rad[i];
-            fi = A.flags[i];
-        }
-        const bool live_i = valid && (fi & NBG_LIVE_MASK) == NBG_F_EXISTS;
-        const bool coll_i = (fi & NBG_F_COLLIDED) != 0;
-        const unsigned bi = NBG_BEHAVIOR(fi);
-        const double gmi = NBG_G * mi;
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        for (ll j0 = s0; j0 < n; j0 += P64_BLOCK) {
-            __syncthreads();
-            const ll jl = j0 + threadIdx.x;
-            if (jl < n) {
-                sx[threadIdx.x] = A.x[jl];
-                sy[threadIdx.x] = A.y[jl];
-                sz[threadIdx.x] = A.z[jl];
-                sm[threadIdx.x] = A.m[jl];
-                sr[threadIdx.x] = A.rad[jl];
-                sf[threadIdx.x] = A.flags[jl];
-            }
-            __syncthreads();
-            if (!live_i) continue;
-            const int cnt = (n - j0) < P64_BLOCK ? (int)(n - j0) : P64_BLOCK;
-            /* unrolled: the divisions and square roots of later j overlap;
-             * the sum still runs in j order */
-#pragma unroll 4
-            for (int t = 0; t < cnt; t++) {
-                const ll j = j0 + t;
-                const double dx = sx[t] - xi;
-                const double dy = sy[t] - yi;
-                const double dz = sz[t] - zi;
-                const double dist = sqrt(dx * dx + dy * dy + dz * dz);
-                const double rr = ri + sr[t];
-                const unsigned fj = sf[t];
-                const bool live_j = (fj & NBG_LIVE_MASK) == NBG_F_EXISTS;
-                if (live_j && j != i && (coll_i || dist > rr)) {
-                    const double force = gmi * sm[t] / (dist * dist);
-                    fx += force * dx / dist;
-                    fy += force * dy / dist;
-                    fz += force * dz / dist;
-                }
-                if (!coll_i && dist <= rr && j != i) {
-                    int type = nbg_detect_event(bi, NBG_BEHAVIOR(fj), ri, sr[t], dist);
-                    if (type >= 0) nbg_emit_event(ctl, ev_keys, ev_cap, i, j, type);
-                }
-            }
-        }
-        if (live_i) {
-            A.fx[i] = fx;
-            A.fy[i] = fy;
-            A.fz[i] = fz;
-        }
+    ex = ey = ez = 0.0;
+    if ((fi & NBG_LIVE_MASK) != NBG_F_EXISTS || j == i) return;
+    const double dist = sqrt(dx * dx + dy * dy + dz * dz);
+    const double rr = ri + rj;
+    const bool coll_i = (fi & NBG_F_COLLIDED) != 0;
+    if (!coll_i && dist <= rr) {
+        const int type = nbg_detect_event(NBG_BEHAVIOR(fi), NBG_BEHAVIOR(fj), ri, rj, dist);
+        if (type >= 0) nbg_emit_event(ctl, ev_keys, ev_cap, i, j, type);
     }
+    if ((fj & NBG_LIVE_MASK) != NBG_F_EXISTS || !(coll_i || dist > rr)) return;
+    const double force = gmi * mj / (dist * dist);
+    ex = force * dx / dist;
+    ey = force * dy / dist;
+    ez = force * dz / dist;
 }
 
-/* Small collections: one thread per body leaves most of the GPU idle (1,000
- * bodies fill 16 SMs), and FP64 runs at 1/64 of the FP32 rate.  So the pair
- * terms are computed for all (i, j) at once and stored, then each body adds
- * its terms in j order: the same expressions, the same additions in the same
- * order, so the result is bit-identical to k_pair_fp64.  A term that the
- * reference skips is stored as +0.0, and adding +0.0 changes no sum here
- * (the sum starts at +0.0 and can never be -0.0).  j runs in passes of jc;
- * the sums are carried between passes in acc.  One collection. */
-/* P64_JS: j per block of k_p64_terms.  Many small blocks keep the FP64
- * pipes fed: 16 j (64 measured 2 % slower from 8,192 to 32,768 bodies), and
- * 4 for capacities up to 8,192, where the whole pass is only a few thousand
- * warps of long FP64 division chains. */
-template <int P64_JS>
-__global__ void __launch_bounds__(P64_BLOCK) k_p64_terms(BodyArrays A, DevCtl *ctl, double *T, ll cap, ll jc,
-                                                         ll jbase, ull *ev_keys, ll ev_cap)
+/* Upper bound on the high word of 2 max(r, 0): dist > r_i + r_j for sure when
+ * dist's high word is above both bodies' bounds.  NaN and huge radii get the
+ * largest value, and their pairs the exact comparison. */
+__device__ __forceinline__ int p64_radius_bound(double r)
 {
-    __shared__ double sx[P64_JS], sy[P64_JS], sz[P64_JS], sm[P64_JS], sr[P64_JS];
-    __shared__ unsigned sf[P64_JS];
-    if (ctl->error) return;
-    const ll n = ctl->n;
-    /* this pass's j: to the end of the collection and of the pass */
-    const ll jend = jbase + jc < n ? jbase + jc : n;
-    if (jbase >= jend) return;
-    /* work items (block of 64 i, block of P64_JS j) of the live bodies only:
-     * a grid sized for the capacity would be mostly empty blocks */
-    const ll nib = (n + P64_BLOCK - 1) / P64_BLOCK;
-    const ll items = nib * ((jend - jbase + P64_JS - 1) / P64_JS);
-    double *tx = T, *ty = T + jc * cap, *tz = T + 2 * jc * cap;
-    for (ll w = blockIdx.x; w < items; w += gridDim.x) {
-        const ll i = (w % nib) * P64_BLOCK + threadIdx.x;
-        const ll j0 = jbase + (w / nib) * P64_JS;
-        const ll jl = j0 + threadIdx.x;
-        __syncthreads(); /* the previous item's readers are done */
-        if (threadIdx.x < P64_JS && jl < jend) {
-            sx[threadIdx.x] = A.x[jl];
-            sy[threadIdx.x] = A.y[jl];
-            sz[threadIdx.x] = A.z[jl];
-            sm[threadIdx.x] = A.m[jl];
-            sr[threadIdx.x] = A.rad[jl];
-            sf[threadIdx.x] = A.flags[jl];
-        }
-        __syncthreads();
-        if (i >= n) continue;
-        const double xi = A.x[i], yi = A.y[i], zi = A.z[i], mi = A.m[i], ri = A.rad[i];
-        const unsigned fi = A.flags[i];
-        const bool live_i = (fi & NBG_LIVE_MASK) == NBG_F_EXISTS;
-        const bool coll_i = (fi & NBG_F_COLLIDED) != 0;
-        const unsigned bi = NBG_BEHAVIOR(fi);
-        const double gmi = NBG_G * mi;
-        const int cnt = (jend - j0) < P64_JS ? (int)(jend - j0) : P64_JS;
-        for (int t = 0; t < cnt; t++) {
-            const ll j = j0 + t;
-            const ll slot = (j - jbase) * cap + i; /* a warp's stores are contiguous */
-            double ex = 0.0, ey = 0.0, ez = 0.0;
-            if (live_i) {
-                const double dx = sx[t] - xi;
-                const double dy = sy[t] - yi;
-                const double dz = sz[t] - zi;
-                const double dist = sqrt(dx * dx + dy * dy + dz * dz);
-                const double rr = ri + sr[t];
-                const unsigned fj = sf[t];
-                const bool live_j = (fj & NBG_LIVE_MASK) == NBG_F_EXISTS;
-                if (live_j && j != i && (coll_i || dist > rr)) {
-                    const double force = gmi * sm[t] / (dist * dist);
-                    ex = force * dx / dist;
-                    ey = force * dy / dist;
-                    ez = force * dz / dist;
-                }
-                if (!coll_i && dist <= rr && j != i) {
-                    const int type = nbg_detect_event(bi, NBG_BEHAVIOR(fj), ri, sr[t], dist);
-                    if (type >= 0) nbg_emit_event(ctl, ev_keys, ev_cap, i, j, type);
-                }
-            }
-            tx[slot] = ex;
-            ty[slot] = ey;
-            tz[slot] = ez;
-        }
-    }
+    const int h = __double2hiint(r);
+    if (r != r || h >= 0x7fe00000) return 0x7fffffff;
+    return h < 0 ? h : h + 0x100000;
 }
 
-/* Each body adds its terms in j order.  A block takes 32 bodies: all its
- * threads load a tile of 32 j x 32 bodies x 3 components (coalesced rows of
- * 32 bodies), the next tile's loads go out while this one is added, and
- * three warps add the columns in j order, one force component each (FP64
- * adds run at 1/64 of the FP32 rate, so one warp adding all three left most
- * of the SM's FP64 units idle).  Each component's sum is formed exactly as
- * the sequential loop forms it. */
-#define SUM_BODIES 32
-#define SUM_J 32
-#define SUM_THREADS 256
-#define SUM_PER_THREAD (3 * SUM_J * SUM_BODIES / SUM_THREADS)
-__global__ void __launch_bounds__(SUM_THREADS, 4) k_p64_sum(BodyArrays A, DevCtl *ctl, const double *T, double *acc,
-                                                         ll cap, ll jc, ll jbase)
+/* beside a body's flags: it is not live, or its mass (or G times it) is not
+ * in nbg_exact.h's range */
+#define P64_ODD 0x10000u
+__device__ __forceinline__ unsigned p64_flags(unsigned f, double m)
 {
-    __shared__ double tile[3][SUM_J][SUM_BODIES];
+    return (f & 0xffffu) | ((f & NBG_LIVE_MASK) == NBG_F_EXISTS && nbx_mass_ok(nbx_bits(m)) ? 0u : P64_ODD);
+}
+
+/* One CTA takes a block of up to 32 bodies i of one collection and walks its
+ * j in tiles.  Eight warps compute the pair terms of a tile, up to 1,536
+ * (i, j), into shared memory; up to three more warps, a lane for each force
+ * component of each body, add the tile before it, each body's terms in j
+ * order.  So every expression and every addition is the reference's
+ * sequential one (the file is compiled with --fmad=false), while a collection
+ * of any size fills the chip: the block is cut so that every resident CTA
+ * gets the same number of bodies.
+ *
+ * Bound by the FP64 pipe and the integer pipes together.  The pipe takes
+ * 11.6 operations a pair (differences 3, squared distance 5, sums 3 in three
+ * warps of 27 lanes for 16,384 bodies) of 19 cycles per SM each, 220 cycles a
+ * warp of pairs; the root, four quotients and four products run beside it on
+ * integers (nbg_exact.h), some 650 issue cycles a scheduler, 190 a pair warp
+ * and SM.  Leaving more products to the pipe, or none of the squares, measured
+ * 1-8 % slower.  16,384 Plummer bodies 28.9 -> 9.0 ms a pass, where the
+ * compiler's expansion of the root and the divisions kept the FP64 pipe 90 %
+ * busy with 68 operations a pair; terms stay on the chip, where storing them
+ * all took 48 bytes of traffic a pair and 3.2 GB at 65,536 bodies.  A body's
+ * sum is one chain of n dependent additions of 64 cycles at least: that is
+ * what a collection of a thousand bodies waits for (174 -> 79 us).  Tiles of
+ * 512 pairs, with a barrier three times as often, measured 11.1 ms. */
+#define P64_PROD 256
+#define P64_THREADS (P64_PROD + 96)
+#define P64_PAIRS (6 * P64_PROD) /* most pairs of a tile */
+#define P64_IB 32                /* most bodies of a block */
+#define P64_JT 192               /* most j of a tile */
+#define P64_MINB 2               /* CTAs per SM */
+static_assert(P64_JT <= P64_PROD, "a tile's j are loaded one per producer");
+static_assert(P64_PAIRS <= 2048, "the reciprocal of ib is exact below 2048");
+static_assert(P64_THREADS - P64_PROD >= 3 * P64_IB, "an adder for every component of a block");
+struct P64Shared {
+    double term[2][3][P64_PAIRS];
+    double jx[2][P64_JT], jy[2][P64_JT], jz[2][P64_JT], jm[2][P64_JT], jr[2][P64_JT];
+    double sx[P64_IB], sy[P64_IB], sz[P64_IB], sg[P64_IB], sr[P64_IB];
+    ll blk;
+    unsigned jf[2][P64_JT], sf[P64_IB];
+    int jb[2][P64_JT], sb[P64_IB];
+};
+__global__ void __launch_bounds__(P64_THREADS, P64_MINB) k_pair_fp64(BodyArrays A, DevCtl *ctl, SimSegs seg, ull *ev_keys,
+                                                              ll ev_cap)
+{
+    extern __shared__ double p64_smem[];
+    P64Shared &S = *(P64Shared *)p64_smem;
+    auto &term = S.term;
+    auto &jx = S.jx, &jy = S.jy, &jz = S.jz, &jm = S.jm, &jr = S.jr;
+    auto &jf = S.jf;
+    auto &jb = S.jb;
+    auto &sx = S.sx, &sy = S.sy, &sz = S.sz, &sg = S.sg, &sr = S.sr;
+    auto &sf = S.sf;
+    auto &sb = S.sb;
+    ll &s_blk = S.blk;
     if (ctl->error) return;
-    const ll n = ctl->n;
-    if (jbase >= n && jbase > 0) return;
-    const ll je = jbase + jc < n ? jbase + jc : n;
-    const ll cnt = je - jbase;
     const int tid = threadIdx.x;
-    const int comp = tid / SUM_BODIES; /* warps 0-2: the component this thread adds */
+    const bool producer = tid < P64_PROD;
+    const int ns = seg.nsims;
+    /* bodies of a block.  One collection: even shares of the resident CTAs'
+     * waves.  Several: 4 to 32, a divisor of the 64-body tiles the layout
+     * counts, small enough for four blocks a CTA. */
+    int ib;
+    ll blocks;
+    if (ns == 1) {
+        const ll n = ctl->n;
+        const ll waves = (n + (ll)P64_IB * gridDim.x - 1) / ((ll)P64_IB * gridDim.x);
+        ib = waves > 0 ? (int)((n + waves * gridDim.x - 1) / (waves * gridDim.x)) : 1;
+        if (ib < 4) ib = 4;
+        blocks = (n + ib - 1) / ib;
+    } else {
+        const ll tiles = seg.tile_off[ns];
+        ib = P64_IB;
+        while (ib > 4 && tiles * (64 / ib) < 4ll * gridDim.x) ib >>= 1;
+        blocks = tiles * (64 / ib);
+    }
+    const int jt = P64_PAIRS / ib < P64_JT ? P64_PAIRS / ib : P64_JT; /* j of a tile */
+    const unsigned rib = ((1u << 20) + (unsigned)ib - 1u) / (unsigned)ib; /* p / ib = p rib >> 20 for p < 2048 */
+    /* the adders: 3 ib threads in a row, one for each component of each body */
+    const int comp = producer ? 3 : (tid - P64_PROD) / ib, lane = tid - P64_PROD - comp * ib;
     const bool adder = comp < 3;
-    for (ll i0 = (ll)blockIdx.x * SUM_BODIES; i0 < n; i0 += (ll)gridDim.x * SUM_BODIES) {
-        const ll i = i0 + (tid & (SUM_BODIES - 1));
-        double f = 0.0;
-        if (adder && jbase > 0 && i < n) f = acc[(ll)comp * cap + i];
-        /* element e of a tile: component e / 1024, row (e / 32) % 32, body e % 32 */
-        double r[SUM_PER_THREAD];
-        auto load = [&](ll jt) {
-#pragma unroll
-            for (int q = 0; q < SUM_PER_THREAD; q++) {
-                const int e = tid + q * SUM_THREADS;
-                const int c = e / (SUM_J * SUM_BODIES), row = (e / SUM_BODIES) % SUM_J, b = e % SUM_BODIES;
-                const ll j = jt + row, ib = i0 + b;
-                r[q] = (j < cnt && ib < n) ? T[(ll)c * jc * cap + j * cap + ib] : 0.0;
+    for (;;) {
+        if (tid == 0) s_blk = (ll)atomicAdd((unsigned long long *)&ctl->work_next, 1ull);
+        __syncthreads();
+        const ll B = s_blk;
+        if (B >= blocks) break;
+        ll s0, n, ibase;
+        if (ns == 1) {
+            s0 = 0;
+            n = ctl->n;
+            ibase = B * ib;
+        } else {
+            const int per = 64 / ib;
+            const ll T = B / per;
+            const int sim = nbg_sim_of(seg.tile_off, ns, T);
+            s0 = seg.off[sim];
+            n = seg.off[sim + 1];
+            ibase = s0 + (T - seg.tile_off[sim]) * 64 + (B - T * per) * ib;
+        }
+        if (tid < ib) {
+            const ll i = ibase + tid;
+            const bool valid = i < n;
+            sx[tid] = valid ? A.x[i] : 0.0;
+            sy[tid] = valid ? A.y[i] : 0.0;
+            sz[tid] = valid ? A.z[i] : 0.0;
+            sg[tid] = valid ? NBG_G * A.m[i] : 0.0;
+            sr[tid] = valid ? A.rad[i] : 0.0;
+            sf[tid] = valid ? p64_flags(A.flags[i], sg[tid]) : P64_ODD;
+            sb[tid] = valid ? p64_radius_bound(A.rad[i]) : 0;
+        }
+        auto load_j = [&](ll jbase, int buf) {
+            const ll j = jbase + tid;
+            if (tid < jt && j >= n) {
+                jf[buf][tid] = P64_ODD; /* past the end: neither live nor near */
+                jx[buf][tid] = jy[buf][tid] = jz[buf][tid] = jm[buf][tid] = 0.0;
+                jr[buf][tid] = __longlong_as_double(0x7ff8000000000000ll);
+            } else if (tid < jt) {
+                jx[buf][tid] = A.x[j];
+                jy[buf][tid] = A.y[j];
+                jz[buf][tid] = A.z[j];
+                jm[buf][tid] = A.m[j];
+                const double r = A.rad[j];
+                jr[buf][tid] = r;
+                jb[buf][tid] = p64_radius_bound(r);
+                jf[buf][tid] = p64_flags(A.flags[j], jm[buf][tid]);
             }
         };
-        load(0);
-        for (ll jt = 0; jt < cnt; jt += SUM_J) {
-            __syncthreads(); /* the previous tile is added */
-#pragma unroll
-            for (int q = 0; q < SUM_PER_THREAD; q++) {
-                const int e = tid + q * SUM_THREADS;
-                tile[e / (SUM_J * SUM_BODIES)][(e / SUM_BODIES) % SUM_J][e % SUM_BODIES] = r[q];
+        /* The straight path: no branch, so that a thread's pairs overlap.
+         * Returns whether it holds; if not, the term is meaningless. */
+        auto core = [&](int ii, int jj, int buf, double &ex, double &ey, double &ez) -> bool {
+            const double dx = jx[buf][jj] - sx[ii];
+            const double dy = jy[buf][jj] - sy[ii];
+            const double dz = jz[buf][jj] - sz[ii];
+            const uint64_t bx = nbx_bits(dx), by = nbx_bits(dy), bz = nbx_bits(dz);
+            const double s = dx * dx + dy * dy + dz * dz;
+            const nbx_root root = nbx_sqrt(nbx_bits(s));
+            const nbx_div &r = root.r;
+            const int bound = sb[ii] > jb[buf][jj] ? sb[ii] : jb[buf][jj];
+            const nbx_num gm = nbx_mul(nbx_unpack(nbx_bits(sg[ii])), nbx_unpack(nbx_bits(jm[buf][jj])));
+            const nbx_num f = nbx_quot(gm, nbx_square(root));
+            const nbx_num ax = nbx_mul(f, nbx_unpack(bx)), ay = nbx_mul(f, nbx_unpack(by)),
+                          az = nbx_mul(f, nbx_unpack(bz));
+            ex = (bx << 1) == 0 ? 0.0 : nbx_double(nbx_pack(nbx_quot(ax, r)));
+            ey = (by << 1) == 0 ? 0.0 : nbx_double(nbx_pack(nbx_quot(ay, r)));
+            ez = (bz << 1) == 0 ? 0.0 : nbx_double(nbx_pack(nbx_quot(az, r)));
+            return nbx_diff_ok(bx) && nbx_diff_ok(by) && nbx_diff_ok(bz) && ((bx | by | bz) << 1) != 0 &&
+                   nbx_square_ok(root) && (int)(nbx_div_bits(r) >> 32) > bound;
+        };
+        auto plain = [&](int ii, int jj, ll jbase, int buf, double &ex, double &ey, double &ez) {
+            p64_pair_plain(ctl, ev_keys, ev_cap, ibase + ii, jbase + jj, sf[ii], jf[buf][jj], jx[buf][jj] - sx[ii],
+                           jy[buf][jj] - sy[ii], jz[buf][jj] - sz[ii], sg[ii], jm[buf][jj], sr[ii], jr[buf][jj], ex, ey,
+                           ez);
+        };
+        double f = 0.0;
+        auto add = [&](ll jbase, int buf) {
+            if (adder) {
+                const int cnt = n - jbase < jt ? (int)(n - jbase) : jt;
+                const double *q = &term[buf][comp][lane];
+#pragma unroll 8
+                for (int t = 0; t < cnt; t++) f += q[t * ib];
+            }
+        };
+        if (producer) load_j(s0, 0);
+        __syncthreads();
+        int buf = 0;
+        for (ll jbase = s0; jbase < n; jbase += jt, buf ^= 1) {
+            if (producer) {
+                if (jbase + jt < n) load_j(jbase + jt, buf ^ 1);
+                /* pair p of the tile: body p % ib, j p / ib */
+                const int np = ib * jt;
+#pragma unroll 1
+                for (int p = tid; p < np; p += P64_PROD) {
+                    const int jj = (int)(((unsigned)p * rib) >> 20), ii = p - jj * ib;
+                    double ex, ey, ez;
+                    const bool ok = core(ii, jj, buf, ex, ey, ez);
+                    if (!ok || ((sf[ii] | jf[buf][jj]) & P64_ODD)) plain(ii, jj, jbase, buf, ex, ey, ez);
+                    term[buf][0][p] = ex;
+                    term[buf][1][p] = ey;
+                    term[buf][2][p] = ez;
+                }
+            } else if (jbase > s0) {
+                add(jbase - jt, buf ^ 1);
             }
             __syncthreads();
-            if (jt + SUM_J < cnt) load(jt + SUM_J);
-            if (adder) {
-                const int m = cnt - jt < SUM_J ? (int)(cnt - jt) : SUM_J;
-                const int b = tid & (SUM_BODIES - 1);
-                for (int t = 0; t < m; t++) f += tile[comp][t][b];
-            }
         }
-        if (adder && i < n) {
-            if (je >= n) {
-                if ((A.flags[i] & NBG_LIVE_MASK) == NBG_F_EXISTS) (comp == 0 ? A.fx : comp == 1 ? A.fy : A.fz)[i] = f;
-            } else {
-                acc[(ll)comp * cap + i] = f;
-            }
+        if (!producer && n > s0) {
+            const ll last = s0 + (n - s0 - 1) / jt * jt;
+            add(last, buf ^ 1);
+            const ll i = ibase + lane;
+            if (adder && i < n && (sf[lane] & NBG_LIVE_MASK) == NBG_F_EXISTS)
+                (comp == 0 ? A.fx : comp == 1 ? A.fy : A.fz)[i] = f;
         }
-        __syncthreads(); /* the tile is free for the next bodies */
+        __syncthreads(); /* the block's shared data and s_blk are rewritten next */
     }
 }
 
@@ -1483,42 +1489,14 @@ void nbg_launch_frag_count(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     k_scan_blocks<<<1, NBG_SCAN_BLOCK, 0, st>>>(ctl, cb.seg, cb.blk_sum, cb.blk_off, 0, cb.cap, cb.frag_cap);
 }
 
-int nbg_pair_fp64_grid(ll cap)
-{
-    ll g = (cap + P64_BLOCK - 1) / P64_BLOCK;
-    return (int)(g < 1 ? 1 : (g > 65535 ? 65535 : g));
-}
-
 void nbg_launch_pair_fp64(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 {
-    if (cb.p64_terms && cb.seg.nsims == 1) {
-        const ll jc = cb.p64_jc;
-        /* a grid-stride loop over the live bodies' work items: at most 32
-         * blocks of two warps per SM, fewer when the capacity is small */
-        const int js = cb.cap <= 8192 ? 4 : 16;
-        const ll want = ((cb.cap + P64_BLOCK - 1) / P64_BLOCK) * ((jc + js - 1) / js);
-        const ll most = (ll)(cb.sms > 0 ? cb.sms : 1) * 32;
-        const unsigned g = (unsigned)(want < most ? want : most);
-        for (ll jbase = 0; jbase < cb.cap; jbase += jc) {
-            if (js == 4)
-                k_p64_terms<4><<<g, P64_BLOCK, 0, st>>>(cb.a, ctl, cb.p64_terms, cb.cap, jc, jbase, cb.ev_keys,
-                                                         cb.ev_cap);
-            else
-                k_p64_terms<16><<<g, P64_BLOCK, 0, st>>>(cb.a, ctl, cb.p64_terms, cb.cap, jc, jbase, cb.ev_keys,
-                                                          cb.ev_cap);
-            /* 32 bodies per block, at most 8 blocks per SM */
-            const ll sb = (cb.cap + SUM_BODIES - 1) / SUM_BODIES, smost = (ll)(cb.sms > 0 ? cb.sms : 1) * 8;
-            k_p64_sum<<<(unsigned)(sb < smost ? sb : smost), SUM_THREADS, 0, st>>>(cb.a, ctl, cb.p64_terms,
-                                                                                  cb.p64_acc, cb.cap, jc, jbase);
-        }
-        return;
-    }
-    k_pair_fp64<<<nbg_pair_fp64_grid(cb.cap), P64_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.ev_keys, cb.ev_cap);
-}
-
-int nbg_pair_fp64_launches(const CycleBufs &cb)
-{
-    return cb.p64_terms && cb.seg.nsims == 1 ? (int)(2 * ((cb.cap + cb.p64_jc - 1) / cb.p64_jc)) : 1;
+    /* one wave of resident CTAs, which take blocks of bodies from a counter */
+    const ll sms = cb.sms > 0 ? cb.sms : 1;
+    const ll most = (cb.cap + 3) / 4 + cb.seg.nsims;
+    cudaFuncSetAttribute(k_pair_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P64Shared));
+    k_pair_fp64<<<(unsigned)(most < P64_MINB * sms ? most : P64_MINB * sms), P64_THREADS, sizeof(P64Shared), st>>>(
+        cb.a, ctl, cb.seg, cb.ev_keys, cb.ev_cap);
 }
 
 /* everything after the pair kernel: order events, emit fragments, resolve,

@@ -79,7 +79,6 @@ struct nbg_ctx {
     size_t scratch_bytes = 0;
     ll launches_per_cycle = 0;
     ll bh_cap = 0; /* capacity the Barnes-Hut buffers were sized for */
-    ll p64_split_max = NBG_P64_SPLIT_MAX_CAP; /* plain form: split pair pass up to this capacity */
     void *ring_host = nullptr; /* the caller's render ring, registered here */
     void *seg_mem = nullptr; /* SimSegs arrays */
     int seg_cap = 0;         /* sims the allocation holds */
@@ -401,39 +400,6 @@ static int ensure_part(nbg_ctx *ctx, ll need)
 }
 
 /* Barnes-Hut buffers for the current capacity and at least `nodes` nodes */
-/* The plain form's split pair pass (k_p64_terms + k_p64_sum) serves one
- * collection of capacity up to p64_split_max: one thread per body would leave
- * the FP64 pipes idle below some 64 thousand bodies.  Its term buffer (3 x
- * 2048 x capacity doubles) is allocated by the first FP64 pass that wants it
- * and freed when the form, the collection count or the capacity no longer
- * do.  If it cannot be allocated, the one-thread-per-body kernel runs: the
- * two give identical results. */
-static int ensure_p64(nbg_ctx *ctx)
-{
-    CycleBufs &cb = ctx->cb;
-    const bool want = ctx->precision == NBG_PRECISION_FP64 && cb.seg.nsims == 1 && !cb.bh && cb.cap > 0 &&
-                      cb.cap <= ctx->p64_split_max;
-    const ll jc = cb.cap < NBG_P64_SPLIT_JC ? cb.cap : NBG_P64_SPLIT_JC;
-    if (want == (cb.p64_terms != nullptr) && (!want || cb.p64_jc == jc)) return NBG_OK;
-    CK(cudaStreamSynchronize(ctx->st));
-    cudaFree(cb.p64_terms);
-    cudaFree(cb.p64_acc);
-    cb.p64_terms = cb.p64_acc = nullptr;
-    cb.p64_jc = 0;
-    invalidate_graph(ctx);
-    if (!want) return NBG_OK;
-    if (cudaMalloc((void **)&cb.p64_terms, (size_t)3 * jc * cb.cap * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void **)&cb.p64_acc, (size_t)3 * cb.cap * sizeof(double)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(cb.p64_terms);
-        cb.p64_terms = nullptr;
-        cb.p64_acc = nullptr;
-        return NBG_OK;
-    }
-    cb.p64_jc = jc;
-    return NBG_OK;
-}
-
 static int ensure_bh(nbg_ctx *ctx, ll nodes)
 {
     BhTree &t = ctx->cb.t;
@@ -455,10 +421,6 @@ static void free_cap_buffers(CycleBufs &cb)
     cudaFree(cb.tile_c);
     cudaFree(cb.tile_t);
     cudaFree(cb.iprep);
-    cudaFree(cb.p64_terms);
-    cudaFree(cb.p64_acc);
-    cb.p64_terms = cb.p64_acc = nullptr;
-    cb.p64_jc = 0;
     cudaFree(cb.part);
     cudaFree(cb.perm);
     cudaFree(cb.sval);
@@ -1597,7 +1559,7 @@ static void launch_cycle(nbg_ctx *ctx, int precision, long ev_base)
      * compaction; Barnes-Hut replaces the pair kernel (nbg_bh_launches) */
     ctx->launches_per_cycle = (cb.ev_radix ? nbg_event_radix_launches(cb) : 0) +
                               (cb.bh ? 13 + nbg_bh_launches(cb, precision == NBG_PRECISION_MIXED)
-                                     : precision == NBG_PRECISION_MIXED ? 45 : 13 + nbg_pair_fp64_launches(cb)) +
+                                     : precision == NBG_PRECISION_MIXED ? 45 : 14) +
                               (cb.ring_head ? 1 : 0);
 }
 
@@ -1701,7 +1663,6 @@ int nbg_step(nbg_ctx *ctx, double dt, double R, int nsteps, nbg_step_info *info)
          * none, and the cycle's kernels write the per-sim event ranges) */
         if ((rc = ensure_ev_cap(ctx, 1)) != NBG_OK) return rc;
         if (ctx->cb.bh && (rc = ensure_bh(ctx, 0)) != NBG_OK) return rc; /* likewise the octree's */
-        if ((rc = ensure_p64(ctx)) != NBG_OK) return rc;
         const int todo = nsteps - done;
         if (ctx->timing || !ctx->use_graph || todo < ctx->graph_cycles || todo == 1) {
             for (int s = 0; s < todo; s++) {
@@ -1825,9 +1786,8 @@ int nbg_force_pass(nbg_ctx *ctx)
     if (ctx->cb.seg.nsims < 1) return fail(ctx, NBG_E_STATE, "no collection is loaded (a segment allocation failed)");
     CK(cudaSetDevice(ctx->device));
     {
-        int rc = ensure_p64(ctx);
-        if (rc != NBG_OK) return rc;
         /* the octree's buffers exist (a failed allocation leaves none) */
+        int rc;
         if (ctx->cb.bh && (rc = ensure_bh(ctx, 0)) != NBG_OK) return rc;
     }
     for (int attempt = 0;; attempt++) {
@@ -2170,8 +2130,7 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value)
         return NBG_OK;
     case NBG_OPT_P64_SPLIT_MAX:
         if (value < 0 || value > NBG_MAX_BODIES) return fail(ctx, NBG_E_ARG, "split limit must be 0..2^30");
-        ctx->p64_split_max = value;
-        return NBG_OK;
+        return NBG_OK; /* one pair pass serves every size */
     case NBG_OPT_SORT_INTERVAL: {
         if (value < 1 || value > 1000) return fail(ctx, NBG_E_ARG, "sort interval must be 1..1000 cycles");
         const int k = (int)value;

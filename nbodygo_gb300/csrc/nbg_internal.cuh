@@ -253,10 +253,6 @@ struct CycleBufs {
     nbg_renderable *ring_rend;
     ll ring_cap;
     int ring_slots;
-    /* plain form, small collections: pair terms (3 x p64_jc x cap) and the
-     * sums carried between passes (3 x cap); NULL when cap is too large */
-    double *p64_terms, *p64_acc;
-    ll p64_jc;
     int bh;             /* forces from the Barnes-Hut octree */
     int bh_shape;       /* register cap of the mixed walk: 0, 1, 2 = 4, 5, 6 CTAs per SM */
     int sms;            /* streaming multiprocessors of the device */
@@ -441,11 +437,6 @@ void nbg_launch_find(const CycleBufs &cb, DevCtl *ctl, int sim, ll id, ll *idx_d
 /* dst[k] = src[index[k]], k < n, every field (index on the device) */
 void nbg_launch_gather(const CycleBufs &cb, const BodyArrays &src, const BodyArrays &dst, const ll *index_dev, ll n,
                        cudaStream_t st);
-int nbg_pair_fp64_grid(ll cap);
-int nbg_pair_fp64_launches(const CycleBufs &cb);
-/* largest capacity the plain form stores its pair terms for */
-#define NBG_P64_SPLIT_MAX_CAP 65536
-#define NBG_P64_SPLIT_JC 2048
 
 /* k_mixed.cu */
 void nbg_launch_mixed_prep(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
