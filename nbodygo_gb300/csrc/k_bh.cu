@@ -57,6 +57,7 @@
  * query stay inside the body's own collection.  Walk groups of 32 bodies
  * start at each collection's first sorted position, as they would alone.
  */
+#include "nbg_exact.h"
 #include "nbg_internal.cuh"
 #include "nbg_math.h"
 #include "nbg_shared.h"
@@ -652,123 +653,28 @@ __device__ __forceinline__ void bh_term(double gm_i, double M, double dx, double
     fz += force * dz / dist;
 }
 
-/* The next group of 32 consecutive sorted bodies for this warp, or -1.  Walk
- * times vary with the bodies' surroundings, so warps take groups from one
- * queue until it is empty instead of a fixed share each: no SM idles while
- * another still holds a long run of groups.  A group is always the same 32
- * bodies, so the results do not depend on which warp takes it. */
-__device__ __forceinline__ int bh_next_group(DevCtl *ctl, ll groups)
+enum { BHW_DROP = 0, BHW_OPEN = 1, BHW_ACCEPT = 2, BHW_MIXED = 3, BHW_BUCKET = 4 };
+
+__device__ __forceinline__ float warp_minf(float v)
 {
-    unsigned g = 0;
-    if ((threadIdx.x & 31) == 0) g = atomicAdd(&ctl->bh_next, 1u);
-    g = __shfl_sync(FULL_MASK, g, 0);
-    return (ll)g < groups ? (int)g : -1;
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(FULL_MASK, v, o));
+    return v;
 }
 
-/* Group g holds sorted positions [p0, p1) of collection s: the groups of a
- * collection start at its first sorted position, 32 bodies each, so a
- * collection's groups are those it would have alone. */
-__device__ __forceinline__ void bh_group(const BhTree &t, int nsims, int g, int &s, ll &p0, ll &p1)
+/* exclusive prefix of v (0..15) over the lanes and the warp's total */
+__device__ __forceinline__ int warp_prefix4(int v, unsigned lt, int &total)
 {
-    s = nbg_sim_of(t.sgrp, nsims, g);
-    p0 = t.stree[s] + 32ll * (g - t.sgrp[s]);
-    p1 = p0 + 32 < t.stree[s + 1] ? p0 + 32 : t.stree[s + 1];
-}
-
-/* one thread per tree body (sorted order, so a warp walks nearby paths) */
-__global__ void __launch_bounds__(BH_BLOCK) k_bh_force(BodyArrays A, DevCtl *ctl, SimSegs seg, const unsigned *vals,
-                                                       BhTree t)
-{
-    if (ctl->error) return;
-    const ll groups = t.sgrp[seg.nsims];
-    unsigned long long terms = 0;
-    /* every lane runs the same number of rounds, for the warp reduction */
-    for (int grp; (grp = bh_next_group(ctl, groups)) >= 0;) {
-        int r;
-        ll p0, p1;
-        bh_group(t, seg.nsims, grp, r, p0, p1);
-        const ll p = p0 + (threadIdx.x & 31);
-        if (p >= p1) continue;
-        const int total = (int)t.sroot[r + 1]; /* the end of the collection's nodes */
-        const unsigned k = vals[p];
-        if (A.flags[k] & NBG_F_IS_SUN) continue; /* k_bh_sun */
-        const double x = A.x[k], y = A.y[k], z = A.z[k];
-        const double gm = NBG_G * A.m[k];
-        double fx = 0, fy = 0, fz = 0;
-        int id = (int)t.sroot[r];
-        while (id < total) {
-            const double Mn = t.mass[id];
-            if (Mn == 0) {
-                id = t.skip[id];
-                continue;
-            }
-            const unsigned fl = t.flags[id];
-            const bool leaf = (fl & BH_F_LEAF) != 0;
-            const double dx = t.cmx[id] - x;
-            const double dy = t.cmy[id] - y;
-            const double dz = t.cmz[id] - z;
-            const double distSq = dx * dx + dy * dy + dz * dz + BH_SOFTENING * BH_SOFTENING;
-            const double dist = sqrt(distSq);
-            if (leaf || (!(fl & BH_F_NAN_CM) && (2 * t.half[id] / dist) < BH_THETA)) {
-                const int s = t.start[id], e = t.end[id];
-                if (leaf && e - s > 1) {
-                    /* a leaf at the deepest level holding several bodies: each
-                     * acts as a leaf of its own */
-                    for (int q = s; q < e; q++) {
-                        const unsigned j = vals[q];
-                        const double mj = A.m[j];
-                        if (j == k || mj == 0) continue;
-                        bh_term(gm, mj, A.x[j] * mj / mj - x, A.y[j] * mj / mj - y, A.z[j] * mj / mj - z, fx, fy,
-                                fz);
-                        terms++;
-                    }
-                } else if (!(leaf && vals[s] == k)) {
-                    const double force = gm * Mn / distSq;
-                    fx += force * dx / dist;
-                    fy += force * dy / dist;
-                    fz += force * dz / dist;
-                    terms++;
-                }
-                id = t.skip[id];
-            } else {
-                id = id + 1;
-            }
-        }
-        A.fx[k] = fx;
-        A.fy[k] = fy;
-        A.fz[k] = fz;
+    int x = 0;
+    total = 0;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        const unsigned m = __ballot_sync(FULL_MASK, (v >> b) & 1);
+        x += __popc(m & lt) << b;
+        total += __popc(m) << b;
     }
-    /* point-mass terms summed, for the measured work */
-    for (int o = 16; o > 0; o >>= 1) terms += __shfl_xor_sync(FULL_MASK, terms, o);
-    if ((threadIdx.x & 31) == 0 && terms) atomicAdd((unsigned long long *)&ctl->acc_bh_terms, terms);
+    return x;
 }
 
-/* ---- 5b. the mixed-precision walk --------------------------------------------
- * The same tree and the same acceptance rule in FP32: centres of mass as
- * hi/lo float pairs (so dx = (cm_hi - x_hi) + (cm_lo - x_lo) keeps ~2^-24 of
- * |dx|), masses relative to the root's, the opening test as
- * r^2 > (2 half / theta)^2 on the softened r^2, and the reciprocal square
- * root of the SFU.
- *
- * A group of 32 bodies (neighbours in key order, one per lane) walks the tree
- * together.  The warp keeps a stack of nodes, each with the lanes that have
- * not accepted an ancestor of it, and visits 32 of them at once, one per
- * lane: most nodes lie so far from the group's box (or so close) that all
- * its bodies accept (or open) them, which one bound decides; accepted nodes
- * are listed in shared memory and summed 32 or more at a time, every lane
- * its own body, two nodes per packed instruction.  Only the nodes in between
- * (1,100 of the 7,900 that a group of a 131,072-body Plummer sphere accepts)
- * take each body's own test, with the same expression and rounding as a walk
- * of that body alone, so every body sums the terms it would alone.  Sums are
- * FP32, folded into (hi, lo) pairs after every list: the GB300 FP64 pipe is
- * 1/64 of the FP32 rate.
- *
- * A walk that took one node at a time for the whole warp was bound by the
- * latency of its node loads (issue slots 25 % busy).  The walk of a 131,072-
- * body Plummer sphere went from 5.0 to 1.56 ms, of 10^6 uniform bodies from
- * 20.3 to 7.3 ms.  What bounds it now is issue and, with a group to a warp,
- * groups of uneven cost: 263,000 instructions a group before the lists were
- * split into far and near ones, 60 % of them in the sums. */
 /* Where the walk finds a node: the children of a node take consecutive
  * slots, so a visit that opens it goes on with one address and a count.
  * Slots 0 .. nsims - 1 are the roots'; the others are handed out a warp of
@@ -816,6 +722,389 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_children(DevCtl *ctl, SimSegs s
         if (t.sroot[s] < t.sroot[s + 1]) t.slot[t.sroot[s]] = s;
 }
 
+/* Group g holds sorted positions [p0, p1) of collection s: the groups of a
+ * collection start at its first sorted position, 32 bodies each, so a
+ * collection's groups are those it would have alone. */
+__device__ __forceinline__ void bh_group(const BhTree &t, int nsims, int g, int &s, ll &p0, ll &p1)
+{
+    s = nbg_sim_of(t.sgrp, nsims, g);
+    p0 = t.stree[s] + 32ll * (g - t.sgrp[s]);
+    p1 = p0 + 32 < t.stree[s + 1] ? p0 + 32 : t.stree[s + 1];
+}
+
+/* every node's records for the FP64 walk, in its slot: centre of mass as hi/lo
+ * floats with the squared opening distance (zero when out of FP32's range:
+ * then the bodies decide in FP64), and centre, mass and half size as doubles */
+#define BH_F_EMPTY 4u /* no mass below */
+__global__ void __launch_bounds__(BH_BLOCK) k_bh_prep64(DevCtl *ctl, BhTree t)
+{
+    if (ctl->error) return;
+    const ll total = ctl->bh_nodes;
+    for (ll id = (ll)blockIdx.x * blockDim.x + threadIdx.x; id < total; id += (ll)gridDim.x * blockDim.x) {
+        const int slot = t.slot[id];
+        const double M = t.mass[id], half = t.half[id];
+        double cx = 0.0, cy = 0.0, cz = 0.0;
+        if (M != 0) {
+            cx = t.cmx[id];
+            cy = t.cmy[id];
+            cz = t.cmz[id];
+        }
+        const float hx = (float)cx, hy = (float)cy, hz = (float)cz;
+        const double o = 2 * half / BH_THETA, o2 = o * o;
+        t.fa[slot] = make_float4(hx, hy, hz, o2 > 1e-30 && o2 < 1e37 ? (float)o2 : 0.f);
+        t.fb[slot] = make_float4((float)(cx - (double)hx), (float)(cy - (double)hy), (float)(cz - (double)hz), 0.f);
+        t.fc[slot] = make_int4(t.cbase[id],
+                               (int)t.ccount[id] | ((int)(t.flags[id] | (M == 0 ? BH_F_EMPTY : 0u)) << 8),
+                               t.start[id], t.end[id]);
+        t.rec[2 * (ll)slot] = make_double2(cx, cy);
+        t.rec[2 * (ll)slot + 1] = make_double2(cz, M);
+        t.shalf[slot] = half;
+    }
+}
+
+/* a node of mass M at (dx, dy, dz) from the body, s the softened squared
+ * distance: the term with the ordinary operators */
+__device__ __noinline__ void bh_term_plain(double gm, double M, double dx, double dy, double dz, double s, double &ex,
+                                           double &ey, double &ez)
+{
+    const double dist = sqrt(s);
+    const double force = gm * M / s;
+    ex = force * dx / dist;
+    ey = force * dy / dist;
+    ez = force * dz / dist;
+}
+
+/* the bodies of a leaf at the deepest level, each a leaf of its own */
+__device__ __noinline__ int bh_bucket64(const BodyArrays &A, const unsigned *vals, int s, int e, unsigned k, double x,
+                                        double y, double z, double gm, double &fx, double &fy, double &fz)
+{
+    int cnt = 0;
+    for (int q = s; q < e; q++) {
+        const unsigned j = vals[q];
+        const double mj = A.m[j];
+        if (j == k || mj == 0) continue;
+        bh_term(gm, mj, A.x[j] * mj / mj - x, A.y[j] * mj / mj - y, A.z[j] * mj / mj - z, fx, fy, fz);
+        cnt++;
+    }
+    return cnt;
+}
+
+#define B64_STACK 256
+#define B64_SPARE 32
+#define B64_LIST 32
+struct alignas(16) Bh64Warp {
+    uint2 stack[B64_STACK]; /* runs of siblings: (first slot, the lanes that have not accepted an ancestor) */
+    double x[B64_LIST], y[B64_LIST], z[B64_LIST], m[B64_LIST]; /* accepted nodes waiting to be summed */
+    unsigned mask[B64_LIST];
+    unsigned char run[B64_STACK];
+};
+
+/* The reference's opening test of one body and node. */
+__device__ __noinline__ bool bh_accepts(double dx, double dy, double dz, double half)
+{
+    const double dist = sqrt(dx * dx + dy * dy + dz * dz + BH_SOFTENING * BH_SOFTENING);
+    return 2 * half / dist < BH_THETA;
+}
+
+/* The FP64 walk.  A CTA's four warps take a group of 32 bodies, one body a
+ * lane, and walk the tree as the mixed walk does (below): 32 nodes at a time
+ * are tested against the group's box in FP32, and nodes the box straddles
+ * against each body.  The FP32 tests decide all but the bodies within a part
+ * in 2^18 of a node's opening distance, which take the reference's test in
+ * FP64.  Every warp makes the whole walk; accepted nodes go to the four in
+ * turn, and each adds its own with the reference's expressions, one node at a
+ * time, every lane its body: root, quotients and products on the integer
+ * pipes, correctly rounded (nbg_exact.h).  A body's terms are those of a walk
+ * of its own, summed in the group's order.
+ *
+ * A thread walking alone spent its time on the FP64 pipe, 85 operations a
+ * term with the compiler's root and divisions, and on the walks of its warp's
+ * other lanes; now a term takes 12 operations of 19 cycles, with 160 cycles of
+ * integer issue beside them.  Tree pass: 2,000 Plummer bodies 8.9 -> 1.24 ms,
+ * 30,011 bodies 29.3 -> 7.0 ms, 131,072 bodies 133 -> 28.9 ms.  Dealing runs
+ * of nodes to the warps, as the mixed walk does, left one warp most of the
+ * near nodes, and so most of the time (19.9 ms at 30,011 bodies); conversions
+ * between FP64 and FP32 run on the FP64 pipe too, so the records hold both
+ * (13.9 ms when the walk converted them). */
+__global__ void __launch_bounds__(BHW_BLOCK, 5) k_bh_force(const __grid_constant__ BodyArrays A, DevCtl *ctl,
+                                                           SimSegs seg, const unsigned *vals,
+                                                           const __grid_constant__ BhTree t)
+{
+    __shared__ Bh64Warp ws[BHW_TEAM];
+    __shared__ double red[BHW_TEAM - 1][3][32];
+    __shared__ int s_grp;
+    if (ctl->error) return;
+    if (ctl->bh_nodes <= 0) return;
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    Bh64Warp &w = ws[wi];
+    const unsigned lt = (1u << lane) - 1u;
+    const ll groups = t.sgrp[seg.nsims];
+    const float soft2 = (float)(BH_SOFTENING * BH_SOFTENING);
+    unsigned long long all_terms = 0;
+    for (;;) {
+        if (threadIdx.x == 0) s_grp = (int)atomicAdd(&ctl->bh_next, 1u);
+        __syncthreads();
+        const int grp = s_grp;
+        __syncthreads();
+        if ((ll)grp >= groups) break;
+        int r;
+        ll p0, p1;
+        bh_group(t, seg.nsims, grp, r, p0, p1);
+        const ll p = p0 + lane;
+        unsigned k = 0;
+        bool have = p < p1;
+        if (have) {
+            k = vals[p];
+            have = !(A.flags[k] & NBG_F_IS_SUN); /* k_bh_sun */
+        }
+        const unsigned every = __ballot_sync(FULL_MASK, have);
+        if (!every) continue; /* the same in every warp */
+        const double bx = have ? A.x[k] : 0.0, by = have ? A.y[k] : 0.0, bz = have ? A.z[k] : 0.0;
+        const double gm = have ? NBG_G * A.m[k] : 0.0;
+        const nbx_num gmu = nbx_unpack(nbx_bits(gm));
+        const bool gm_ok = nbx_mass_ok(nbx_bits(gm));
+        /* the group's box in FP32, widened past every rounding, and the
+         * body's position as hi/lo floats for its own tests */
+        float gx, gy, gz, ex, ey, ez;
+        const float v[3] = {(float)bx, (float)by, (float)bz};
+        const float vl[3] = {(float)(bx - (double)v[0]), (float)(by - (double)v[1]), (float)(bz - (double)v[2])};
+        {
+            float g3[3], e3[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float lo = warp_minf(have ? v[c] : 3e38f), hi = -warp_minf(have ? -v[c] : 3e38f);
+                g3[c] = 0.5f * lo + 0.5f * hi;
+                e3[c] = fmaxf(hi - g3[c], g3[c] - lo) + 0x1p-20f * fmaxf(fabsf(lo), fabsf(hi));
+            }
+            gx = g3[0], gy = g3[1], gz = g3[2];
+            ex = e3[0], ey = e3[1], ez = e3[2];
+        }
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        unsigned terms = 0;
+        int cl = 0, top = 1;
+        unsigned turn = 0; /* nodes accepted so far; warp wi takes those with turn % BHW_TEAM == wi */
+        if (lane == 0) {
+            w.stack[0] = make_uint2((unsigned)r, every);
+            w.run[0] = 1;
+        }
+        __syncwarp();
+        /* the listed nodes' terms */
+        auto flush = [&]() {
+#pragma unroll 1
+            for (int q = 0; q < cl; q++) {
+                const double dx = w.x[q] - bx, dy = w.y[q] - by, dz = w.z[q] - bz;
+                const double M = w.m[q];
+                const bool mine = (w.mask[q] >> lane) & 1u;
+                const uint64_t ux = nbx_bits(dx), uy = nbx_bits(dy), uz = nbx_bits(dz);
+                const double s = dx * dx + dy * dy + dz * dz + BH_SOFTENING * BH_SOFTENING;
+                const nbx_root root = nbx_sqrt(nbx_bits(s));
+                const nbx_num f = nbx_quot(nbx_mul(gmu, nbx_unpack(nbx_bits(M))), nbx_operand(root));
+                double tx = nbx_zero(ux) ? 0.0 : nbx_double(nbx_pack(nbx_quot(nbx_mul(f, nbx_unpack(ux)), root.r)));
+                double ty = nbx_zero(uy) ? 0.0 : nbx_double(nbx_pack(nbx_quot(nbx_mul(f, nbx_unpack(uy)), root.r)));
+                double tz = nbx_zero(uz) ? 0.0 : nbx_double(nbx_pack(nbx_quot(nbx_mul(f, nbx_unpack(uz)), root.r)));
+                if (mine) {
+                    if (!(nbx_diff_ok(ux) && nbx_diff_ok(uy) && nbx_diff_ok(uz) && gm_ok && nbx_mass_ok(nbx_bits(M))))
+                        bh_term_plain(gm, M, dx, dy, dz, s, tx, ty, tz);
+                    fx += tx;
+                    fy += ty;
+                    fz += tz;
+                    terms++;
+                }
+            }
+            cl = 0;
+            __syncwarp();
+        };
+        while (top > 0) {
+            /* the next 32 nodes, as in the mixed walk */
+            int take = B64_STACK - B64_SPARE - top;
+            take = take > 32 ? 32 : take < 1 ? 1 : take;
+            int cls = BHW_DROP, nc = 0, s = 0, e = 0, cb = 0;
+            unsigned mask = 0;
+            unsigned slot = 0;
+            float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+            int4 nd = make_int4(0, 0, 0, 0);
+            {
+                uint2 en = make_uint2(0u, 0u);
+                int rn = 0;
+                if (lane < top) {
+                    en = w.stack[top - 1 - lane];
+                    rn = w.run[top - 1 - lane];
+                }
+                int tot;
+                const int x = warp_prefix4(rn, lt, tot);
+                if (take > tot) take = tot;
+                const unsigned mark = __reduce_or_sync(FULL_MASK, rn > 0 && x < take ? 1u << x : 0u);
+                const unsigned m = mark & (0xffffffffu >> (31 - lane));
+                const int from = __popc(m) - 1, off = lane - (31 - __clz(m));
+                slot = __shfl_sync(FULL_MASK, en.x, from) + (unsigned)off;
+                mask = __shfl_sync(FULL_MASK, en.y, from);
+                if (lane < take) {
+                    na = t.fa[slot];
+                    nb = t.fb[slot];
+                    nd = t.fc[slot];
+                }
+                if (x < take && x + rn > take) {
+                    w.stack[top - 1 - lane] = make_uint2(en.x + (unsigned)(take - x), en.y);
+                    w.run[top - 1 - lane] = (unsigned char)(x + rn - take);
+                }
+                top -= __popc(__ballot_sync(FULL_MASK, rn > 0 && x + rn <= take));
+            }
+            const float o2 = na.w; /* the opening distance squared */
+            if (lane < take) {
+                cb = nd.x;
+                nc = nd.y & 0xff;
+                s = nd.z;
+                e = nd.w;
+                const unsigned fl = (unsigned)nd.y >> 8;
+                if (fl & BH_F_EMPTY) {
+                    cls = BHW_DROP; /* nothing with mass below: skipped by every body */
+                } else if (fl & BH_F_LEAF) {
+                    cls = e - s > 1 ? BHW_BUCKET : BHW_ACCEPT;
+                    /* a one-body leaf holds sorted position s: not for itself */
+                    if (cls == BHW_ACCEPT && s >= p0 && s < p0 + 32) mask &= ~(1u << (int)(s - p0));
+                } else if (fl & BH_F_NAN_CM) {
+                    cls = BHW_OPEN;
+                } else {
+                    const float ux = fabsf(na.x - gx), uy = fabsf(na.y - gy), uz = fabsf(na.z - gz);
+                    const float mx = ex + 0x1p-20f * fabsf(na.x), my = ey + 0x1p-20f * fabsf(na.y);
+                    const float mz = ez + 0x1p-20f * fabsf(na.z);
+                    const float nx = fmaxf(ux - mx, 0.f), ny = fmaxf(uy - my, 0.f), nz = fmaxf(uz - mz, 0.f);
+                    const float qx = ux + mx, qy = uy + my, qz = uz + mz;
+                    const float rn = nx * nx + ny * ny + nz * nz, rf = qx * qx + qy * qy + qz * qz + soft2;
+                    cls = o2 == 0.f ? BHW_MIXED
+                          : rn * (1.0f - 0x1p-18f) > o2 && rn < 1e37f ? BHW_ACCEPT
+                          : rf * (1.0f + 0x1p-18f) < o2 ? BHW_OPEN : BHW_MIXED;
+                }
+            }
+            __syncwarp();
+            {
+                const unsigned om = __ballot_sync(FULL_MASK, cls == BHW_OPEN);
+                if (cls == BHW_OPEN) {
+                    const int at = top + __popc(om & lt);
+                    w.stack[at] = make_uint2((unsigned)cb, mask);
+                    w.run[at] = (unsigned char)nc;
+                }
+                top += __popc(om);
+            }
+            /* the nodes the box straddles: each body's own test */
+            const unsigned mm = __ballot_sync(FULL_MASK, cls == BHW_MIXED);
+            {
+                for (unsigned mq = mm; mq; mq &= mq - 1u) {
+                    const int src = __ffs(mq) - 1;
+                    const float dx = (__shfl_sync(FULL_MASK, na.x, src) - v[0]) + (__shfl_sync(FULL_MASK, nb.x, src) - vl[0]);
+                    const float dy = (__shfl_sync(FULL_MASK, na.y, src) - v[1]) + (__shfl_sync(FULL_MASK, nb.y, src) - vl[1]);
+                    const float dz = (__shfl_sync(FULL_MASK, na.z, src) - v[2]) + (__shfl_sync(FULL_MASK, nb.z, src) - vl[2]);
+                    const float q2 = __shfl_sync(FULL_MASK, o2, src);
+                    const unsigned mk = __shfl_sync(FULL_MASK, mask, src);
+                    const float r2 = dx * dx + dy * dy + dz * dz + soft2;
+                    const bool mine = (mk >> lane) & 1u;
+                    const bool in = q2 != 0.f && r2 < 1e37f;
+                    bool accept = in && r2 * (1.0f - 0x1p-18f) > q2;
+                    const bool sure = accept || (in && r2 * (1.0f + 0x1p-18f) < q2);
+                    if (__any_sync(FULL_MASK, mine && !sure)) {
+                        const ll sl = (ll)__shfl_sync(FULL_MASK, slot, src);
+                        if (!sure) {
+                            const double2 ra = t.rec[2 * sl], rb = t.rec[2 * sl + 1];
+                            accept = bh_accepts(ra.x - bx, ra.y - by, rb.x - bz, t.shalf[sl]);
+                        }
+                    }
+                    const unsigned am = __ballot_sync(FULL_MASK, mine && accept);
+                    const unsigned om = mk & ~am;
+                    if (lane == src) {
+                        if (om) {
+                            w.stack[top] = make_uint2((unsigned)cb, om);
+                            w.run[top] = (unsigned char)nc;
+                        }
+                        mask = am;
+                        cls = am ? BHW_ACCEPT : BHW_DROP;
+                    }
+                    top += om ? 1 : 0;
+                }
+            }
+            /* accepted nodes, in turn to the team's warps */
+            {
+                const unsigned am = __ballot_sync(FULL_MASK, cls == BHW_ACCEPT);
+                const bool put = cls == BHW_ACCEPT && ((turn + __popc(am & lt)) % BHW_TEAM) == (unsigned)wi;
+                turn += __popc(am);
+                const unsigned pm = __ballot_sync(FULL_MASK, put);
+                if (cl + __popc(pm) > B64_LIST) flush();
+                if (put) {
+                    const int at = cl + __popc(pm & lt);
+                    const double2 ra = t.rec[2 * (ll)slot], rb = t.rec[2 * (ll)slot + 1];
+                    w.x[at] = ra.x;
+                    w.y[at] = ra.y;
+                    w.z[at] = rb.x;
+                    w.m[at] = rb.y;
+                    w.mask[at] = mask;
+                }
+                cl += __popc(pm);
+            }
+            for (unsigned bm = __ballot_sync(FULL_MASK, cls == BHW_BUCKET && wi == 0); bm; bm &= bm - 1u) {
+                const int src = __ffs(bm) - 1;
+                const unsigned mk = __shfl_sync(FULL_MASK, mask, src);
+                const int bs = __shfl_sync(FULL_MASK, s, src), be = __shfl_sync(FULL_MASK, e, src);
+                if ((mk >> lane) & 1u) {
+                    double tx = 0.0, ty = 0.0, tz = 0.0;
+                    terms += bh_bucket64(A, vals, bs, be, k, bx, by, bz, gm, tx, ty, tz);
+                    fx += tx;
+                    fy += ty;
+                    fz += tz;
+                }
+                __syncwarp();
+            }
+            __syncwarp();
+        }
+        flush();
+        /* the team's sums, in warp order */
+        if (wi > 0) {
+            red[wi - 1][0][lane] = fx;
+            red[wi - 1][1][lane] = fy;
+            red[wi - 1][2][lane] = fz;
+        }
+        __syncthreads();
+        if (wi == 0 && have) {
+            for (int q = 0; q < BHW_TEAM - 1; q++) {
+                fx += red[q][0][lane];
+                fy += red[q][1][lane];
+                fz += red[q][2][lane];
+            }
+            A.fx[k] = fx;
+            A.fy[k] = fy;
+            A.fz[k] = fz;
+        }
+        all_terms += terms;
+    }
+    /* point-mass terms summed, for the measured work */
+    for (int o = 16; o > 0; o >>= 1) all_terms += __shfl_xor_sync(FULL_MASK, all_terms, o);
+    if (lane == 0 && all_terms) atomicAdd((unsigned long long *)&ctl->acc_bh_terms, all_terms);
+}
+
+/* ---- 5b. the mixed-precision walk --------------------------------------------
+ * The same tree and the same acceptance rule in FP32: centres of mass as
+ * hi/lo float pairs (so dx = (cm_hi - x_hi) + (cm_lo - x_lo) keeps ~2^-24 of
+ * |dx|), masses relative to the root's, the opening test as
+ * r^2 > (2 half / theta)^2 on the softened r^2, and the reciprocal square
+ * root of the SFU.
+ *
+ * A group of 32 bodies (neighbours in key order, one per lane) walks the tree
+ * together.  The warp keeps a stack of nodes, each with the lanes that have
+ * not accepted an ancestor of it, and visits 32 of them at once, one per
+ * lane: most nodes lie so far from the group's box (or so close) that all
+ * its bodies accept (or open) them, which one bound decides; accepted nodes
+ * are listed in shared memory and summed 32 or more at a time, every lane
+ * its own body, two nodes per packed instruction.  Only the nodes in between
+ * (1,100 of the 7,900 that a group of a 131,072-body Plummer sphere accepts)
+ * take each body's own test, with the same expression and rounding as a walk
+ * of that body alone, so every body sums the terms it would alone.  Sums are
+ * FP32, folded into (hi, lo) pairs after every list: the GB300 FP64 pipe is
+ * 1/64 of the FP32 rate.
+ *
+ * A walk that took one node at a time for the whole warp was bound by the
+ * latency of its node loads (issue slots 25 % busy).  The walk of a 131,072-
+ * body Plummer sphere went from 5.0 to 1.56 ms, of 10^6 uniform bodies from
+ * 20.3 to 7.3 ms.  What bounds it now is issue and, with a group to a warp,
+ * groups of uneven cost: 263,000 instructions a group before the lists were
+ * split into far and near ones, 60 % of them in the sums. */
 /* every node's record for the walk, in its slot */
 __global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(DevCtl *ctl, SimSegs seg, BhTree t)
 {
@@ -917,28 +1206,6 @@ struct alignas(16) BhWarp {
     int cb[BHW_MIX], nc[BHW_MIX];
     unsigned char run[BHW_STACK]; /* nodes of each run */
 };
-enum { BHW_DROP = 0, BHW_OPEN = 1, BHW_ACCEPT = 2, BHW_MIXED = 3, BHW_BUCKET = 4 };
-
-__device__ __forceinline__ float warp_minf(float v)
-{
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(FULL_MASK, v, o));
-    return v;
-}
-
-/* exclusive prefix of v (0..15) over the lanes and the warp's total */
-__device__ __forceinline__ int warp_prefix4(int v, unsigned lt, int &total)
-{
-    int x = 0;
-    total = 0;
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-        const unsigned m = __ballot_sync(FULL_MASK, (v >> b) & 1);
-        x += __popc(m & lt) << b;
-        total += __popc(m) << b;
-    }
-    return x;
-}
-
 /* FP32 partial sums and the (hi, lo) pairs they are folded into */
 struct BhSum {
     float2 ax, ay, az;
@@ -1487,6 +1754,8 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
     ALLOC(t.flags, node_cap);
     ALLOC(t.fa, node_cap + NBG_MAX_SIMS); /* a slot per collection's root, used or not */
     ALLOC(t.fb, node_cap + NBG_MAX_SIMS);
+    ALLOC(t.rec, 2 * (node_cap + NBG_MAX_SIMS));
+    ALLOC(t.shalf, node_cap + NBG_MAX_SIMS);
     ALLOC(t.fc, node_cap + NBG_MAX_SIMS);
     ALLOC(t.fd, node_cap);
     ALLOC(t.cbase, node_cap);
@@ -1511,7 +1780,7 @@ void nbg_bh_free(BhTree &t)
 {
     void *ps[] = {t.key[0], t.key[1], t.val[0], t.val[1], t.hist, t.base, t.blk, t.mass, t.mx, t.my,
                   t.mz, t.cmx, t.cmy, t.cmz, t.cx, t.cy, t.cz, t.half, t.skip, t.start,
-                  t.end, t.first, t.level, t.flags, t.fa, t.fb, t.fc, t.fd, t.cbase, t.ccount, t.slot,
+                  t.end, t.first, t.level, t.flags, t.fa, t.fb, t.rec, t.shalf, t.fc, t.fd, t.cbase, t.ccount, t.slot,
                   t.sbox, t.scount, t.stree, t.sroot, t.sgrp, t.sunit};
     for (void *p : ps) cudaFree(p);
     memset(&t, 0, sizeof t);
@@ -1556,8 +1825,8 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
     if (ng < 1) ng = 1;
     for (int level = BH_LEVELS; level >= 0; level--)
         k_bh_mass<<<ng, BH_BLOCK, 0, st>>>(cb.a, ctl, t.val[0], t, level);
+    k_bh_children<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
     if (mixed) {
-        k_bh_children<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
         k_bh_prep_mixed<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
         /* one wave of resident CTAs, which share the queue of units; 4 CTAs
          * per SM (121 registers, no spill) measured fastest, 2.38 ms for the
@@ -1571,7 +1840,10 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
         default: k_bh_force_mixed<4><<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
         }
     } else {
-        k_bh_force<<<g, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t);
+        k_bh_prep64<<<ng, BH_BLOCK, 0, st>>>(ctl, t);
+        const ll wgroups = cap / 32 + 1 + seg.nsims;
+        const int gw = (int)(wgroups < (ll)cb.sms * 5 ? wgroups : (ll)cb.sms * 5);
+        k_bh_force<<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t);
     }
     k_bh_sun<<<64, BH_BLOCK, 0, st>>>(cb.a, ctl, seg);
     k_bh_collide<<<g, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t, cb.ev_keys, cb.ev_cap);
@@ -1582,5 +1854,5 @@ int nbg_bh_launches(const CycleBufs &cb, bool mixed)
     const int passes = cb.seg.nsims > 1 ? 10 : 8;
     /* reset, bounds, segs, keys; the sort; count, top, scan, roots, nodes;
      * masses; (prep,) walk; suns; collisions */
-    return 4 + 3 * passes + 5 + (BH_LEVELS + 1) + (mixed ? 3 : 1) + 2;
+    return 4 + 3 * passes + 5 + (BH_LEVELS + 1) + 3 + 2;
 }

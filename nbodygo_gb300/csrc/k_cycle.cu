@@ -330,12 +330,12 @@ __device__ __forceinline__ unsigned p64_flags(unsigned f, double m)
  * warp of pairs; the root, four quotients and four products run beside it on
  * integers (nbg_exact.h), some 650 issue cycles a scheduler, 190 a pair warp
  * and SM.  Leaving more products to the pipe, or none of the squares, measured
- * 1-8 % slower.  16,384 Plummer bodies 28.9 -> 9.0 ms a pass, where the
+ * 1-8 % slower.  16,384 Plummer bodies 28.9 -> 8.4 ms a pass, where the
  * compiler's expansion of the root and the divisions kept the FP64 pipe 90 %
  * busy with 68 operations a pair; terms stay on the chip, where storing them
  * all took 48 bytes of traffic a pair and 3.2 GB at 65,536 bodies.  A body's
  * sum is one chain of n dependent additions of 64 cycles at least: that is
- * what a collection of a thousand bodies waits for (174 -> 79 us).  Tiles of
+ * what a collection of a thousand bodies waits for (174 -> 75 us).  Tiles of
  * 512 pairs, with a barrier three times as often, measured 11.1 ms. */
 #define P64_PROD 256
 #define P64_THREADS (P64_PROD + 96)
@@ -454,10 +454,10 @@ __global__ void __launch_bounds__(P64_THREADS, P64_MINB) k_pair_fp64(BodyArrays 
             const nbx_num f = nbx_quot(gm, nbx_square(root));
             const nbx_num ax = nbx_mul(f, nbx_unpack(bx)), ay = nbx_mul(f, nbx_unpack(by)),
                           az = nbx_mul(f, nbx_unpack(bz));
-            ex = (bx << 1) == 0 ? 0.0 : nbx_double(nbx_pack(nbx_quot(ax, r)));
-            ey = (by << 1) == 0 ? 0.0 : nbx_double(nbx_pack(nbx_quot(ay, r)));
-            ez = (bz << 1) == 0 ? 0.0 : nbx_double(nbx_pack(nbx_quot(az, r)));
-            return nbx_diff_ok(bx) && nbx_diff_ok(by) && nbx_diff_ok(bz) && ((bx | by | bz) << 1) != 0 &&
+            ex = nbx_zero(bx) ? 0.0 : nbx_double(nbx_pack(nbx_quot(ax, r)));
+            ey = nbx_zero(by) ? 0.0 : nbx_double(nbx_pack(nbx_quot(ay, r)));
+            ez = nbx_zero(bz) ? 0.0 : nbx_double(nbx_pack(nbx_quot(az, r)));
+            return nbx_diff_ok(bx) && nbx_diff_ok(by) && nbx_diff_ok(bz) && !nbx_zero(bx | by | bz) &&
                    nbx_square_ok(root) && (int)(nbx_div_bits(r) >> 32) > bound;
         };
         auto plain = [&](int ii, int jj, ll jbase, int buf, double &ex, double &ey, double &ez) {

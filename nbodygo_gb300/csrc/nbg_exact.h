@@ -103,7 +103,10 @@ NBG_XFN int nbx_within(uint64_t bits, uint32_t span)
     return ((uint32_t)(bits >> 52) & 0x7ffu) - (1023u - span) <= 2u * span;
 }
 NBG_XFN int nbx_root_ok(uint64_t bits) { return !(bits >> 63) && nbx_within(bits, 302); }
-NBG_XFN int nbx_diff_ok(uint64_t bits) { return nbx_within(bits, 150) || (bits << 1) == 0; }
+/* +-0, from the words: asked of the 64-bit pattern the compiler makes it a
+ * comparison on the FP64 pipe */
+NBG_XFN int nbx_zero(uint64_t bits) { return (((uint32_t)(bits >> 32) << 1) | (uint32_t)bits) == 0; }
+NBG_XFN int nbx_diff_ok(uint64_t bits) { return nbx_within(bits, 150) || nbx_zero(bits); }
 NBG_XFN int nbx_mass_ok(uint64_t bits) { return nbx_within(bits, 200); }
 
 #define NBX_ONE 0x10000000000000ull /* 2^52 */
@@ -163,9 +166,10 @@ struct nbx_div {
  * 2^odd) and the exact remainder, d^2 = S 2^(52 + odd) - rem. */
 struct nbx_root {
     nbx_div r;
-    uint64_t S;
+    uint64_t S, y1; /* y1 = 2^63 / sqrt(S 2^odd / 2^52) within 2^-59 */
     int64_t rem;
     uint32_t odd;
+    int e; /* the operand's exponent field */
 };
 
 /* RN(sqrt(s)) as a divisor, for s_bits in range.  Its value is
@@ -204,8 +208,10 @@ NBG_XFN nbx_root nbx_sqrt(uint64_t s_bits)
     v.r.y = y1 + (uint64_t)(((int64_t)(int32_t)(rem >> 22) * (y8 * y8 * y8)) >> 44);
     v.r.e = (int)((ef + 1023u - odd) >> 1);
     v.S = S;
+    v.y1 = y1;
     v.rem = rem;
     v.odd = odd;
+    v.e = (int)ef;
     return v;
 }
 
@@ -238,6 +244,16 @@ NBG_XFN nbx_div nbx_square(const nbx_root &v)
     const uint64_t y = nbx_mulhi(v.r.y, v.r.y) << (1 + v.odd);
     const int32_t y8 = (int32_t)(y >> 55);
     q.y = y + (uint64_t)(((int64_t)(int32_t)(diff >> (21 + v.odd)) * (y8 * y8)) >> 36);
+    return q;
+}
+
+/* The operand of a root itself as a divisor. */
+NBG_XFN nbx_div nbx_operand(const nbx_root &v)
+{
+    nbx_div q;
+    q.d = v.S;
+    q.e = v.e;
+    q.y = nbx_mulhi(v.y1, v.y1) << (1 + v.odd);
     return q;
 }
 

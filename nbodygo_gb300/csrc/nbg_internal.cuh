@@ -92,7 +92,7 @@ struct DevCtl {
     ll bh_nodes;
     ull bh_rmax;
     unsigned bh_next; /* the walk's next 32-body group (one per warp) */
-    unsigned bh_slots; /* mixed walk: child slots handed out */
+    unsigned bh_slots; /* the walk's child slots handed out */
     /* Hilbert order of the mixed path (perm): valid while no body changed
      * index; re-sorted when invalid or sort_interval cycles after the last
      * sort (0: NBG_SORT_INTERVAL_DEFAULT).  sort_now is this cycle's decision. */
@@ -184,11 +184,14 @@ struct BhTree {
     ll *base;           /* nodes starting at each sorted position, then their scan */
     ll *blk;            /* per-block sums of that scan */
     double *mass, *mx, *my, *mz, *cmx, *cmy, *cmz, *cx, *cy, *cz, *half;
-    float4 *fa, *fb;    /* mixed walk, by slot: (cm hi xyz, mass / root mass), (cm lo xyz, opening r^2) */
-    int4 *fc;           /* mixed walk, by slot: (first child's slot, children | flags << 8, start, end) */
+    float4 *fa, *fb;    /* mixed walk, by slot: (cm hi xyz, mass / root mass), (cm lo xyz, opening r^2);
+                         * FP64 walk: (cm hi xyz, opening r^2), (cm lo xyz, 0) */
+    double2 *rec;       /* FP64 walk, by slot: (cm x, y), (cm z, mass) */
+    double *shalf;      /* and half size */
+    int4 *fc;           /* by slot: (first child's slot, children | flags << 8, start, end) */
     float4 *fd;         /* collision query: the node's cube (centre xyz, half) in FP32 */
     int *skip, *start, *end, *first;
-    int *cbase;            /* mixed walk: slot of the first of the node's children */
+    int *cbase;            /* slot of the first of the node's children */
     unsigned char *ccount; /* and how many there are */
     int *slot;             /* the node's own slot */
     unsigned char *level, *flags;

@@ -57,6 +57,8 @@ static void one(double s, double g, double m, const double d[3])
     const double dist = sqrt(s), gm = g * m;
     same("sqrt", dist, nbx_div_bits(r), s, 0);
     const double d2 = dist * dist, f = gm / d2;
+    same("force over the operand", gm / s,
+         nbx_pack(nbx_quot(nbx_mul(nbx_unpack(nbx_bits(g)), nbx_unpack(nbx_bits(m))), nbx_operand(root))), gm, s);
     if (!nbx_square_ok(root)) return;
     const nbx_div r2 = nbx_square(root);
     same("square", d2, nbx_div_bits(r2), dist, dist);

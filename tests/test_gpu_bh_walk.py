@@ -7,6 +7,7 @@ import pytest
 from nbodygo_gb300 import _abi as A
 from nbodygo_gb300 import workloads as W
 from nbodygo_gb300.api import Simulation
+from oracle.oracle import OracleSim
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,34 @@ def test_both_sides_of_a_warp_to_a_group(n):
 @pytest.mark.parametrize("n", [64, 3000, 70001])
 def test_shared_leaves(n):
     _close(_clustered(n, 70 + n))
+
+
+@pytest.mark.parametrize("scale,mass", [(1e60, 1e70), (1e-30, 1e-10), (1.0, 1e-90), (1e25, 1.0)])
+def test_fp64_walk_out_of_fp32_range(scale, mass):
+    """Coordinates and masses that FP32 cannot hold: the bodies decide in
+    FP64, and terms outside nbg_exact.h's range take the ordinary operators."""
+    b = W.plummer(700, seed=12)
+    for c in "xyz":
+        b[c] *= scale
+    b["mass"][:] = mass
+    b["radius"][:] = 0.0
+    b["collision"][:] = A.NONE
+    f, _ = _forces(b, "fp64")
+    o = OracleSim(threads=8)
+    o.set_barnes_hut(True)
+    o.set_bodies(b)
+    g = np.stack(o.forces())
+    mag, err = np.linalg.norm(g / np.abs(g).max(), axis=0), np.linalg.norm((f - g) / np.abs(g).max(), axis=0)
+    assert np.all(err <= 1e-12 * mag)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 65, 500, 4001])
+def test_fp64_walk_matches_the_oracle(n):
+    b = W.plummer(n, seed=80 + n)
+    b["collision"][:] = A.NONE
+    f, _ = _forces(b, "fp64")
+    o = OracleSim(threads=8)
+    o.set_barnes_hut(True)
+    o.set_bodies(b)
+    g = np.stack(o.forces())
+    assert np.all(np.linalg.norm(f - g, axis=0) <= 1e-12 * np.linalg.norm(g, axis=0))
