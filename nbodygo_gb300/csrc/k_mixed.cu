@@ -76,6 +76,7 @@ __device__ __forceinline__ bool is_special(double x, double y, double z, double 
 __global__ void k_mix_reduce(BodyArrays A, DevCtl *ctl, SimSegs seg)
 {
     if (ctl->error) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) nbg_sort_decide(ctl);
     const ll n = ctl->n;
     float rmax = 0.f, xmax = 0.f;
     double mmax = 0.0;
@@ -115,92 +116,26 @@ __global__ void k_mix_reduce(BodyArrays A, DevCtl *ctl, SimSegs seg)
     }
 }
 
-/* Packs body perm[p] at sorted position p:
- * jhi = (x_hi, y_hi, z_hi, m/m_scale), jlo = (x_lo, y_lo, z_lo, radius).
- * A special body (see is_special) gets a far sentinel position, no mass and
- * x_lo = NaN, which is how the kernels recognise it. */
-__global__ void k_mix_pack(BodyArrays A, DevCtl *ctl, const unsigned *perm, float4 *jhi, float4 *jlo)
+/* Body k packed: h = (x_hi, y_hi, z_hi, m/m_scale), l = (x_lo, y_lo, z_lo,
+ * radius).  A special body (see is_special) gets a far sentinel position, no
+ * mass and x_lo = NaN, which is how the kernels recognise it. */
+__device__ __forceinline__ void pack_body(const BodyArrays &A, ll k, double ms, float4 &h, float4 &l)
 {
-    if (ctl->error) return;
-    const ll n = ctl->n;
-    double ms = ctl->m_scale;
-    if (!(ms > 0.0)) ms = 1.0;
-    for (ll p = (ll)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (ll)gridDim.x * blockDim.x) {
-        const ll k = perm[p];
-        const double x = A.x[k], y = A.y[k], z = A.z[k], r = A.rad[k];
-        if (is_special(x, y, z, r)) {
-            jhi[p] = make_float4(SENTINEL_POS, SENTINEL_POS, SENTINEL_POS, 0.f);
-            jlo[p] = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
-            continue;
-        }
-        const float xh = (float)x, yh = (float)y, zh = (float)z;
-        const float xl = (float)(x - (double)xh), yl = (float)(y - (double)yh), zl = (float)(z - (double)zh);
-        const bool live = (A.flags[k] & NBG_LIVE_MASK) == NBG_F_EXISTS;
-        const float m = live ? (float)(A.m[k] / ms) : 0.f;
-        jhi[p] = make_float4(xh, yh, zh, m);
-        jlo[p] = make_float4(xl, yl, zl, (float)r);
+    const double x = A.x[k], y = A.y[k], z = A.z[k], r = A.rad[k];
+    if (is_special(x, y, z, r)) {
+        h = make_float4(SENTINEL_POS, SENTINEL_POS, SENTINEL_POS, 0.f);
+        l = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+        return;
     }
+    const float xh = (float)x, yh = (float)y, zh = (float)z;
+    const float xl = (float)(x - (double)xh), yl = (float)(y - (double)yh), zl = (float)(z - (double)zh);
+    const bool live = (A.flags[k] & NBG_LIVE_MASK) == NBG_F_EXISTS;
+    const float m = live ? (float)(A.m[k] / ms) : 0.f;
+    h = make_float4(xh, yh, zh, m);
+    l = make_float4(xl, yl, zl, (float)r);
 }
 
 __device__ __forceinline__ bool packed_special(const float4 &lo) { return lo.x != lo.x; }
-
-/* origin of each i-tile: centre of the bounding box of its bodies */
-#define TILES_BLOCK 128
-__global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(DevCtl *ctl, SimSegs seg, const float4 *jhi,
-                                                           const float4 *jlo, float4 *tile_c, float *tile_t, int itile)
-{
-    __shared__ float red[6][TILES_BLOCK / 32];
-    if (ctl->error) return;
-    const ll ntiles = seg.mtile_off[seg.nsims];
-    for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int sim = nbg_sim_of(seg.mtile_off, seg.nsims, tile);
-    const ll base = seg.off[sim] + (tile - seg.mtile_off[sim]) * itile;
-    const ll n = seg.off[sim + 1] < base + itile ? seg.off[sim + 1] : base + itile;
-    float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
-    for (ll p = base + threadIdx.x; p < n; p += TILES_BLOCK) {
-        if (packed_special(jlo[p])) continue;
-        float4 h = jhi[p];
-        lo[0] = fminf(lo[0], h.x);
-        lo[1] = fminf(lo[1], h.y);
-        lo[2] = fminf(lo[2], h.z);
-        hi[0] = fmaxf(hi[0], h.x);
-        hi[1] = fmaxf(hi[1], h.y);
-        hi[2] = fmaxf(hi[2], h.z);
-    }
-    for (int o = 16; o > 0; o >>= 1)
-        for (int c = 0; c < 3; c++) {
-            lo[c] = fminf(lo[c], __shfl_xor_sync(FULL_MASK, lo[c], o));
-            hi[c] = fmaxf(hi[c], __shfl_xor_sync(FULL_MASK, hi[c], o));
-        }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0)
-        for (int c = 0; c < 3; c++) {
-            red[c][w] = lo[c];
-            red[3 + c][w] = hi[c];
-        }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float c3[3], e2 = 0.f, amax = 0.f;
-        for (int c = 0; c < 3; c++) {
-            float l = red[c][0], h = red[3 + c][0];
-            for (int q = 1; q < TILES_BLOCK / 32; q++) {
-                l = fminf(l, red[c][q]);
-                h = fmaxf(h, red[3 + c][q]);
-            }
-            c3[c] = (l <= h) ? 0.5f * l + 0.5f * h : 0.f;
-            const float e = l <= h ? fmaxf(h - c3[c], c3[c] - l) : 0.f;
-            e2 += e * e;
-            amax = fmaxf(amax, l <= h ? fmaxf(fabsf(l), fabsf(h)) : 0.f);
-        }
-        /* .w: a radius about the origin that holds every body of the tile,
-         * rounded up past the FP32 arithmetic and the bodies' lo parts */
-        const float rad = sqrtf(e2) * (1.0f + 0x1p-16f) + amax * 0x1p-20f;
-        tile_c[tile] = make_float4(c3[0], c3[1], c3[2], rad);
-        if (tile_t) tile_t[tile] = 0.f;
-    }
-    __syncthreads(); /* red[] is rewritten by the next tile */
-    }
-}
 
 /* ---- the pair kernel ----------------------------------------------------- */
 
@@ -258,60 +193,132 @@ __device__ __forceinline__ void fold64(float &hi, float &lo, double v)
     lo += vl;
 }
 
-/* i-body at sorted position p (p >= n: none) re-centred on the tile origin
- * c, and its near-pair threshold t on r^2 (FP32, conservative): pairs closer
- * than max(r_i + r_max + the FP32 error bound, kappa |x - c|_max) take the
- * exact path.  A special body sits at the sentinel with t = -1. */
-__device__ __forceinline__ void i_body_setup(const float4 *__restrict__ jhi, const float4 *__restrict__ jlo, ll p, ll n,
-                                             const float4 &c, float rmax, float xmax, double kappa, float &xr,
-                                             float &yr, float &zr, float &t)
+/* The packed body h, l re-centred on its tile's origin c, and its near-pair
+ * threshold t on r^2 (FP32, conservative): pairs closer than max(r_i + r_max +
+ * the FP32 error bound, kappa |x - c|_max) take the exact path.  A special
+ * body sits at the sentinel with t = -1. */
+__device__ __forceinline__ float4 i_body_setup(const float4 &h, const float4 &l, const float4 &c, float rmax,
+                                               float xmax, double kappa)
 {
-    xr = yr = zr = 0.f;
-    t = -1.f;
-    if (p >= n) return;
-    const float4 h = jhi[p], l = jlo[p];
-    if (packed_special(l)) {
-        xr = yr = zr = SENTINEL_POS;
-        return;
-    }
-    xr = (h.x - c.x) + l.x;
-    yr = (h.y - c.y) + l.y;
-    zr = (h.z - c.z) + l.z;
+    if (packed_special(l)) return make_float4(SENTINEL_POS, SENTINEL_POS, SENTINEL_POS, -1.f);
+    const float xr = (h.x - c.x) + l.x, yr = (h.y - c.y) + l.y, zr = (h.z - c.z) + l.z;
     const double ri = (double)l.w + fabs((double)l.w) * 0x1p-22; /* rounded up */
     const double D = fmax(0.0, ri + (double)rmax);
     const double amax = (double)fmaxf(fabsf(xr), fmaxf(fabsf(yr), fabsf(zr)));
     const double eps = 0x1p-19 * (amax + D) + 0x1p-44 * (double)xmax + 0x1p-100;
     const double b = fmax(D + eps, kappa * amax) * (1.0 + 0x1p-18);
-    t = __double2float_ru(b * b);
+    return make_float4(xr, yr, zr, __double2float_ru(b * b));
 }
 
-/* every i-body's re-centred position and near-pair threshold, once per
- * cycle; the pair kernel reads them for each chunk that covers the body */
-__global__ void k_mix_iprep(DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi,
-                            const float4 *__restrict__ jlo, const float4 *__restrict__ tile_c, float4 *iprep,
-                            float *tile_t, int itile)
+/* Everything the pair kernel reads of a tile, one CTA a tile: its bodies
+ * packed in sorted order, its origin (the centre of their bounding box) and a
+ * radius that holds them, each i-body's re-centred position and near-pair
+ * threshold, the largest threshold, and the chunks that share the tile
+ * (tile_rng, if given) for k_mix_out.  One launch where packing, tile origins
+ * and i-bodies were three, each reading back what the one before wrote:
+ * 19.3 -> 13.4 us for 2,501 bodies, 29.5 -> 13.6 us for 20,011 (one launch
+ * each under the profiler, caches cold). */
+#define TILES_BLOCK 256
+#define TILES_ITEMS (NBG_MIX_MAX_ITILE / TILES_BLOCK)
+__global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl *ctl, SimSegs seg,
+                                                           const unsigned *__restrict__ perm, float4 *jhi, float4 *jlo,
+                                                           float4 *tile_c, float *tile_t, float4 *iprep,
+                                                           int2 *tile_rng, int itile)
 {
+    __shared__ float red[6][TILES_BLOCK / 32];
+    __shared__ float4 s_c;
+    __shared__ unsigned s_t;
     if (ctl->error) return;
-    const ll n = ctl->n;
+    const ll ntiles = seg.mtile_off[seg.nsims];
+    double ms = ctl->m_scale;
+    if (!(ms > 0.0)) ms = 1.0;
     const float rmax = __uint_as_float(ctl->rmax_bits);
     const float xmax = __uint_as_float(ctl->xmax_bits);
     const double kappa0 = (double)ctl->near_kappa;
-    for (ll p = (ll)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (ll)gridDim.x * blockDim.x) {
-        const int sim = nbg_sim_of(seg.off, seg.nsims, p);
-        const ll s0 = seg.off[sim];
+    const int tid = threadIdx.x, w = tid >> 5;
+    for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int sim = nbg_sim_of(seg.mtile_off, seg.nsims, tile);
+        const ll s0 = seg.off[sim], s1 = seg.off[sim + 1];
+        const ll t = tile - seg.mtile_off[sim];
+        const ll base = s0 + t * itile;
+        const ll n = s1 < base + itile ? s1 : base + itile;
+        float4 h[TILES_ITEMS], l[TILES_ITEMS];
+        float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+#pragma unroll
+        for (int q = 0; q < TILES_ITEMS; q++) {
+            const ll p = base + q * TILES_BLOCK + tid;
+            if (p >= n) continue;
+            pack_body(A, (ll)perm[p], ms, h[q], l[q]);
+            jhi[p] = h[q];
+            jlo[p] = l[q];
+            if (packed_special(l[q])) continue;
+            lo[0] = fminf(lo[0], h[q].x);
+            lo[1] = fminf(lo[1], h[q].y);
+            lo[2] = fminf(lo[2], h[q].z);
+            hi[0] = fmaxf(hi[0], h[q].x);
+            hi[1] = fmaxf(hi[1], h[q].y);
+            hi[2] = fmaxf(hi[2], h[q].z);
+        }
+        for (int o = 16; o > 0; o >>= 1)
+            for (int c = 0; c < 3; c++) {
+                lo[c] = fminf(lo[c], __shfl_xor_sync(FULL_MASK, lo[c], o));
+                hi[c] = fmaxf(hi[c], __shfl_xor_sync(FULL_MASK, hi[c], o));
+            }
+        if ((tid & 31) == 0)
+            for (int c = 0; c < 3; c++) {
+                red[c][w] = lo[c];
+                red[3 + c][w] = hi[c];
+            }
+        __syncthreads();
+        if (tid == 0) {
+            float c3[3], e2 = 0.f, amax = 0.f;
+            for (int c = 0; c < 3; c++) {
+                float a = red[c][0], b = red[3 + c][0];
+                for (int q = 1; q < TILES_BLOCK / 32; q++) {
+                    a = fminf(a, red[c][q]);
+                    b = fmaxf(b, red[3 + c][q]);
+                }
+                c3[c] = (a <= b) ? 0.5f * a + 0.5f * b : 0.f;
+                const float e = a <= b ? fmaxf(b - c3[c], c3[c] - a) : 0.f;
+                e2 += e * e;
+                amax = fmaxf(amax, a <= b ? fmaxf(fabsf(a), fabsf(b)) : 0.f);
+            }
+            /* .w: a radius about the origin that holds every body of the tile,
+             * rounded up past the FP32 arithmetic and the bodies' lo parts */
+            const float rad = sqrtf(e2) * (1.0f + 0x1p-16f) + amax * 0x1p-20f;
+            s_c = make_float4(c3[0], c3[1], c3[2], rad);
+            s_t = 0u;
+            tile_c[tile] = s_c;
+        }
+        if (tile_rng && (tid == 32 || tid == 64)) {
+            const ll tu = seg.item_off[sim] + t * (s1 - s0); /* the tile's first unit */
+            const int c = nbg_work_chunk(tid == 32 ? tu : tu + (s1 - s0) - 1, ctl->splits, ctl->work_total);
+            (tid == 32 ? tile_rng[tile].x : tile_rng[tile].y) = c;
+        }
+        __syncthreads();
+        const float4 c = s_c;
         /* In a small collection one or two tiles span it all, so a body's
          * offset from its tile origin is large next to its neighbours'
          * distances, and the neighbours carry much of its force: twice the
          * factor there.  Such collections hold a small share of the work. */
-        const double kappa = seg.off[sim + 1] - s0 <= NBG_NEAR_SMALL_N ? 2.0 * kappa0 : kappa0;
-        const ll tile = seg.mtile_off[sim] + (p - s0) / itile;
-        const float4 c = tile_c[tile];
-        float xr, yr, zr, t;
-        i_body_setup(jhi, jlo, p, seg.off[sim + 1], c, rmax, xmax, kappa, xr, yr, zr, t);
-        iprep[p] = make_float4(xr, yr, zr, t);
-        /* the tile's largest near-pair threshold (positive floats order as
-         * their bit patterns) */
-        if (tile_t && t > 0.f) atomicMax((unsigned *)&tile_t[tile], __float_as_uint(t));
+        const double kappa = s1 - s0 <= NBG_NEAR_SMALL_N ? 2.0 * kappa0 : kappa0;
+        float tmax = 0.f;
+#pragma unroll
+        for (int q = 0; q < TILES_ITEMS; q++) {
+            const ll p = base + q * TILES_BLOCK + tid;
+            if (p >= n) continue;
+            const float4 v = i_body_setup(h[q], l[q], c, rmax, xmax, kappa);
+            iprep[p] = v;
+            tmax = fmaxf(tmax, v.w);
+        }
+        if (tile_t) {
+            /* positive floats order as their bit patterns */
+            const unsigned m = __reduce_max_sync(FULL_MASK, __float_as_uint(tmax));
+            if ((tid & 31) == 0) atomicMax(&s_t, m);
+            __syncthreads();
+            if (tid == 0) tile_t[tile] = __uint_as_float(s_t);
+        }
+        __syncthreads(); /* the shared values are rewritten by the next tile */
     }
 }
 
@@ -795,13 +802,14 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
  * that share the tile are cut into OUT_SLICES runs, one per row of 32
  * threads, each row adds its run in chunk order, and the rows' sums are added
  * in row order, so the result is the same on every run.  Small collections
- * are cut finely (156 shares a tile at 20,011 bodies), and one thread adding
- * all shares of its body was bound by that chain of loads: 350 us there, now
- * 18 us; the tile's range of chunks is found once per CTA. */
+ * are cut finely (some 100 shares a tile at 20,011 bodies), and one thread
+ * adding all shares of its body was bound by that chain of loads: the kernels
+ * beside the pairs took 546 us a cycle there with 24,320 chunks, now 190 us. */
 #define OUT_SLICES 8
 #define OUT_BODIES 32
 __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A, DevCtl *ctl, SimSegs seg,
-                                                                   const unsigned *perm, const double *part, int itile)
+                                                                   const unsigned *perm, const double *part,
+                                                                   const int2 *tile_rng, int itile)
 {
     __shared__ double red[3][OUT_SLICES][OUT_BODIES];
     __shared__ int range[2];
@@ -820,12 +828,18 @@ __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A
         const ll s0 = seg.off[sim], n = seg.off[sim + 1];
         const ll t = g - seg.mtile_off[sim];
         if (s0 + t * itile + li - col >= n) continue; /* no body in this group (uniform) */
-        if (threadIdx.x < 2) {
-            const ll tu = seg.item_off[sim] + t * (n - s0); /* the tile's first unit */
-            range[threadIdx.x] = nbg_work_chunk(threadIdx.x == 0 ? tu : tu + (n - s0) - 1, C, W);
+        int2 rng;
+        if (tile_rng) {
+            rng = tile_rng[g];
+        } else {
+            if (threadIdx.x < 2) {
+                const ll tu = seg.item_off[sim] + t * (n - s0); /* the tile's first unit */
+                range[threadIdx.x] = nbg_work_chunk(threadIdx.x == 0 ? tu : tu + (n - s0) - 1, C, W);
+            }
+            __syncthreads();
+            rng = make_int2(range[0], range[1]);
         }
-        __syncthreads();
-        const int c0 = range[0], cnt = range[1] - range[0] + 1;
+        const int c0 = rng.x, cnt = rng.y - rng.x + 1;
         const int a = c0 + (int)((ll)cnt * row / OUT_SLICES), b = c0 + (int)((ll)cnt * (row + 1) / OUT_SLICES);
         double sx = 0, sy = 0, sz = 0;
         const double *o = part + (g + a) * 3 * itile + li;
@@ -1385,13 +1399,15 @@ void nbg_launch_mixed_prep(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     const int fg = nbg_flat_grid(cb, cb.cap);
     k_mix_reduce<<<fg, 256, 0, st>>>(cb.a, ctl, cb.seg);
     nbg_launch_spatial_sort(cb, ctl, st);
-    k_mix_pack<<<fg, 256, 0, st>>>(cb.a, ctl, cb.perm, cb.jhi, cb.jlo);
     const int itile = cb.itile > 0 ? cb.itile : NBG_MIX_ITILE;
     ll tiles = (cb.cap + itile - 1) / itile + cb.seg.nsims;
     if (tiles > (ll)(cb.sms > 0 ? cb.sms : 1) * 64) tiles = (ll)(cb.sms > 0 ? cb.sms : 1) * 64;
-    k_mix_tiles<<<(int)tiles, TILES_BLOCK, 0, st>>>(ctl, cb.seg, cb.jhi, cb.jlo, cb.tile_c, cb.tile_t, itile);
-    k_mix_iprep<<<fg, 256, 0, st>>>(ctl, cb.seg, cb.jhi, cb.jlo, cb.tile_c, cb.iprep, cb.tile_t, itile);
+    k_mix_tiles<<<(int)tiles, TILES_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.perm, cb.jhi, cb.jlo, cb.tile_c, cb.tile_t,
+                                                    cb.iprep, nbg_mix_is_sym(cb.mix_variant) ? nullptr : cb.tile_rng,
+                                                    itile);
 }
+
+int nbg_mixed_launches(const CycleBufs &cb) { return 4 + nbg_spatial_sort_launches(cb); }
 
 void nbg_launch_mixed_pair(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 {
@@ -1425,7 +1441,7 @@ void nbg_launch_mixed_out(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     {
         const int itile = cb.itile > 0 ? cb.itile : NBG_MIX_ITILE;
         k_mix_out<<<nbg_flat_grid(cb, (cb.cap + (ll)itile * cb.seg.nsims) * OUT_SLICES), OUT_SLICES * OUT_BODIES, 0, st>>>(
-            cb.a, ctl, cb.seg, cb.perm, cb.part, itile);
+            cb.a, ctl, cb.seg, cb.perm, cb.part, cb.tile_rng, itile);
     }
 }
 

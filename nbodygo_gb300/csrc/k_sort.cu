@@ -38,34 +38,33 @@ __device__ __forceinline__ unsigned quant10(float x, float inv_span)
  * Hilbert key over [-x_max, x_max]^3.  Several sims: the sim index in the top
  * 11 bits and a 21-bit Hilbert key over the sim's own box, so every sim keeps
  * its range of positions and is ordered inside it. */
+__device__ __forceinline__ unsigned order_key(const BodyArrays &A, const DevCtl *ctl, const SimSegs &seg, ll k)
+{
+    const double x = A.x[k], y = A.y[k], z = A.z[k], r = A.rad[k];
+    const bool finite = fabs(x) <= 1.7976931348623157e308 && fabs(y) <= 1.7976931348623157e308 &&
+                        fabs(z) <= 1.7976931348623157e308 && r == r;
+    if (seg.nsims == 1) {
+        const float xmax = __uint_as_float(ctl->xmax_bits);
+        const float inv_span = xmax > 0.f ? 0.5f / xmax : 0.f;
+        return finite ? nbg_hilbert(quant10((float)x, inv_span), quant10((float)y, inv_span),
+                                    quant10((float)z, inv_span), 10)
+                      : 1u << 30;
+    }
+    const int sim = nbg_sim_of(seg.off, seg.nsims, k);
+    const float xmax = __uint_as_float(seg.xmax_bits[sim]);
+    const float inv_span = xmax > 0.f ? 0.5f / xmax : 0.f;
+    const unsigned m = finite ? nbg_hilbert(quant10((float)x, inv_span) >> 3, quant10((float)y, inv_span) >> 3,
+                                            quant10((float)z, inv_span) >> 3, 7)
+                              : 0x1fffffu;
+    return ((unsigned)sim << 21) | m;
+}
+
 __global__ void k_order_keys(BodyArrays A, DevCtl *ctl, SimSegs seg, unsigned *keys, unsigned *vals)
 {
     if (ctl->error || !ctl->sort_now) return;
     const ll n = ctl->n;
-    const bool multi = seg.nsims > 1;
     for (ll k = (ll)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (ll)gridDim.x * blockDim.x) {
-        const double x = A.x[k], y = A.y[k], z = A.z[k], r = A.rad[k];
-        const bool finite = fabs(x) <= 1.7976931348623157e308 && fabs(y) <= 1.7976931348623157e308 &&
-                            fabs(z) <= 1.7976931348623157e308 && r == r;
-        unsigned key;
-        if (!multi) {
-            const float xmax = __uint_as_float(ctl->xmax_bits);
-            const float inv_span = xmax > 0.f ? 0.5f / xmax : 0.f;
-            key = 1u << 30;
-            if (finite)
-                key = nbg_hilbert(quant10((float)x, inv_span), quant10((float)y, inv_span),
-                                  quant10((float)z, inv_span), 10);
-        } else {
-            const int sim = nbg_sim_of(seg.off, seg.nsims, k);
-            const float xmax = __uint_as_float(seg.xmax_bits[sim]);
-            const float inv_span = xmax > 0.f ? 0.5f / xmax : 0.f;
-            unsigned m = 0x1fffffu;
-            if (finite)
-                m = nbg_hilbert(quant10((float)x, inv_span) >> 3, quant10((float)y, inv_span) >> 3,
-                                quant10((float)z, inv_span) >> 3, 7);
-            key = ((unsigned)sim << 21) | m;
-        }
-        keys[k] = key;
+        keys[k] = order_key(A, ctl, seg, k);
         vals[k] = (unsigned)k;
     }
 }
@@ -205,6 +204,63 @@ __global__ void __launch_bounds__(1024) k_rs_scan_fin(DevCtl *ctl, int what, ll 
     }
 }
 
+/* The histogram and its scan in one launch, for histograms of at most
+ * one scan chunk: the block that arrives last scans them all.  The order of
+ * up to 131,072 bodies takes 9 launches in place of 21 (20,011 bodies, mean of
+ * a cycle that sorts and three that keep their order: 64 us against 101); a
+ * longer histogram would leave the last block's 256 threads a scan of more than
+ * 32 entries each, and keeps its three launches. */
+template <typename K>
+__global__ void __launch_bounds__(RS_BLOCK) k_rs_hist_scan(DevCtl *ctl, int what, const K *keys, int shift, ll *hist)
+{
+    __shared__ unsigned cnt[RS_BINS];
+    __shared__ ll wtot[RS_BLOCK / 32];
+    __shared__ unsigned s_last;
+    const ll n = rs_count(ctl, what);
+    if (n == 0) return;
+    const ll nb = (n + RS_TILE - 1) / RS_TILE;
+    const ll b = blockIdx.x;
+    if (b >= nb) return;
+    for (int d = threadIdx.x; d < RS_BINS; d += RS_BLOCK) cnt[d] = 0;
+    __syncthreads();
+    const ll base = b * RS_TILE;
+    for (int q = 0; q < RS_ITEMS; q++) {
+        ll k = base + (ll)q * RS_BLOCK + threadIdx.x;
+        if (k < n) atomicAdd(&cnt[(unsigned)(keys[k] >> shift) & 0xffu], 1u);
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < RS_BINS; d += RS_BLOCK) hist[(ll)d * nb + b] = cnt[d];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(&ctl->ticket, 1u) == (unsigned)nb - 1u ? 1u : 0u;
+        if (s_last) ctl->ticket = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    /* thread d takes digit d's nb entries */
+    ll *row = hist + (ll)threadIdx.x * nb;
+    ll s = 0;
+    for (ll q = 0; q < nb; q++) s += __ldcg(&row[q]);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    ll x = s;
+    for (int o = 1; o < 32; o <<= 1) {
+        const ll y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wtot[w] = x;
+    __syncthreads();
+    ll ex = x - s;
+    for (int v = 0; v < w; v++) ex += wtot[v];
+    for (ll q = 0; q < nb; q++) {
+        const ll v = __ldcg(&row[q]);
+        row[q] = ex;
+        ex += v;
+    }
+}
+static_assert(RS_BLOCK == RS_BINS, "a thread per digit");
+
 /* stable scatter: element order within a block is kept per digit (vals
  * NULL: keys only) */
 template <typename K>
@@ -256,28 +312,93 @@ ll nbg_sort_scratch_hist(ll cap)
     return h + (h + RS_SCAN_CHUNK - 1) / RS_SCAN_CHUNK;
 }
 
-/* Whether this cycle sorts.  Bodies move a small fraction of a tile's size
- * per cycle, so an order a few cycles old still gives compact tiles; which i
- * a tile holds never changes a result's correctness, only its FP32 error
- * and the near-pair count.  An order is dropped (sort_valid = 0) whenever a
- * body changes index or the arrays are replaced: compaction, loads, edits,
- * reallocation, and a cycle that failed and is run again. */
-__global__ void k_sort_decide(DevCtl *ctl)
+/* The order of a collection of up to RSS_MAX bodies by one block, when the
+ * cycle sorts: keys, then four stable LSD passes of 8-bit digits in shared
+ * memory.  A warp takes 128 consecutive elements, ranks them by digit with
+ * match masks in element order, and the ranks are offset by the counts of
+ * the warps before it: the same order as the multi-block sort, in one launch
+ * in place of 21 (2,501 bodies, mean of a cycle that sorts and three that keep
+ * their order: 8.5 us against 93). */
+#define RSS_BLOCK 1024
+#define RSS_WARPS (RSS_BLOCK / 32)
+#define RSS_MAX 4096
+#define RSS_ROUNDS (RSS_MAX / RSS_BLOCK)
+__global__ void __launch_bounds__(RSS_BLOCK) k_sort_small(BodyArrays A, DevCtl *ctl, SimSegs seg, unsigned *perm)
 {
-    if (ctl->error) return;
-    const int k = ctl->sort_interval > 0 ? ctl->sort_interval : NBG_SORT_INTERVAL_DEFAULT;
-    const bool now = !ctl->sort_valid || ctl->cycle - ctl->sort_cycle >= (ull)k;
-    ctl->sort_now = now;
-    if (now) {
-        ctl->sort_valid = 1;
-        ctl->sort_cycle = ctl->cycle;
+    __shared__ unsigned skey[RSS_MAX];
+    __shared__ unsigned short sval[RSS_MAX], cnt[RSS_WARPS][RS_BINS];
+    __shared__ unsigned base[RS_BINS], wtot[RS_BINS / 32];
+    if (ctl->error || !ctl->sort_now) return;
+    const int n = (int)ctl->n;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int k = tid; k < n; k += RSS_BLOCK) {
+        skey[k] = order_key(A, ctl, seg, k);
+        sval[k] = (unsigned short)k;
     }
+    for (int pass = 0; pass < 4; pass++) {
+        const int shift = 8 * pass;
+        for (int c = tid; c < RSS_WARPS * RS_BINS; c += RSS_BLOCK) (&cnt[0][0])[c] = 0;
+        __syncthreads();
+        unsigned key[RSS_ROUNDS], rank[RSS_ROUNDS];
+        unsigned short val[RSS_ROUNDS];
+#pragma unroll
+        for (int q = 0; q < RSS_ROUNDS; q++) {
+            const int e = w * (32 * RSS_ROUNDS) + q * 32 + lane;
+            const bool ok = e < n;
+            key[q] = ok ? skey[e] : 0u;
+            val[q] = ok ? sval[e] : (unsigned short)0;
+            const unsigned d = ok ? (key[q] >> shift) & 0xffu : RS_BINS;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const unsigned before = __popc(peers & lt);
+            const unsigned old = ok ? cnt[w][d] : 0u;
+            rank[q] = old + before;
+            __syncwarp();
+            if (ok && before == 0) cnt[w][d] = (unsigned short)(old + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        /* per digit: the warps' counts become their offsets; then the digits'
+         * starts, a scan over the 256 totals */
+        unsigned tot = 0;
+        if (tid < RS_BINS) {
+            for (int v = 0; v < RSS_WARPS; v++) {
+                const unsigned c = cnt[v][tid];
+                cnt[v][tid] = (unsigned short)tot;
+                tot += c;
+            }
+            unsigned x = tot;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            base[tid] = x - tot;
+            if (lane == 31) wtot[w] = x;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < RSS_ROUNDS; q++) {
+            const int e = w * (32 * RSS_ROUNDS) + q * 32 + lane;
+            if (e < n) {
+                const unsigned d = (key[q] >> shift) & 0xffu;
+                unsigned pos = base[d] + cnt[w][d] + rank[q];
+                for (unsigned v = 0; v < d / 32; v++) pos += wtot[v];
+                skey[pos] = key[q];
+                sval[pos] = val[q];
+            }
+        }
+        __syncthreads();
+    }
+    for (int k = tid; k < n; k += RSS_BLOCK) perm[k] = sval[k];
 }
 
 /* Leaves the sorted permutation in cb.perm (when this cycle sorts). */
 void nbg_launch_spatial_sort(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 {
-    k_sort_decide<<<1, 1, 0, st>>>(ctl);
+    if (cb.cap <= RSS_MAX) {
+        k_sort_small<<<1, RSS_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.perm);
+        return;
+    }
     const int g = nbg_flat_grid(cb, cb.cap);
     k_order_keys<<<g, 256, 0, st>>>(cb.a, ctl, cb.seg, cb.skey[0], cb.perm);
     const int nb = (int)((cb.cap + RS_TILE - 1) / RS_TILE);
@@ -285,10 +406,14 @@ void nbg_launch_spatial_sort(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     unsigned *kin = cb.skey[0], *vin = cb.perm, *kout = cb.skey[1], *vout = cb.sval;
     for (int pass = 0; pass < 4; pass++) {
         const int shift = 8 * pass;
-        k_rs_hist<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, shift, cb.shist);
-        k_rs_scan_part<<<nchunk, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
-        k_rs_scan_top<<<1, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
-        k_rs_scan_fin<<<nchunk, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
+        if (nchunk == 1) {
+            k_rs_hist_scan<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, shift, cb.shist);
+        } else {
+            k_rs_hist<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, shift, cb.shist);
+            k_rs_scan_part<<<nchunk, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
+            k_rs_scan_top<<<1, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
+            k_rs_scan_fin<<<nchunk, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
+        }
         k_rs_scatter<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, vin, kout, vout, shift, cb.shist);
         unsigned *t = kin;
         kin = kout;
@@ -298,6 +423,13 @@ void nbg_launch_spatial_sort(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
         vout = t;
     }
     /* four passes: the result is back in skey[0] / perm */
+}
+
+int nbg_spatial_sort_launches(const CycleBufs &cb)
+{
+    if (cb.cap <= RSS_MAX) return 1;
+    const ll hist = ((cb.cap + RS_TILE - 1) / RS_TILE) * RS_BINS;
+    return 1 + 4 * (hist <= RS_SCAN_CHUNK ? 2 : 5);
 }
 
 /* Events beyond the one-block sort: a stable LSD radix sort of their keys

@@ -361,6 +361,7 @@ static int ensure_cap(nbg_ctx *ctx, ll need, ll keep)
     const ll tiles = (cap + NBG_MIX_MIN_ITILE - 1) / NBG_MIX_MIN_ITILE + NBG_MAX_SIMS + 1;
     CAP_ALLOC(ctx->cb.tile_c, tiles * sizeof(float4));
     CAP_ALLOC(ctx->cb.tile_t, tiles * sizeof(float));
+    CAP_ALLOC(ctx->cb.tile_rng, tiles * sizeof(int2));
     CAP_ALLOC(ctx->cb.iprep, cap * sizeof(float4));
     const ll pdoubles = part_need(ctx, cap);
     CAP_ALLOC(ctx->cb.part, pdoubles * sizeof(double));
@@ -420,6 +421,7 @@ static void free_cap_buffers(CycleBufs &cb)
     cudaFree(cb.jlo);
     cudaFree(cb.tile_c);
     cudaFree(cb.tile_t);
+    cudaFree(cb.tile_rng);
     cudaFree(cb.iprep);
     cudaFree(cb.part);
     cudaFree(cb.perm);
@@ -432,6 +434,7 @@ static void free_cap_buffers(CycleBufs &cb)
     cb.nblk_cap = 0;
     cb.jhi = cb.jlo = cb.tile_c = cb.iprep = nullptr;
     cb.tile_t = nullptr;
+    cb.tile_rng = nullptr;
     cb.part = nullptr;
     cb.part_doubles = 0;
     cb.perm = cb.sval = cb.skey[0] = cb.skey[1] = nullptr;
@@ -1532,8 +1535,7 @@ static void launch_cycle(nbg_ctx *ctx, int precision, long ev_base)
     const CycleBufs &cb = ctx->cb;
     cudaStream_t st = ctx->st;
     if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base), st);
-    nbg_launch_begin(cb, ctx->ctl, st);
-    nbg_launch_frag_count(cb, ctx->ctl, st);
+    nbg_launch_begin_cycle(cb, ctx->ctl, st);
     if (cb.bh) {
         if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 1), st);
         nbg_launch_bh(cb, ctx->ctl, st, precision == NBG_PRECISION_MIXED);
@@ -1552,15 +1554,13 @@ static void launch_cycle(nbg_ctx *ctx, int precision, long ev_base)
     /* the mixed direct path keeps its Hilbert order through compaction */
     nbg_launch_after_pair(cb, ctx->ctl, st, !cb.bh && precision == NBG_PRECISION_MIXED);
     if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 3), st);
-    /* begin, fragment count + scan, 10 after the pair kernel, and the pair
-     * kernel; mixed adds reduce, the sort decision and 21 sort launches
-     * (which return at once in cycles that keep the order), pack, tile
-     * origins, i-body set-up, the output and 4 that carry the order through
-     * compaction; Barnes-Hut replaces the pair kernel (nbg_bh_launches) */
-    ctx->launches_per_cycle = (cb.ev_radix ? nbg_event_radix_launches(cb) : 0) +
-                              (cb.bh ? 13 + nbg_bh_launches(cb, precision == NBG_PRECISION_MIXED)
-                                     : precision == NBG_PRECISION_MIXED ? 45 : 14) +
-                              (cb.ring_head ? 1 : 0);
+    /* the cycle's own, and the force pass: the plain pair kernel, or what
+     * the mixed form and Barnes-Hut count (the sort's launches return at once
+     * in cycles that keep the order) */
+    const bool mixed = precision == NBG_PRECISION_MIXED;
+    ctx->launches_per_cycle = nbg_cycle_launches(cb, !cb.bh && mixed) +
+                              (cb.ev_radix ? nbg_event_radix_launches(cb) : 0) +
+                              (cb.bh ? nbg_bh_launches(cb, mixed) : mixed ? nbg_mixed_launches(cb) : 1) + (cb.ring_head ? 1 : 0);
 }
 
 /* One CUDA graph of ctx->graph_cycles consecutive cycles. */

@@ -93,6 +93,8 @@ struct DevCtl {
     ull bh_rmax;
     unsigned bh_next; /* the walk's next 32-body group (one per warp) */
     unsigned bh_slots; /* the walk's child slots handed out */
+    unsigned ticket;   /* blocks of the running kernel that have arrived (last_block) */
+    unsigned pad3;
     /* Hilbert order of the mixed path (perm): valid while no body changed
      * index; re-sorted when invalid or sort_interval cycles after the last
      * sort (0: NBG_SORT_INTERVAL_DEFAULT).  sort_now is this cycle's decision. */
@@ -104,6 +106,23 @@ struct DevCtl {
 };
 
 #define NBG_SORT_INTERVAL_DEFAULT 4
+
+/* Whether this cycle sorts.  Bodies move a small fraction of a tile's size
+ * per cycle, so an order a few cycles old still gives compact tiles; which i
+ * a tile holds never changes a result's correctness, only its FP32 error
+ * and the near-pair count.  An order is dropped (sort_valid = 0) whenever a
+ * body changes index or the arrays are replaced: compaction, loads, edits,
+ * reallocation, and a cycle that failed and is run again. */
+__device__ __forceinline__ void nbg_sort_decide(DevCtl *ctl)
+{
+    const int k = ctl->sort_interval > 0 ? ctl->sort_interval : NBG_SORT_INTERVAL_DEFAULT;
+    const bool now = !ctl->sort_valid || ctl->cycle - ctl->sort_cycle >= (ull)k;
+    ctl->sort_now = now;
+    if (now) {
+        ctl->sort_valid = 1;
+        ctl->sort_cycle = ctl->cycle;
+    }
+}
 
 /* events sorted by one block in shared memory; more take the multi-block
  * radix sort (when the cycle's launches include it) */
@@ -238,6 +257,7 @@ struct CycleBufs {
     float4 *jhi, *jlo;
     float4 *tile_c;     /* per i-tile: origin (xyz) and a radius holding its bodies (w) */
     float *tile_t;      /* per i-tile: the largest near-pair threshold of its bodies (NULL: not kept) */
+    int2 *tile_rng;     /* per i-tile: the first and last chunk that share it (NULL: not kept) */
     float4 *iprep;      /* per sorted position: re-centred x, y, z and near-pair threshold */
     double *part;
     unsigned *perm;     /* sorted position -> body index */
@@ -428,7 +448,9 @@ int nbg_bh_launches(const CycleBufs &cb, bool mixed); /* kernels nbg_launch_bh l
 
 /* k_cycle.cu (compiled with --fmad=false) */
 void nbg_launch_begin(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
-void nbg_launch_frag_count(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
+/* the start of a whole cycle: begin, and the fragments it emits */
+void nbg_launch_begin_cycle(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
+int nbg_cycle_launches(const CycleBufs &cb, bool carry_order);
 void nbg_launch_pair_fp64(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
 void nbg_launch_after_pair(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool carry_order);
 /* sim < 0: every collection (the whole array) */
@@ -445,12 +467,14 @@ void nbg_launch_gather(const CycleBufs &cb, const BodyArrays &src, const BodyArr
 void nbg_launch_mixed_prep(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
 void nbg_launch_mixed_pair(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
 void nbg_launch_mixed_out(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
+int nbg_mixed_launches(const CycleBufs &cb); /* kernels of a mixed force pass, after begin */
 int nbg_mixed_slots(int device, int variant);
 ll nbg_sym_units(ll blocks);
 MixVariantInfo nbg_mix_variant_info(int variant);
 
 /* k_sort.cu */
 void nbg_launch_spatial_sort(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
+int nbg_spatial_sort_launches(const CycleBufs &cb);
 void nbg_launch_event_radix(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
 ull *nbg_launch_incidence_radix(const CycleBufs &cb, DevCtl *ctl, int bits, cudaStream_t st);
 int nbg_event_radix_launches(const CycleBufs &cb);
