@@ -210,11 +210,23 @@ __device__ __forceinline__ float4 i_body_setup(const float4 &h, const float4 &l,
     return make_float4(xr, yr, zr, __double2float_ru(b * b));
 }
 
+__device__ __forceinline__ float amax_of(float x, float y, float z) { return fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))); }
+
+/* near_kappa for a collection of n bodies.  In a small one, one or two tiles
+ * span it all, so a body's offset from its tile origin is large next to its
+ * neighbours' distances, and the neighbours carry much of its force: twice the
+ * factor there.  Such collections hold a small share of the work. */
+__device__ __forceinline__ double near_kappa_of(const DevCtl *ctl, ll n)
+{
+    return n <= NBG_NEAR_SMALL_N ? 2.0 * (double)ctl->near_kappa : (double)ctl->near_kappa;
+}
+
 /* Everything the pair kernel reads of a tile, one CTA a tile: its bodies
  * packed in sorted order, its origin (the centre of their bounding box) and a
  * radius that holds them, each i-body's re-centred position and near-pair
- * threshold, the largest threshold, and the chunks that share the tile
- * (tile_rng, if given) for k_mix_out.  One launch where packing, tile origins
+ * threshold, the tile's largest re-centred coordinate and radius (tile_r, if
+ * given), and the chunks that share the tile (tile_rng, if given) for
+ * k_mix_out.  One launch where packing, tile origins
  * and i-bodies were three, each reading back what the one before wrote:
  * 19.3 -> 13.4 us for 2,501 bodies, 29.5 -> 13.6 us for 20,011 (one launch
  * each under the profiler, caches cold). */
@@ -222,19 +234,18 @@ __device__ __forceinline__ float4 i_body_setup(const float4 &h, const float4 &l,
 #define TILES_ITEMS (NBG_MIX_MAX_ITILE / TILES_BLOCK)
 __global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl *ctl, SimSegs seg,
                                                            const unsigned *__restrict__ perm, float4 *jhi, float4 *jlo,
-                                                           float4 *tile_c, float *tile_t, float4 *iprep,
+                                                           float4 *tile_c, float2 *tile_r, float4 *iprep,
                                                            int2 *tile_rng, int itile)
 {
     __shared__ float red[6][TILES_BLOCK / 32];
     __shared__ float4 s_c;
-    __shared__ unsigned s_t;
+    __shared__ unsigned s_r[2];
     if (ctl->error) return;
     const ll ntiles = seg.mtile_off[seg.nsims];
     double ms = ctl->m_scale;
     if (!(ms > 0.0)) ms = 1.0;
     const float rmax = __uint_as_float(ctl->rmax_bits);
     const float xmax = __uint_as_float(ctl->xmax_bits);
-    const double kappa0 = (double)ctl->near_kappa;
     const int tid = threadIdx.x, w = tid >> 5;
     for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int sim = nbg_sim_of(seg.mtile_off, seg.nsims, tile);
@@ -287,7 +298,7 @@ __global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl 
              * rounded up past the FP32 arithmetic and the bodies' lo parts */
             const float rad = sqrtf(e2) * (1.0f + 0x1p-16f) + amax * 0x1p-20f;
             s_c = make_float4(c3[0], c3[1], c3[2], rad);
-            s_t = 0u;
+            s_r[0] = s_r[1] = 0u;
             tile_c[tile] = s_c;
         }
         if (tile_rng && (tid == 32 || tid == 64)) {
@@ -297,28 +308,102 @@ __global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl 
         }
         __syncthreads();
         const float4 c = s_c;
-        /* In a small collection one or two tiles span it all, so a body's
-         * offset from its tile origin is large next to its neighbours'
-         * distances, and the neighbours carry much of its force: twice the
-         * factor there.  Such collections hold a small share of the work. */
-        const double kappa = s1 - s0 <= NBG_NEAR_SMALL_N ? 2.0 * kappa0 : kappa0;
-        float tmax = 0.f;
+        const double kappa = near_kappa_of(ctl, s1 - s0);
+        float amax = 0.f, rad = 0.f;
 #pragma unroll
         for (int q = 0; q < TILES_ITEMS; q++) {
             const ll p = base + q * TILES_BLOCK + tid;
             if (p >= n) continue;
             const float4 v = i_body_setup(h[q], l[q], c, rmax, xmax, kappa);
             iprep[p] = v;
-            tmax = fmaxf(tmax, v.w);
+            if (packed_special(l[q])) continue;
+            amax = fmaxf(amax, amax_of(v.x, v.y, v.z));
+            rad = fmaxf(rad, l[q].w);
         }
-        if (tile_t) {
+        if (tile_r) {
             /* positive floats order as their bit patterns */
-            const unsigned m = __reduce_max_sync(FULL_MASK, __float_as_uint(tmax));
-            if ((tid & 31) == 0) atomicMax(&s_t, m);
+            const unsigned ma = __reduce_max_sync(FULL_MASK, __float_as_uint(amax));
+            const unsigned mr = __reduce_max_sync(FULL_MASK, __float_as_uint(rad * (1.0f + 0x1p-20f)));
+            if ((tid & 31) == 0) {
+                atomicMax(&s_r[0], ma);
+                atomicMax(&s_r[1], mr);
+            }
             __syncthreads();
-            if (tid == 0) tile_t[tile] = __uint_as_float(s_t);
+            if (tid == 0) tile_r[tile] = make_float2(__uint_as_float(s_r[0]), __uint_as_float(s_r[1]));
         }
         __syncthreads(); /* the shared values are rewritten by the next tile */
+    }
+}
+
+/* The near-pair thresholds of i_body_setup reach as far as the largest body
+ * of all, so one star in a disk makes near pairs of every body's nearest 60.
+ * Here each tile's bodies get their thresholds against the largest radius R
+ * among the tiles that could hold a body touching one of theirs (by the
+ * tiles' bounding spheres and largest radii); a pair across any other two
+ * tiles cannot overlap.  FP32, with margins that cover its roundings (a few
+ * times 2^-24 each); a threshold never grows.  One CTA a tile, after
+ * k_mix_tiles.  The one-sided pair pass of a 131,072-body disk around a body
+ * of radius 20 takes 6.36 ms instead of 7.10 ms; below REACH_MIN_CAP bodies
+ * there are too few tiles for one to keep clear of the large body's.  (The
+ * symmetric kernel forms its thresholds per pair of blocks instead.) */
+#define REACH_MIN_CAP 32768
+__device__ __forceinline__ float touch_distance(float amax, float r, float R, float xmax)
+{
+    const float D = fmaxf(0.f, (r + fabsf(r) * 0x1p-22f) + R);
+    return (D + (0x1p-19f * (amax + D) + 0x1p-44f * xmax + 0x1p-100f)) * (1.0f + 0x1p-17f);
+}
+
+/* the near-pair threshold on r^2 of a body with largest re-centred coordinate
+ * amax and radius r (or of several, given the largest of each) against bodies
+ * of radius at most R; t is its threshold against r_max, which it never
+ * exceeds */
+__device__ __forceinline__ float near_threshold(float amax, float r, float R, float xmax, float kappa, float t)
+{
+    const float b = fmaxf(touch_distance(amax, r, R, xmax), kappa * amax * (1.0f + 0x1p-17f));
+    return fminf(t, b * b * (1.0f + 0x1p-20f));
+}
+
+__global__ void __launch_bounds__(TILES_BLOCK) k_mix_reach(DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jlo,
+                                                           const float4 *__restrict__ tile_c,
+                                                           const float2 *__restrict__ tile_r, float4 *iprep,
+                                                           int itile)
+{
+    __shared__ unsigned s_R;
+    if (ctl->error) return;
+    const ll ntiles = seg.mtile_off[seg.nsims];
+    const float rmax = __uint_as_float(ctl->rmax_bits), xmax = __uint_as_float(ctl->xmax_bits);
+    const int tid = threadIdx.x;
+    for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int sim = nbg_sim_of(seg.mtile_off, seg.nsims, tile);
+        const ll s0 = seg.off[sim], s1 = seg.off[sim + 1];
+        const float4 c = tile_c[tile];
+        const float2 mine = tile_r[tile];
+        if (tid == 0) s_R = 0u;
+        __syncthreads();
+        float R = 0.f;
+        for (ll o = seg.mtile_off[sim] + tid; o < seg.mtile_off[sim + 1]; o += TILES_BLOCK) {
+            const float rb = tile_r[o].y;
+            if (!(rb > R)) continue;
+            const float4 d = tile_c[o];
+            const float ex = d.x - c.x, ey = d.y - c.y, ez = d.z - c.z;
+            const float gap = sqrtf(ex * ex + ey * ey + ez * ez) * (1.0f - 0x1p-18f) - c.w - d.w;
+            if (!(gap > touch_distance(mine.x, mine.y, rb, xmax) * (1.0f + 0x1p-10f))) R = rb;
+        }
+        /* positive floats order as their bit patterns */
+        const unsigned m = __reduce_max_sync(FULL_MASK, __float_as_uint(R));
+        if ((tid & 31) == 0) atomicMax(&s_R, m);
+        __syncthreads();
+        R = __uint_as_float(s_R);
+        if (R < rmax) {
+            const float kappa = (float)near_kappa_of(ctl, s1 - s0);
+            const ll base = s0 + (tile - seg.mtile_off[sim]) * itile;
+            const ll n = s1 < base + itile ? s1 : base + itile;
+            for (ll p = base + tid; p < n; p += TILES_BLOCK) {
+                const float4 v = iprep[p];
+                iprep[p].w = near_threshold(amax_of(v.x, v.y, v.z), jlo[p].w, R, xmax, kappa, v.w);
+            }
+        }
+        __syncthreads(); /* s_R is rewritten by the next tile */
     }
 }
 
@@ -899,15 +984,20 @@ __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A
  * A diagonal unit (a == a) is one-sided: every body of the block against
  * every other, i-sums only (both directions of each pair are in the block).
  *
- * Near pairs.  A pair closer than the i-body's near-pair threshold (the one
- * the one-sided kernel uses, from the i-side error bound, which the shared dx
- * carries to both directions) is masked out of both fast sums.  After the
- * unit, the lanes that met one re-evaluate their near pairs exactly in FP64
- * (candidate_pair: the reference's expressions, the overlap skip, the event
- * i -> j), and the owners of the j that were met re-evaluate the same pairs
- * from their side (the event j -> i and the j term).  Both sides decide
- * "near" with the same FP32 expression, so they agree pair by pair.  Every
- * sum is formed in a fixed order: results do not depend on scheduling.
+ * Near pairs.  A pair closer than the i-body's near-pair threshold against
+ * block b (from the i-side error bound, which the shared dx carries to both
+ * directions) is masked out of both fast sums.  After the unit, each warp
+ * looks over block b for its flagged i-bodies, 32 j at a time, and evaluates
+ * the near pairs it lists 32 at a time in FP64 (candidate_pair: the
+ * reference's expressions, the overlap skip, the event i -> j); then over
+ * block a for the j that were met (the event j -> i and the j term).  Both
+ * sides decide "near" with the same FP32 expression, so they agree pair by
+ * pair.  Every sum is formed in a fixed order: results do not depend on
+ * scheduling.  What a unit costs is the rotation, 183,000 cycles far and
+ * 200,000 masked, plus the near pairs: with each lane evaluating its own,
+ * one after the other, the largest unit of a 131,072-body Plummer + disk took 5
+ * million cycles, half of the pass (6.81 ms; now 5.80; the disk 9.69 -> 6.31,
+ * the uniform ball 5.45 -> 5.09).
  *
  * Sums.  i-sums fold into (hi, lo) pairs every 256 j and go to the one-sided
  * kernel's per-(row, chunk) FP64 slots; j-sums of a unit (128 terms per
@@ -951,10 +1041,68 @@ __device__ __forceinline__ float sym_r2(float xj, float yj, float zj, float nxi,
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
+/* A warp's near pairs of one unit, as (own, other) indices in two blocks, with
+ * each own body's pairs in a run.  drain() evaluates 32 at a time, one a lane
+ * (candidate_pair: FP64), and hands each own body's sum over the batch, in
+ * list order, to add(own, x, y, z).  The whole warp calls every member. */
+#define SYM_LIST 64
+struct SymNear {
+    unsigned *list; /* shared: own << 16 | other */
+    int cnt;
+
+    template <class ADD>
+    __device__ __forceinline__ void drain(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
+                                          const unsigned *__restrict__ perm, ll own0, ll oth0, ADD add)
+    {
+        const int lane = threadIdx.x & 31;
+        double ms = ctl->m_scale;
+        if (!(ms > 0.0)) ms = 1.0;
+        const double inv_ms = 1.0 / ms;
+        __syncwarp();
+        for (int b = 0; b < cnt; b += 32) {
+            const bool live = b + lane < cnt;
+            const unsigned e = live ? list[b + lane] : 0xffffffffu;
+            const unsigned own = e >> 16;
+            double tx = 0.0, ty = 0.0, tz = 0.0;
+            if (live)
+                candidate_pair(A, ctl, ev_keys, ev_cap, (ll)perm[own0 + own], (ll)perm[oth0 + (e & 0xffffu)], inv_ms,
+                               tx, ty, tz);
+            __syncwarp();
+            /* a run's first lane gathers it */
+            const unsigned run = __match_any_sync(FULL_MASK, own);
+            const bool first = live && __ffs(run) - 1 == lane;
+            const int len = first ? __popc(run) : 0;
+            const int most = __reduce_max_sync(FULL_MASK, len);
+            double sx = tx, sy = ty, sz = tz;
+            for (int d = 1; d < most; d++) {
+                const double ux = __shfl_down_sync(FULL_MASK, tx, d), uy = __shfl_down_sync(FULL_MASK, ty, d),
+                             uz = __shfl_down_sync(FULL_MASK, tz, d);
+                if (d < len) {
+                    sx += ux;
+                    sy += uy;
+                    sz += uz;
+                }
+            }
+            if (first) add((int)own, sx, sy, sz);
+        }
+        cnt = 0;
+        __syncwarp();
+    }
+
+    /* room for 32 more (drain() when false) */
+    __device__ __forceinline__ bool room() const { return cnt + 32 <= SYM_LIST; }
+    __device__ __forceinline__ void push(bool hit, unsigned own, unsigned other)
+    {
+        const unsigned m = __ballot_sync(FULL_MASK, hit);
+        if (hit) list[cnt + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = own << 16 | other;
+        cnt += __popc(m);
+    }
+};
+
 template <int MINB>
 __global__ void __launch_bounds__(SYM_THREADS, MINB)
-k_pair_sym(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi, const float4 *__restrict__ jlo,
-           const float4 *__restrict__ tile_c, const float *__restrict__ tile_t, const float4 *__restrict__ iprep,
+k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi, const float4 *__restrict__ jlo,
+           const float4 *__restrict__ tile_c, const float2 *__restrict__ tile_r, const float4 *__restrict__ iprep,
            const unsigned *__restrict__ perm, double *__restrict__ part, float *__restrict__ jpart, ull *ev_keys,
            ll ev_cap)
 {
@@ -964,13 +1112,13 @@ k_pair_sym(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jh
     __shared__ float2 jacc[SYM_WARPS][3][SYM_JP]; /* per-warp j sums of the unit */
     __shared__ float sfold[6][SYM_B];             /* i sums: (hi, lo) per component */
     __shared__ unsigned char jnear[SYM_B];        /* j met a near pair in this unit */
+    __shared__ float sthr[SYM_B];                 /* block a's thresholds against block b */
+    __shared__ unsigned s_list[SYM_WARPS][SYM_LIST];
     __shared__ ll s_chunk;
     if (ctl->error) return;
     const int C = ctl->splits;
     const ll W = ctl->work_total;
-    double ms = ctl->m_scale;
-    if (!(ms > 0.0)) ms = 1.0;
-    const double inv_ms = 1.0 / ms;
+    const float xmax = __uint_as_float(ctl->xmax_bits);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int src = (lane + 1) & 31;
 
@@ -996,27 +1144,26 @@ k_pair_sym(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jh
         const float4 c = tile_c[g];
 
         /* block a: re-centred positions (negated, duplicated for the packed
-         * arithmetic), thresholds, and masses (negated) for the j terms;
+         * arithmetic) and masses (negated) for the j terms;
          * slots past the collection sit at the sentinel, massless */
         float2 nx[SYM_KI], ny[SYM_KI], nz[SYM_KI], nm[SYM_KI];
-        float thr[SYM_KI];
+        const float2 ra = tile_r[g];
+        const float kappa = (float)near_kappa_of(ctl, n - s0);
 #pragma unroll
         for (int k = 0; k < SYM_KI; k++) {
             const ll p = ibase + (ll)k * SYM_THREADS + tid;
-            float xr = SENTINEL_POS, yr = SENTINEL_POS, zr = SENTINEL_POS, t = -1.f, m = 0.f;
+            float xr = SENTINEL_POS, yr = SENTINEL_POS, zr = SENTINEL_POS, m = 0.f;
             if (p < n) {
                 const float4 q = iprep[p];
                 xr = q.x;
                 yr = q.y;
                 zr = q.z;
-                t = q.w;
                 m = jhi[p].w;
             }
             nx[k] = make_float2(-xr, -xr);
             ny[k] = make_float2(-yr, -yr);
             nz[k] = make_float2(-zr, -zr);
             nm[k] = make_float2(-m, -m);
-            thr[k] = t;
 #pragma unroll
             for (int cc = 0; cc < 6; cc++) sfold[cc][k * SYM_THREADS + tid] = 0.f;
         }
@@ -1071,14 +1218,27 @@ k_pair_sym(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jh
                 }
             };
             /* A unit whose blocks' bounding spheres lie farther apart than
-             * block a's largest near-pair radius holds no near pair: its
-             * loop needs no mask (uniform over the CTA). */
+             * block a's largest near-pair radius against block b holds no
+             * near pair: its loop needs no mask (uniform over the CTA). */
             bool far = false;
+            const float R = tile_r[seg.mtile_off[sim] + bb].y;
             if (!diag) {
                 const float4 cj = tile_c[seg.mtile_off[sim] + bb];
                 const float ex = cj.x - c.x, ey = cj.y - c.y, ez = cj.z - c.z;
                 const float gap = sqrtf(ex * ex + ey * ey + ez * ez) * (1.0f - 0x1p-18f) - c.w - cj.w;
-                far = gap > 0.f && gap * gap > tile_t[g] * (1.0f + 0x1p-10f);
+                far = gap > 0.f && gap * gap > near_threshold(ra.x, ra.y, R, xmax, kappa, 3.0e38f) * (1.0f + 0x1p-10f);
+            }
+            float thr[SYM_KI];
+            if (!far) {
+#pragma unroll
+                for (int k = 0; k < SYM_KI; k++) {
+                    const ll p = ibase + (ll)k * SYM_THREADS + tid;
+                    thr[k] = -1.f;
+                    if (p < n)
+                        thr[k] = near_threshold(amax_of(nx[k].x, ny[k].x, nz[k].x), jlo[p].w, R, xmax, kappa,
+                                                iprep[p].w);
+                    sthr[k * SYM_THREADS + tid] = thr[k];
+                }
             }
             auto rotate = [&](auto masked) {
                 constexpr bool MASK = decltype(masked)::value;
@@ -1171,34 +1331,44 @@ k_pair_sym(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jh
                     if (selfnear[k] > 1) nearmask |= 1u << k;
             }
 
-            /* exact pass, i side: this thread's near pairs, j in block order */
+            /* exact pass, i side: the warp looks over block b for each of its
+             * flagged i-bodies in turn, 32 j at a time */
+            if (!far && __any_sync(FULL_MASK, nearmask != 0)) {
+                SymNear near = {s_list[w], 0};
+                auto add = [&](int own, double ux, double uy, double uz) {
+                    fold64(sfold[0][own], sfold[1][own], ux);
+                    fold64(sfold[2][own], sfold[3][own], uy);
+                    fold64(sfold[4][own], sfold[5][own], uz);
+                };
+                const int jn = (int)(n - jb < SYM_B ? n - jb : SYM_B);
+                unsigned who = 0;
 #pragma unroll
-            for (int k = 0; k < SYM_KI; k++) {
-                if (!(nearmask & (1u << k))) continue;
-                const int li = k * SYM_THREADS + tid;
-                const ll p = ibase + li;
-                const ll i = perm[p];
-                for (int jj = 0; jj < SYM_B; jj++) {
-                    const ll q = jb + jj;
-                    if (q >= n || (diag && jj == li)) continue;
-                    const float4 qa = sA[jj >> 1], qb = sB[jj >> 1];
-                    const int e = jj & 1;
-                    const float r2 = sym_r2(e ? qa.y : qa.x, e ? qa.w : qa.z, e ? qb.y : qb.x, nx[k].x, ny[k].x,
-                                            nz[k].x);
-                    if (!(r2 < thr[k])) continue;
-                    double tx, ty, tz;
-                    candidate_pair(A, ctl, ev_keys, ev_cap, i, (ll)perm[q], inv_ms, tx, ty, tz);
-                    fold64(sfold[0][li], sfold[1][li], tx);
-                    fold64(sfold[2][li], sfold[3][li], ty);
-                    fold64(sfold[4][li], sfold[5][li], tz);
-                    jnear[jj] = 1;
+                for (int k = 0; k < SYM_KI; k++) {
+                    who = __ballot_sync(FULL_MASK, nearmask & (1u << k));
+                    while (who) {
+                        const int l = __ffs(who) - 1;
+                        who &= who - 1u;
+                        const int own = k * SYM_THREADS + w * 32 + l;
+                        const float xi = __shfl_sync(FULL_MASK, nx[k].x, l), yi = __shfl_sync(FULL_MASK, ny[k].x, l),
+                                    zi = __shfl_sync(FULL_MASK, nz[k].x, l), ti = __shfl_sync(FULL_MASK, thr[k], l);
+#pragma unroll 1
+                        for (int j0 = 0; j0 < jn; j0 += 32) {
+                            const int jj = j0 + lane, e = jj & 1;
+                            const float4 qa = sA[jj >> 1], qb = sB[jj >> 1];
+                            const float r2 = sym_r2(e ? qa.y : qa.x, e ? qa.w : qa.z, e ? qb.y : qb.x, xi, yi, zi);
+                            const bool hit = r2 < ti && jj < jn && !(diag && jj == own);
+                            if (hit) jnear[jj] = 1;
+                            if (!near.room()) near.drain(A, ctl, ev_keys, ev_cap, perm, ibase, jb, add);
+                            near.push(hit, own, jj);
+                        }
+                    }
                 }
+                near.drain(A, ctl, ev_keys, ev_cap, perm, ibase, jb, add);
             }
             if (diag) continue; /* a diagonal unit has no j slot */
             __syncthreads(); /* jacc and jnear complete */
 
-            /* j side: the unit's sums in warp order, plus the exact terms of
-             * the j that met a near pair, i in block order */
+            /* j side: the unit's sums in warp order */
             float *jo = jpart + u * 3 * SYM_B;
             for (int jj = tid; jj < SYM_B; jj += SYM_THREADS) {
                 const int pp = jj >> 1, e = jj & 1;
@@ -1209,31 +1379,42 @@ k_pair_sym(BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jh
                     sy += e ? jacc[ww][1][pp].y : jacc[ww][1][pp].x;
                     sz += e ? jacc[ww][2][pp].y : jacc[ww][2][pp].x;
                 }
-                const ll q = jb + jj;
-                if (jnear[jj] && q < n) {
-                    const float4 qa = sA[pp], qb = sB[pp];
-                    const float xj = e ? qa.y : qa.x, yj = e ? qa.w : qa.z, zj = e ? qb.y : qb.x;
-                    const ll j = perm[q];
-                    double ex = 0.0, ey = 0.0, ez = 0.0;
-                    for (int ii = 0; ii < SYM_B; ii++) {
-                        const ll p = ibase + ii;
-                        if (p >= n) break;
-                        const float4 ip = iprep[p];
-                        const float r2 = sym_r2(xj, yj, zj, -ip.x, -ip.y, -ip.z);
-                        if (!(r2 < ip.w)) continue;
-                        double tx, ty, tz;
-                        candidate_pair(A, ctl, ev_keys, ev_cap, j, (ll)perm[p], inv_ms, tx, ty, tz);
-                        ex += tx;
-                        ey += ty;
-                        ez += tz;
-                    }
-                    sx = (float)((double)sx + ex);
-                    sy = (float)((double)sy + ey);
-                    sz = (float)((double)sz + ez);
-                }
                 jo[jj] = sx;
                 jo[SYM_B + jj] = sy;
                 jo[2 * SYM_B + jj] = sz;
+            }
+            if (far) continue;
+            /* exact pass, j side: for each j that met a near pair, block a */
+            __syncthreads(); /* the sums are written */
+            {
+                SymNear near = {s_list[w], 0};
+                auto add = [&](int own, double ux, double uy, double uz) {
+                    jo[own] = (float)((double)jo[own] + ux);
+                    jo[SYM_B + own] = (float)((double)jo[SYM_B + own] + uy);
+                    jo[2 * SYM_B + own] = (float)((double)jo[2 * SYM_B + own] + uz);
+                };
+                const int in = (int)(n - ibase < SYM_B ? n - ibase : SYM_B);
+                for (int j0 = w * 32; j0 < SYM_B; j0 += SYM_THREADS) {
+                    unsigned who = __ballot_sync(FULL_MASK, jnear[j0 + lane] != 0);
+                    while (who) {
+                        const int jj = j0 + __ffs(who) - 1, e = jj & 1;
+                        who &= who - 1u;
+                        const float4 qa = sA[jj >> 1], qb = sB[jj >> 1];
+                        const float xj = e ? qa.y : qa.x, yj = e ? qa.w : qa.z, zj = e ? qb.y : qb.x;
+#pragma unroll 1
+                        for (int i0 = 0; i0 < in; i0 += 32) {
+                            const int ii = i0 + lane;
+                            bool hit = false;
+                            if (ii < in) {
+                                const float4 ip = iprep[ibase + ii];
+                                hit = sym_r2(xj, yj, zj, -ip.x, -ip.y, -ip.z) < sthr[ii];
+                            }
+                            if (!near.room()) near.drain(A, ctl, ev_keys, ev_cap, perm, jb, ibase, add);
+                            near.push(hit, jj, ii);
+                        }
+                    }
+                }
+                near.drain(A, ctl, ev_keys, ev_cap, perm, jb, ibase, add);
             }
         }
         /* this chunk's share of row a's i sums: slot g + chunk */
@@ -1345,7 +1526,8 @@ __global__ void k_sym_out(BodyArrays A, DevCtl *ctl, SimSegs seg, const unsigned
 /* the kernel of a shape */
 #define MIX_KERNEL(kind, b, k, jt, u, mb) k_pair_mixed<b, k, jt, u, mb, (kind) >= 1, (kind) == 2, (kind) == 3>
 
-/* the symmetric kernel's shapes: registers capped for 4 or 5 CTAs per SM */
+/* the symmetric kernel's shapes: registers capped for 4 or 5 CTAs per SM
+ * (shared memory holds 4) */
 #define SYM_MINB_A 4
 #define SYM_MINB_B 5
 
@@ -1393,6 +1575,10 @@ int nbg_mixed_slots(int device, int variant)
     return slots;
 }
 
+static int mix_reach(const CycleBufs &cb)
+{
+    return cb.tile_r && cb.cap >= REACH_MIN_CAP && !nbg_mix_is_sym(cb.mix_variant);
+}
 
 void nbg_launch_mixed_prep(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 {
@@ -1402,12 +1588,16 @@ void nbg_launch_mixed_prep(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     const int itile = cb.itile > 0 ? cb.itile : NBG_MIX_ITILE;
     ll tiles = (cb.cap + itile - 1) / itile + cb.seg.nsims;
     if (tiles > (ll)(cb.sms > 0 ? cb.sms : 1) * 64) tiles = (ll)(cb.sms > 0 ? cb.sms : 1) * 64;
-    k_mix_tiles<<<(int)tiles, TILES_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.perm, cb.jhi, cb.jlo, cb.tile_c, cb.tile_t,
-                                                    cb.iprep, nbg_mix_is_sym(cb.mix_variant) ? nullptr : cb.tile_rng,
-                                                    itile);
+    k_mix_tiles<<<(int)tiles, TILES_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.perm, cb.jhi, cb.jlo, cb.tile_c,
+                                                    mix_reach(cb) || nbg_mix_is_sym(cb.mix_variant) ? cb.tile_r : nullptr,
+                                                    cb.iprep,
+                                                    nbg_mix_is_sym(cb.mix_variant) ? nullptr : cb.tile_rng, itile);
+    if (mix_reach(cb))
+        k_mix_reach<<<(int)tiles, TILES_BLOCK, 0, st>>>(ctl, cb.seg, cb.jlo, cb.tile_c, cb.tile_r, cb.iprep,
+                                                        itile);
 }
 
-int nbg_mixed_launches(const CycleBufs &cb) { return 4 + nbg_spatial_sort_launches(cb); }
+int nbg_mixed_launches(const CycleBufs &cb) { return 4 + mix_reach(cb) + nbg_spatial_sort_launches(cb); }
 
 void nbg_launch_mixed_pair(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 {
@@ -1422,12 +1612,12 @@ void nbg_launch_mixed_pair(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 #undef X
     case NBG_MIX_SYM:
         k_pair_sym<SYM_MINB_A><<<cb.slots, SYM_THREADS, 0, st>>>(cb.a, ctl, cb.seg, cb.jhi, cb.jlo, cb.tile_c,
-                                                                 cb.tile_t, cb.iprep, cb.perm, cb.part, cb.jpart,
+                                                                 cb.tile_r, cb.iprep, cb.perm, cb.part, cb.jpart,
                                                                  cb.ev_keys, cb.ev_cap);
         break;
     case NBG_MIX_SYM + 1:
         k_pair_sym<SYM_MINB_B><<<cb.slots, SYM_THREADS, 0, st>>>(cb.a, ctl, cb.seg, cb.jhi, cb.jlo, cb.tile_c,
-                                                                 cb.tile_t, cb.iprep, cb.perm, cb.part, cb.jpart,
+                                                                 cb.tile_r, cb.iprep, cb.perm, cb.part, cb.jpart,
                                                                  cb.ev_keys, cb.ev_cap);
         break;
     }

@@ -360,7 +360,7 @@ static int ensure_cap(nbg_ctx *ctx, ll need, ll keep)
     /* every sim may end in a partial tile: at most cap / itile + nsims tiles */
     const ll tiles = (cap + NBG_MIX_MIN_ITILE - 1) / NBG_MIX_MIN_ITILE + NBG_MAX_SIMS + 1;
     CAP_ALLOC(ctx->cb.tile_c, tiles * sizeof(float4));
-    CAP_ALLOC(ctx->cb.tile_t, tiles * sizeof(float));
+    CAP_ALLOC(ctx->cb.tile_r, tiles * sizeof(float2));
     CAP_ALLOC(ctx->cb.tile_rng, tiles * sizeof(int2));
     CAP_ALLOC(ctx->cb.iprep, cap * sizeof(float4));
     const ll pdoubles = part_need(ctx, cap);
@@ -420,7 +420,7 @@ static void free_cap_buffers(CycleBufs &cb)
     cudaFree(cb.jhi);
     cudaFree(cb.jlo);
     cudaFree(cb.tile_c);
-    cudaFree(cb.tile_t);
+    cudaFree(cb.tile_r);
     cudaFree(cb.tile_rng);
     cudaFree(cb.iprep);
     cudaFree(cb.part);
@@ -433,7 +433,7 @@ static void free_cap_buffers(CycleBufs &cb)
     cb.blk_sum = cb.blk_off = nullptr;
     cb.nblk_cap = 0;
     cb.jhi = cb.jlo = cb.tile_c = cb.iprep = nullptr;
-    cb.tile_t = nullptr;
+    cb.tile_r = nullptr;
     cb.tile_rng = nullptr;
     cb.part = nullptr;
     cb.part_doubles = 0;

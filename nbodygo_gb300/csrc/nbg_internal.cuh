@@ -256,7 +256,7 @@ struct CycleBufs {
     /* mixed form (indexed by sorted position) */
     float4 *jhi, *jlo;
     float4 *tile_c;     /* per i-tile: origin (xyz) and a radius holding its bodies (w) */
-    float *tile_t;      /* per i-tile: the largest near-pair threshold of its bodies (NULL: not kept) */
+    float2 *tile_r;     /* per i-tile: its bodies' largest re-centred coordinate and radius (NULL: not kept) */
     int2 *tile_rng;     /* per i-tile: the first and last chunk that share it (NULL: not kept) */
     float4 *iprep;      /* per sorted position: re-centred x, y, z and near-pair threshold */
     double *part;
