@@ -369,7 +369,12 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
 #define NBG_OPT_EV_CAP 3     /* event-list capacity (rounded up to a power of two) */
 #define NBG_OPT_FRAG_CAP 4   /* fragments one cycle may emit */
 #define NBG_OPT_GRAPH_CYCLES 6 /* cycles captured in one CUDA graph (default 1) */
-#define NBG_OPT_MIX_SHAPE 7    /* shape of the mixed pair kernel, 0..NBG_MIX_SHAPES-1 (see nbg_autotune) */
+/* shape of the mixed pair kernel, 0..NBG_MIX_SHAPES-1 (see nbg_autotune).  A
+ * context that was neither given one nor tuned nor restored from a snapshot takes a
+ * one-sided shape (6 for fewer than 32,768 bodies in all, 2 for more), or 15
+ * (symmetric) when every loaded collection has 114,688 bodies or more and the j
+ * partials fit in an eighth of the device's memory. */
+#define NBG_OPT_MIX_SHAPE 7
 #define NBG_MIX_SHAPES 19
 /* 1: forces from the Barnes-Hut octree of cmd/body/octree.go (opening angle
  * 0.3, softening 1e-4, suns summed directly) with the FP64 arithmetic of the

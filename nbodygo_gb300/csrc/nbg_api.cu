@@ -67,6 +67,8 @@ struct nbg_ctx {
     /* collection of each staged add, in the order of cb.adds: grouped by
      * collection, arrival order within one (the order k_append_adds reads) */
     std::vector<int> add_sim;
+    int shape_given = 0; /* the mixed kernel's shape was set or tuned (1), restored from a snapshot (2) */
+    unsigned long long device_bytes = 0;
     bool timing = false;
     nbg_timing tacc{};
     std::vector<cudaEvent_t> evs;
@@ -441,6 +443,10 @@ static void free_cap_buffers(CycleBufs &cb)
     cb.shist = nullptr;
 }
 
+extern "C" {
+static int select_variant(nbg_ctx *ctx, int v);
+}
+
 /* the symmetric mixed kernel's j-partial slots: at least `need` units (with
  * a quarter to spare, as collections grow by fragments and adds) */
 static int ensure_jpart(nbg_ctx *ctx, ll need)
@@ -460,6 +466,16 @@ static int ensure_jpart(nbg_ctx *ctx, ll need)
     ctx->cb.jpart_units = units;
     invalidate_graph(ctx);
     return NBG_OK;
+}
+
+/* the same for a running cycle: a shape that was not asked for gives way to
+ * the one-sided kernel where its j partials do not fit */
+static int grow_jpart(nbg_ctx *ctx, ll need)
+{
+    const int rc = ensure_jpart(ctx, need);
+    if (rc == NBG_OK || ctx->shape_given == 1) return rc;
+    cudaGetLastError();
+    return select_variant(ctx, NBG_MIX_ONE_SIDED);
 }
 
 static int ensure_frag_cap(nbg_ctx *ctx, ll need)
@@ -845,9 +861,12 @@ int nbg_create(int device, int precision, int64_t capacity, nbg_ctx **out)
             break;
         }
         ctx->cb.work_cap = 0;
-        ctx->cb.mix_variant = 0;
-        ctx->cb.itile = nbg_mix_variant_info(0).block * nbg_mix_variant_info(0).k;
-        ctx->cb.slots = nbg_mixed_slots(device, 0);
+        ctx->cb.mix_variant = NBG_MIX_ONE_SIDED_FEW;
+        ctx->cb.itile =
+            nbg_mix_variant_info(NBG_MIX_ONE_SIDED_FEW).block * nbg_mix_variant_info(NBG_MIX_ONE_SIDED_FEW).k;
+        ctx->cb.slots = nbg_mixed_slots(device, NBG_MIX_ONE_SIDED_FEW);
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) ctx->device_bytes = total_b;
         ctx->cb.sms = 0;
         cudaDeviceGetAttribute(&ctx->cb.sms, cudaDevAttrMultiProcessorCount, device);
         if (ctx->cb.sms < 1) ctx->cb.sms = 1;
@@ -991,6 +1010,10 @@ int nbg_set_collections(nbg_ctx *ctx, int64_t nsims, const int64_t *counts, cons
     bool reshaped = false;
     if ((rc = set_segments(ctx, (int)nsims, (const ll *)counts, &reshaped)) != NBG_OK) return rc;
     if (reshaped) invalidate_graph(ctx);
+    if (!ctx->shape_given) {
+        const int v = nbg_default_shape((int)nsims, (const ll *)counts, ctx->device_bytes);
+        if (v != ctx->cb.mix_variant && (rc = select_variant(ctx, v)) != NBG_OK) return rc;
+    }
     k_set_loaded<<<1, 1, 0, ctx->st>>>(ctx->ctl, n);
     CK(cudaGetLastError());
     ctx->n_host = n;
@@ -1307,7 +1330,6 @@ int nbg_get_body_in(nbg_ctx *ctx, int64_t sim, int64_t id, nbg_soa *h, int32_t *
  *     current, so the FP32 pair sums group the same bodies.
  * Values are stored in the machine's byte order (little-endian on x86-64 and
  * aarch64); the header records the field count and per-body bytes. */
-static int select_variant(nbg_ctx *ctx, int v);
 
 #define NBG_SNAP_HEADER_BYTES 256
 #define NBG_SNAP_VERSION 1
@@ -1479,6 +1501,7 @@ int nbg_load_state(nbg_ctx *ctx, const void *buf, int64_t size)
     ctx->precision = H.precision;
     if ((rc = nbg_set_option(ctx, NBG_OPT_BARNES_HUT, H.barnes_hut)) != NBG_OK) return rc;
     if (H.mix_variant != ctx->cb.mix_variant && (rc = select_variant(ctx, H.mix_variant)) != NBG_OK) return rc;
+    ctx->shape_given = 2;
     ctx->pending_adds = 0;
     ctx->add_sim.clear();
     if ((rc = ensure_cap(ctx, H.n + H.pending_adds + 1, 0)) != NBG_OK) return rc;
@@ -1728,7 +1751,7 @@ int nbg_step(nbg_ctx *ctx, double dt, double R, int nsteps, nbg_step_info *info)
         else if (h->error_what == 5)
             rc = ensure_bh(ctx, h->error_need);
         else if (h->error_what == 6)
-            rc = ensure_jpart(ctx, h->error_need);
+            rc = grow_jpart(ctx, h->error_need);
         else
             rc = ensure_frag_cap(ctx, h->error_need);
         if (rc != NBG_OK) return rc;
@@ -1815,7 +1838,7 @@ int nbg_force_pass(nbg_ctx *ctx)
             /* a buffer of the force pass was short: grow it, run again */
             rc = h->error_what == 4 ? ensure_part(ctx, h->error_need)
                  : h->error_what == 5 ? ensure_bh(ctx, h->error_need)
-                                      : ensure_jpart(ctx, h->error_need);
+                                      : grow_jpart(ctx, h->error_need);
             if (rc != NBG_OK) return rc;
             continue;
         }
@@ -1934,6 +1957,7 @@ int nbg_autotune(nbg_ctx *ctx, const char *cache_path, int *variant, double *bes
         }
     }
     if ((rc = select_variant(ctx, best)) != NBG_OK) return rc;
+    ctx->shape_given = 1;
     if (!nbg_mix_is_sym(best) && ctx->cb.jpart) {
         /* a one-sided shape won: the symmetric kernel's slots go */
         CK(cudaStreamSynchronize(ctx->st));
@@ -2086,6 +2110,7 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value)
         return NBG_OK;
     case NBG_OPT_MIX_SHAPE:
         if (value < 0 || value >= NBG_MIX_VARIANTS) return fail(ctx, NBG_E_ARG, "unknown kernel shape");
+        ctx->shape_given = 1;
         return select_variant(ctx, (int)value);
     case NBG_OPT_BH_SHAPE:
         if (value < 0 || value > 2) return fail(ctx, NBG_E_ARG, "Barnes-Hut walk shape must be 0..2");

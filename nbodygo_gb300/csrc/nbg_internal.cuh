@@ -416,6 +416,38 @@ __host__ __device__ __forceinline__ unsigned nbg_hilbert(unsigned x, unsigned y,
 #define NBG_MIX_BLOCK 128
 #define NBG_MIX_K 4
 #define NBG_MIX_ITILE (NBG_MIX_BLOCK * NBG_MIX_K)
+
+/* The shape of a context that was not given one: one-sided, 256 bodies a tile,
+ * with j tiles of 256 bodies (shape 2) or, for few bodies, of 128 (shape 6:
+ * shorter careful passes; the longer tiles are 5% faster once they fill the
+ * chip).  Shapes 0 / 2 / 6, pair pass in us: Plummer 2,000 bodies 110 / 97 /
+ * 97, 20,000 424 / 227 / 202, 50,000 1,053 / 1,009 / 1,012, 131,072 6,652 /
+ * 6,351 / 6,675.  Or the symmetric kernel when every collection has NBG_MIX_SYM_MIN_N bodies.  Fewer make too few block pairs to share
+ * evenly, and the block pairs around a large body take longest: one-sided
+ * against symmetric pair pass, in ms, for a uniform ball / a disk around a
+ * star, 1.65 / 1.84 and 1.54 / 2.29 at 65,536 bodies, 3.61 / 3.70 and 2.94 /
+ * 4.09 at 98,304, 6.35 / 6.36 and 5.10 / 6.34 at 131,072, 32.8 / 30.3 and
+ * 25.9 / 28.2 at 300,000.  The symmetric kernel's j partials grow with
+ * the square of the body count (units: block pairs, 6 KB each); more than an
+ * eighth of the device's memory is not taken unasked. */
+#define NBG_MIX_ONE_SIDED 2
+#define NBG_MIX_ONE_SIDED_FEW 6
+#define NBG_MIX_FEW_N 32768
+#define NBG_MIX_SYM_MIN_N 114688
+static inline int nbg_default_shape(int nsims, const ll *counts, unsigned long long device_bytes)
+{
+    unsigned long long units = 0;
+    ll n = 0;
+    for (int s = 0; s < nsims; s++) n += counts[s];
+    if (n < NBG_MIX_FEW_N) return NBG_MIX_ONE_SIDED_FEW;
+    for (int s = 0; s < nsims; s++) {
+        if (counts[s] < NBG_MIX_SYM_MIN_N) return NBG_MIX_ONE_SIDED;
+        const unsigned long long T = ((unsigned long long)counts[s] + NBG_MIX_ITILE - 1) / NBG_MIX_ITILE;
+        units += T * (T + 1) / 2;
+    }
+    const unsigned long long unit_bytes = 3ull * NBG_MIX_ITILE * sizeof(float);
+    return (units + units / 4) > device_bytes / 8 / unit_bytes ? NBG_MIX_ONE_SIDED : NBG_MIX_SYM;
+}
 #define NBG_MIX_JT 256
 
 /* The reference's event rules (body.go:174-184): the event type for bodies

@@ -1,0 +1,42 @@
+// The mixed kernel's shape by default (nbg_internal.cuh): symmetric where every
+// collection is large and the j partials take at most an eighth of the memory.
+#include <cstdio>
+
+#include "nbg_internal.cuh"
+
+int main()
+{
+    int bad = 0;
+    const unsigned long long gb = 1ull << 30, big = 280 * gb;
+    const ll m = NBG_MIX_SYM_MIN_N;
+    auto want = [&](int nsims, const ll *c, unsigned long long bytes, int v) {
+        if (nbg_default_shape(nsims, c, bytes) != v) {
+            printf("%d collections, the first of %lld bodies: %d, not %d\n", nsims, (long long)c[0],
+                   nbg_default_shape(nsims, c, bytes), v);
+            bad++;
+        }
+    };
+    const ll none[] = {0}, one[] = {1}, below[] = {m - 1}, at[] = {m}, m1[] = {1 << 20}, huge[] = {1ll << 30};
+    const ll few[] = {NBG_MIX_FEW_N - 1}, more[] = {NBG_MIX_FEW_N / 2, NBG_MIX_FEW_N / 2};
+    want(1, none, big, NBG_MIX_ONE_SIDED_FEW);
+    want(1, one, big, NBG_MIX_ONE_SIDED_FEW);
+    want(1, few, big, NBG_MIX_ONE_SIDED_FEW);
+    want(1, more, big, NBG_MIX_ONE_SIDED_FEW);
+    want(2, more, big, NBG_MIX_ONE_SIDED);
+    want(1, below, big, NBG_MIX_ONE_SIDED);
+    want(1, at, big, NBG_MIX_SYM);
+    want(1, m1, big, NBG_MIX_SYM);
+    want(1, m1, 64 * gb, NBG_MIX_ONE_SIDED); // 16 GB of j partials
+    want(1, huge, big, NBG_MIX_ONE_SIDED);
+    want(1, at, 0, NBG_MIX_ONE_SIDED); // size unknown
+    const ll two[] = {m, 2 * m}, mixed[] = {2 * m, 0, 3 * m};
+    want(2, two, big, NBG_MIX_SYM);
+    want(3, mixed, big, NBG_MIX_ONE_SIDED);
+    // every unit counts: collections that fit alone, together past the eighth
+    static ll many[64];
+    for (ll &c : many) c = 1 << 18;
+    want(1, many, big, NBG_MIX_SYM);
+    want(64, many, big, NBG_MIX_ONE_SIDED);
+    printf("default shape bad %d\n", bad);
+    return bad != 0;
+}
