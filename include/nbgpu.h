@@ -372,7 +372,7 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
 /* shape of the mixed pair kernel, 0..NBG_MIX_SHAPES-1 (see nbg_autotune).  A
  * context that was neither given one nor tuned nor restored from a snapshot takes a
  * one-sided shape (6 for fewer than 32,768 bodies in all, 2 for more), or 15
- * (symmetric) when every loaded collection has 114,688 bodies or more and the j
+ * (symmetric) when every loaded collection has 98,304 bodies or more and the j
  * partials fit in an eighth of the device's memory. */
 #define NBG_OPT_MIX_SHAPE 7
 #define NBG_MIX_SHAPES 19
@@ -439,7 +439,7 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value);
  * two of the symmetric kernel, which computes each unordered pair once
  * and adds its term to both bodies (512-body blocks, 4 i-bodies per thread,
  * j pairs rotated through each warp's lanes):
- *  15: 128x4, 4 CTAs/SM              16: 128x4, 5 CTAs/SM
+ *  15: 128x4, 3 CTAs/SM              16: 128x4, 4 CTAs/SM
  * and two more one-sided shapes of kind B, sums in shared memory with the
  * raw j tiles brought into shared memory by bulk copies (cp.async.bulk on an
  * mbarrier) issued two tiles ahead and re-centred from there:

@@ -1002,8 +1002,9 @@ __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A
  * scheduling.  What a unit costs is the rotation, 183,000 cycles far and
  * 200,000 masked, plus the near pairs: with each lane evaluating its own,
  * one after the other, the largest unit of a 131,072-body Plummer + disk took 5
- * million cycles, half of the pass (6.81 ms; now 5.80; the disk 9.69 -> 6.31,
- * the uniform ball 5.45 -> 5.09).
+ * million cycles, half of the pass (6.81 ms; now 5.60; the disk 9.69 -> 5.68,
+ * the uniform ball 5.45 -> 4.91, 131,072 bodies each, with the register
+ * budget below).
  *
  * Sums.  i-sums fold into (hi, lo) pairs every 256 j and go to the one-sided
  * kernel's per-(row, chunk) FP64 slots; j-sums of a unit (128 terms per
@@ -1532,10 +1533,15 @@ __global__ void k_sym_out(BodyArrays A, DevCtl *ctl, SimSegs seg, const unsigned
 /* the kernel of a shape */
 #define MIX_KERNEL(kind, b, k, jt, u, mb) k_pair_mixed<b, k, jt, u, mb, (kind) >= 1, (kind) == 2, (kind) == 3>
 
-/* the symmetric kernel's shapes: registers capped for 4 or 5 CTAs per SM
- * (shared memory holds 4) */
-#define SYM_MINB_A 4
-#define SYM_MINB_B 5
+/* the symmetric kernel's shapes: registers capped for 3 or 4 CTAs per SM.  The
+ * rotation is bound by issue: a packed instruction takes two slots, and 3.5
+ * shuffles, 2 reciprocal square roots and the loop come to its 16 packed ones,
+ * so 167 registers, which leave the scheduler more to choose from, serve it
+ * better than a fourth CTA: 25.9 -> 24.9 ms at 300,000 bodies.  (8
+ * i-bodies a thread halve the shuffles, but leave 8 warps on an SM: 24.8 ms,
+ * and 28.0 where there are near pairs, against 26.3.) */
+#define SYM_MINB_A 3
+#define SYM_MINB_B 4
 
 MixVariantInfo nbg_mix_variant_info(int variant)
 {

@@ -425,15 +425,15 @@ __host__ __device__ __forceinline__ unsigned nbg_hilbert(unsigned x, unsigned y,
  * 6,351 / 6,675.  Or the symmetric kernel when every collection has NBG_MIX_SYM_MIN_N bodies.  Fewer make too few block pairs to share
  * evenly, and the block pairs around a large body take longest: one-sided
  * against symmetric pair pass, in ms, for a uniform ball / a disk around a
- * star, 1.65 / 1.84 and 1.54 / 2.29 at 65,536 bodies, 3.61 / 3.70 and 2.94 /
- * 4.09 at 98,304, 6.35 / 6.36 and 5.10 / 6.34 at 131,072, 32.8 / 30.3 and
- * 25.9 / 28.2 at 300,000.  The symmetric kernel's j partials grow with
+ * star, 1.65 / 1.84 and 1.54 / 2.29 at 65,536 bodies, 3.61 / 3.74 and 2.84 /
+ * 3.85 at 98,304, 6.34 / 6.45 and 4.91 / 5.68 at 131,072, 99.9 / 86.4 and
+ * 75.4 / 66.1 at 524,288.  The symmetric kernel's j partials grow with
  * the square of the body count (units: block pairs, 6 KB each); more than an
  * eighth of the device's memory is not taken unasked. */
 #define NBG_MIX_ONE_SIDED 2
 #define NBG_MIX_ONE_SIDED_FEW 6
 #define NBG_MIX_FEW_N 32768
-#define NBG_MIX_SYM_MIN_N 114688
+#define NBG_MIX_SYM_MIN_N 98304
 static inline int nbg_default_shape(int nsims, const ll *counts, unsigned long long device_bytes)
 {
     unsigned long long units = 0;

@@ -14,7 +14,7 @@ from nbodygo_gb300 import workloads as W
 from nbodygo_gb300.api import Simulation
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-MIN_N = 114688
+MIN_N = 98304
 
 
 def test_rule(tmp_path):
