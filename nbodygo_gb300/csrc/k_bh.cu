@@ -22,7 +22,7 @@
  *      node the next node and the end of its subtree the first node starting
  *      at the end of its body range (the skip pointer), so the force pass
  *      walks the tree without a stack;
- *   4. masses and centres of mass are summed bottom-up, level by level, over
+ *   4. masses and moments are summed from the leaves up, in one launch, over
  *      the children in octant order.
  *
  * The force pass (accumForce, octree.go:265-305) walks the tree for every
@@ -573,7 +573,6 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_nodes(DevCtl *ctl, SimSegs seg,
             t.start[id] = (int)p;
             t.end[id] = (int)end;
             t.skip[id] = (int)(end >= M ? total : base[end]);
-            t.level[id] = (unsigned char)d;
             t.flags[id] = (end - p == 1 || d == BH_LEVELS) ? BH_F_LEAF : 0u;
             t.cx[id] = cx;
             t.cy[id] = cy;
@@ -592,20 +591,33 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_nodes(DevCtl *ctl, SimSegs seg,
     }
 }
 
-/* ---- 4. mass and centre of mass, one level per launch, deepest first ------ */
+/* ---- 4. masses, from the leaves up ------------------------------------------ */
 
-__global__ void __launch_bounds__(BH_BLOCK) k_bh_mass(BodyArrays A, DevCtl *ctl, const unsigned *vals, BhTree t,
-                                                      int level)
+/* Each node's mass, moments and first body (in array order).  A leaf is one
+ * lane's; of a node's children the lane that finishes last (they count
+ * themselves in the node's first, which holds no body yet) takes the node, so
+ * nothing waits and no sum depends on who is last.  The nodes that a warp has
+ * taken are summed eight at a time, a lane for the mass and each moment, over
+ * the children in their order: an FP64 add costs the same for one lane as for
+ * 32, and one lane a node would spend four times as many.  (The centres of mass
+ * are divided out with every lane busy, in the preparation of the walks.)  One
+ * launch where each of 22 levels' launches read every node's level: 194 -> 47 us
+ * for 131,072 Plummer bodies, 785 -> 210 us for 1,048,576 uniform ones. */
+__global__ void __launch_bounds__(BH_BLOCK) k_bh_mass(BodyArrays A, DevCtl *ctl, const unsigned *vals, BhTree t)
 {
     if (ctl->error) return;
     const ll total = ctl->bh_nodes;
-    for (ll id = (ll)blockIdx.x * blockDim.x + threadIdx.x; id < total; id += (ll)gridDim.x * blockDim.x) {
-        if (t.level[id] != level) continue;
-        double M = 0, mx = 0, my = 0, mz = 0;
-        int first = 0x7fffffff;
-        if (t.flags[id] & BH_F_LEAF) {
-            for (int q = t.start[id]; q < t.end[id]; q++) {
-                const unsigned k = vals[q];
+    const int lane = threadIdx.x & 31, q = lane & 3;
+    double *const sum = q == 0 ? t.mass : q == 1 ? t.mx : q == 2 ? t.my : t.mz;
+    for (ll base = (ll)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
+         base += (ll)gridDim.x * blockDim.x) {
+        int node = (int)base + lane;
+        bool done = base + lane < total && (t.flags[base + lane] & BH_F_LEAF);
+        if (done) {
+            double M = 0, mx = 0, my = 0, mz = 0;
+            int first = 0x7fffffff;
+            for (int e = t.start[node]; e < t.end[node]; e++) {
+                const unsigned k = vals[e];
                 const double m = A.m[k];
                 M = M + m;
                 mx = mx + A.x[k] * m;
@@ -613,30 +625,68 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_mass(BodyArrays A, DevCtl *ctl,
                 mz = mz + A.z[k] * m;
                 if ((int)k < first) first = (int)k;
             }
-        } else {
-            const int stop = t.skip[id];
-            for (int c = (int)id + 1; c < stop; c = t.skip[c]) {
-                M = M + t.mass[c];
-                mx = mx + t.mx[c];
-                my = my + t.my[c];
-                mz = mz + t.mz[c];
-                if (t.first[c] < first) first = t.first[c];
+            t.mass[node] = M;
+            t.mx[node] = mx;
+            t.my[node] = my;
+            t.mz[node] = mz;
+            t.first[node] = first;
+        }
+        for (;;) {
+            __threadfence(); /* this node's sums before its count */
+            __syncwarp();
+            int p = done ? t.parent[node] : -1;
+            if (p >= 0 && atomicAdd(&t.first[p], 1) != (int)t.ccount[p] - 1) p = -1;
+            unsigned todo = __ballot_sync(FULL_MASK, p >= 0);
+            if (!todo) break;
+            __threadfence(); /* every child's sums after the last count */
+            __syncwarp();
+            while (todo) {
+                unsigned m = todo; /* the lane>>2-th of the nodes left */
+                for (int g = 0; g < (lane >> 2); g++) m &= m - 1u;
+                const int id = __shfl_sync(FULL_MASK, p, m ? __ffs(m) - 1 : 0);
+                if (m) {
+                    const int stop = t.skip[id];
+                    double v = 0;
+                    int first = 0x7fffffff;
+                    for (int c = id + 1; c < stop; c = t.skip[c]) {
+                        v = v + __ldcg(&sum[c]);
+                        const int f = __ldcg(&t.first[c]);
+                        if (f < first) first = f;
+                    }
+                    sum[id] = v;
+                    if (q == 0) t.first[id] = first;
+                }
+                for (int g = 0; g < 8; g++) todo &= todo - 1u;
             }
+            done = p >= 0;
+            node = p;
         }
-        t.mass[id] = M;
-        t.mx[id] = mx;
-        t.my[id] = my;
-        t.mz[id] = mz;
-        t.first[id] = first;
-        if (M != 0) {
-            t.cmx[id] = mx / M;
-            t.cmy[id] = my / M;
-            t.cmz[id] = mz / M;
-        }
-        /* the reference's running centre is 0 / 0 when the node's first body
-         * (in array order) is massless, and stays NaN */
-        if (A.m[first] == 0) t.flags[id] |= BH_F_NAN_CM;
     }
+}
+
+/* The centre of mass of node id, whose mass is M: its moments over its mass,
+ * correctly rounded, by integer arithmetic where the operands allow. */
+__device__ __forceinline__ void bh_centre(const BhTree &t, ll id, double M, double &cx, double &cy, double &cz)
+{
+    const double mx = t.mx[id], my = t.my[id], mz = t.mz[id];
+    const uint64_t bm = nbx_bits(M), bx = nbx_bits(mx), by = nbx_bits(my), bz = nbx_bits(mz);
+    if (nbx_root_ok(bm) && nbx_within(bx, 302) && nbx_within(by, 302) && nbx_within(bz, 302)) {
+        const nbx_div d = nbx_operand(nbx_sqrt(bm));
+        cx = nbx_double(nbx_pack(nbx_quot(nbx_unpack(bx), d)));
+        cy = nbx_double(nbx_pack(nbx_quot(nbx_unpack(by), d)));
+        cz = nbx_double(nbx_pack(nbx_quot(nbx_unpack(bz), d)));
+    } else {
+        cx = mx / M;
+        cy = my / M;
+        cz = mz / M;
+    }
+}
+
+/* A node's flags for the walks.  The reference's running centre is 0 / 0 when
+ * the node's first body (in array order) is massless, and stays NaN. */
+__device__ __forceinline__ unsigned bh_walk_flags(const BodyArrays &A, const BhTree &t, ll id)
+{
+    return t.flags[id] | (A.m[t.first[id]] == 0 ? BH_F_NAN_CM : 0u);
 }
 
 /* ---- 5. forces ------------------------------------------------------------- */
@@ -713,13 +763,20 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_children(DevCtl *ctl, SimSegs s
             const int first = (int)at + seg.nsims + x - nc;
             t.cbase[id] = first;
             t.ccount[id] = (unsigned char)nc;
+            t.first[id] = 0; /* k_bh_mass counts the children that are done here */
 #pragma unroll
             for (int q = 0; q < 8; q++)
-                if (q < nc) t.slot[child[q]] = first + q;
+                if (q < nc) {
+                    t.slot[child[q]] = first + q;
+                    t.parent[child[q]] = (int)id;
+                }
         }
     }
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < seg.nsims; s += gridDim.x * blockDim.x)
-        if (t.sroot[s] < t.sroot[s + 1]) t.slot[t.sroot[s]] = s;
+        if (t.sroot[s] < t.sroot[s + 1]) {
+            t.slot[t.sroot[s]] = s;
+            t.parent[t.sroot[s]] = -1;
+        }
 }
 
 /* Group g holds sorted positions [p0, p1) of collection s: the groups of a
@@ -736,7 +793,7 @@ __device__ __forceinline__ void bh_group(const BhTree &t, int nsims, int g, int 
  * floats with the squared opening distance (zero when out of FP32's range:
  * then the bodies decide in FP64), and centre, mass and half size as doubles */
 #define BH_F_EMPTY 4u /* no mass below */
-__global__ void __launch_bounds__(BH_BLOCK) k_bh_prep64(DevCtl *ctl, BhTree t)
+__global__ void __launch_bounds__(BH_BLOCK) k_bh_prep64(BodyArrays A, DevCtl *ctl, BhTree t)
 {
     if (ctl->error) return;
     const ll total = ctl->bh_nodes;
@@ -744,17 +801,13 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_prep64(DevCtl *ctl, BhTree t)
         const int slot = t.slot[id];
         const double M = t.mass[id], half = t.half[id];
         double cx = 0.0, cy = 0.0, cz = 0.0;
-        if (M != 0) {
-            cx = t.cmx[id];
-            cy = t.cmy[id];
-            cz = t.cmz[id];
-        }
+        if (M != 0) bh_centre(t, id, M, cx, cy, cz);
         const float hx = (float)cx, hy = (float)cy, hz = (float)cz;
         const double o = 2 * half / BH_THETA, o2 = o * o;
         t.fa[slot] = make_float4(hx, hy, hz, o2 > 1e-30 && o2 < 1e37 ? (float)o2 : 0.f);
         t.fb[slot] = make_float4((float)(cx - (double)hx), (float)(cy - (double)hy), (float)(cz - (double)hz), 0.f);
         t.fc[slot] = make_int4(t.cbase[id],
-                               (int)t.ccount[id] | ((int)(t.flags[id] | (M == 0 ? BH_F_EMPTY : 0u)) << 8),
+                               (int)t.ccount[id] | ((int)(bh_walk_flags(A, t, id) | (M == 0 ? BH_F_EMPTY : 0u)) << 8),
                                t.start[id], t.end[id]);
         t.rec[2 * (ll)slot] = make_double2(cx, cy);
         t.rec[2 * (ll)slot + 1] = make_double2(cz, M);
@@ -1106,19 +1159,26 @@ __global__ void __launch_bounds__(BHW_BLOCK, 5) k_bh_force(const __grid_constant
  * groups of uneven cost: 263,000 instructions a group before the lists were
  * split into far and near ones, 60 % of them in the sums. */
 /* every node's record for the walk, in its slot */
-__global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(DevCtl *ctl, SimSegs seg, BhTree t)
+__global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(BodyArrays A, DevCtl *ctl, SimSegs seg, BhTree t)
 {
     if (ctl->error) return;
     const ll total = ctl->bh_nodes;
     if (total <= 0) return;
+    ll root = -1;
+    double inv_root = 0.0;
     for (ll id = (ll)blockIdx.x * blockDim.x + threadIdx.x; id < total; id += (ll)gridDim.x * blockDim.x) {
         /* masses relative to the root of the node's own tree */
-        const double mroot = t.mass[t.sroot[nbg_sim_of(t.sroot, seg.nsims, id)]];
-        const double inv_root = mroot != 0 ? 1.0 / mroot : 0.0;
+        const ll r = t.sroot[nbg_sim_of(t.sroot, seg.nsims, id)];
+        if (r != root) {
+            const double mroot = t.mass[r];
+            inv_root = mroot != 0 ? 1.0 / mroot : 0.0;
+            root = r;
+        }
         const double M = t.mass[id];
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
         if (M != 0) {
-            const double cx = t.cmx[id], cy = t.cmy[id], cz = t.cmz[id];
+            double cx, cy, cz;
+            bh_centre(t, id, M, cx, cy, cz);
             a.x = (float)cx;
             a.y = (float)cy;
             a.z = (float)cz;
@@ -1132,7 +1192,8 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(DevCtl *ctl, SimSegs
         const int slot = t.slot[id];
         t.fa[slot] = a;
         t.fb[slot] = b;
-        t.fc[slot] = make_int4(t.cbase[id], (int)t.ccount[id] | ((int)t.flags[id] << 8), t.start[id], t.end[id]);
+        t.fc[slot] = make_int4(t.cbase[id], (int)t.ccount[id] | ((int)bh_walk_flags(A, t, id) << 8), t.start[id],
+                               t.end[id]);
     }
 }
 
@@ -1739,9 +1800,6 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
     ALLOC(t.mx, node_cap);
     ALLOC(t.my, node_cap);
     ALLOC(t.mz, node_cap);
-    ALLOC(t.cmx, node_cap);
-    ALLOC(t.cmy, node_cap);
-    ALLOC(t.cmz, node_cap);
     ALLOC(t.cx, node_cap);
     ALLOC(t.cy, node_cap);
     ALLOC(t.cz, node_cap);
@@ -1750,7 +1808,7 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
     ALLOC(t.start, node_cap);
     ALLOC(t.end, node_cap);
     ALLOC(t.first, node_cap);
-    ALLOC(t.level, node_cap);
+    ALLOC(t.parent, node_cap);
     ALLOC(t.flags, node_cap);
     ALLOC(t.fa, node_cap + NBG_MAX_SIMS); /* a slot per collection's root, used or not */
     ALLOC(t.fb, node_cap + NBG_MAX_SIMS);
@@ -1779,8 +1837,8 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
 void nbg_bh_free(BhTree &t)
 {
     void *ps[] = {t.key[0], t.key[1], t.val[0], t.val[1], t.hist, t.base, t.blk, t.mass, t.mx, t.my,
-                  t.mz, t.cmx, t.cmy, t.cmz, t.cx, t.cy, t.cz, t.half, t.skip, t.start,
-                  t.end, t.first, t.level, t.flags, t.fa, t.fb, t.rec, t.shalf, t.fc, t.fd, t.cbase, t.ccount, t.slot,
+                  t.mz, t.cx, t.cy, t.cz, t.half, t.skip, t.start,
+                  t.end, t.first, t.parent, t.flags, t.fa, t.fb, t.rec, t.shalf, t.fc, t.fd, t.cbase, t.ccount, t.slot,
                   t.sbox, t.scount, t.stree, t.sroot, t.sgrp, t.sunit};
     for (void *p : ps) cudaFree(p);
     memset(&t, 0, sizeof t);
@@ -1823,11 +1881,10 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
     k_bh_nodes<<<g, BH_BLOCK, 0, st>>>(ctl, seg, t.key[0], t.base, t);
     int ng = (int)((t.node_cap + BH_BLOCK - 1) / BH_BLOCK < gmost ? (t.node_cap + BH_BLOCK - 1) / BH_BLOCK : gmost);
     if (ng < 1) ng = 1;
-    for (int level = BH_LEVELS; level >= 0; level--)
-        k_bh_mass<<<ng, BH_BLOCK, 0, st>>>(cb.a, ctl, t.val[0], t, level);
     k_bh_children<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
+    k_bh_mass<<<ng, BH_BLOCK, 0, st>>>(cb.a, ctl, t.val[0], t);
     if (mixed) {
-        k_bh_prep_mixed<<<ng, BH_BLOCK, 0, st>>>(ctl, seg, t);
+        k_bh_prep_mixed<<<ng, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t);
         /* one wave of resident CTAs, which share the queue of units; 4 CTAs
          * per SM (121 registers, no spill) measured fastest, 2.38 ms for the
          * tree pass of 131,072 Plummer bodies against 2.52 with 5 or 6 */
@@ -1840,7 +1897,7 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
         default: k_bh_force_mixed<4><<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t); break;
         }
     } else {
-        k_bh_prep64<<<ng, BH_BLOCK, 0, st>>>(ctl, t);
+        k_bh_prep64<<<ng, BH_BLOCK, 0, st>>>(cb.a, ctl, t);
         const ll wgroups = cap / 32 + 1 + seg.nsims;
         const int gw = (int)(wgroups < (ll)cb.sms * 5 ? wgroups : (ll)cb.sms * 5);
         k_bh_force<<<gw, BHW_BLOCK, 0, st>>>(cb.a, ctl, seg, t.val[0], t);
@@ -1853,6 +1910,6 @@ int nbg_bh_launches(const CycleBufs &cb, bool mixed)
 {
     const int passes = cb.seg.nsims > 1 ? 10 : 8;
     /* reset, bounds, segs, keys; the sort; count, top, scan, roots, nodes;
-     * masses; (prep,) walk; suns; collisions */
-    return 4 + 3 * passes + 5 + (BH_LEVELS + 1) + 3 + 2;
+     * children, masses; prep, walk; suns, collisions */
+    return 4 + 3 * passes + 5 + 2 + 2 + 2;
 }

@@ -202,7 +202,7 @@ struct BhTree {
     ll *hist;           /* radix digit histogram */
     ll *base;           /* nodes starting at each sorted position, then their scan */
     ll *blk;            /* per-block sums of that scan */
-    double *mass, *mx, *my, *mz, *cmx, *cmy, *cmz, *cx, *cy, *cz, *half;
+    double *mass, *mx, *my, *mz, *cx, *cy, *cz, *half;
     float4 *fa, *fb;    /* mixed walk, by slot: (cm hi xyz, mass / root mass), (cm lo xyz, opening r^2);
                          * FP64 walk: (cm hi xyz, opening r^2), (cm lo xyz, 0) */
     double2 *rec;       /* FP64 walk, by slot: (cm x, y), (cm z, mass) */
@@ -213,7 +213,8 @@ struct BhTree {
     int *cbase;            /* slot of the first of the node's children */
     unsigned char *ccount; /* and how many there are */
     int *slot;             /* the node's own slot */
-    unsigned char *level, *flags;
+    int *parent;           /* the node's parent, -1 for a root */
+    unsigned char *flags;
     /* one tree per collection, all in one depth-first node array: per
      * collection s its bounding box (sbox[6 s ..]: lo xyz, hi xyz as
      * order-preserving integers), tree bodies (scount), first sorted
