@@ -60,16 +60,19 @@
 #include "nbg_exact.h"
 #include "nbg_internal.cuh"
 #include "nbg_math.h"
+#include "nbg_octant.h"
 #include "nbg_shared.h"
 
 #define BH_THETA 0.3
 #define BH_SOFTENING 1e-4
-#define BH_LEVELS 21
+#define BH_LEVELS NBG_OCT_LEVELS
 #define BH_BLOCK 256
 #define BH_RS_BLOCK 256
-#define BH_RS_ITEMS 16
+#define BH_RS_ITEMS 4
 #define BH_RS_TILE (BH_RS_BLOCK * BH_RS_ITEMS)
 #define BH_RS_BINS 256
+#define BH_RS_NARROW 192 /* most blocks whose scatter sums the histogram itself */
+#define BH_RS_PASSES 10
 #define BH_SCAN_BLOCK 1024
 #define BH_SCAN_ITEMS 4
 #define BH_SCAN_TILE (BH_SCAN_BLOCK * BH_SCAN_ITEMS)
@@ -121,10 +124,11 @@ __device__ __forceinline__ void bh_root(const BhTree &t, int s, double &cx, doub
 
 /* ---- 1. bounds, keys -------------------------------------------------------- */
 
-/* empty boxes and counts for every collection */
+/* empty boxes and counts for every collection, and no digits counted */
 __global__ void __launch_bounds__(1024) k_bh_reset(DevCtl *ctl, SimSegs seg, BhTree t)
 {
     if (ctl->error) return;
+    for (int d = threadIdx.x; d < BH_RS_PASSES * BH_RS_BINS; d += blockDim.x) t.digits[d] = 0;
     for (int s = threadIdx.x; s < seg.nsims; s += blockDim.x) {
         ull *b = t.sbox + 6 * (ll)s;
         for (int c = 0; c < 3; c++) {
@@ -143,11 +147,47 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_bounds(BodyArrays A, DevCtl *ct
     const ll n = ctl->n;
     const int lane = threadIdx.x & 31;
     double rmax = 0;
+    ull lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
+    unsigned cnt = 0;
+    if (seg.nsims == 1) {
+        /* one collection: a lane keeps its own box, and the warp reduces once
+         * (reducing every 32 bodies, as below, took 83 us for 1,048,576 against
+         * 34) */
+        for (ll k = (ll)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (ll)gridDim.x * blockDim.x) {
+            const double r = A.rad[k];
+            if (r > rmax) rmax = r;
+            if (!tree_body(A, k)) continue;
+            const ull p[3] = {dbl_ord(A.x[k]), dbl_ord(A.y[k]), dbl_ord(A.z[k])};
+            for (int c = 0; c < 3; c++) {
+                lo[c] = p[c] < lo[c] ? p[c] : lo[c];
+                hi[c] = p[c] > hi[c] ? p[c] : hi[c];
+            }
+            cnt++;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            for (int c = 0; c < 3; c++) {
+                const ull l = __shfl_xor_sync(FULL_MASK, lo[c], o), h = __shfl_xor_sync(FULL_MASK, hi[c], o);
+                lo[c] = l < lo[c] ? l : lo[c];
+                hi[c] = h > hi[c] ? h : hi[c];
+            }
+            cnt += __shfl_xor_sync(FULL_MASK, cnt, o);
+        }
+        if (lane == 0 && cnt > 0) {
+            for (int c = 0; c < 3; c++) {
+                atomicMin((unsigned long long *)&t.sbox[c], (unsigned long long)lo[c]);
+                atomicMax((unsigned long long *)&t.sbox[3 + c], (unsigned long long)hi[c]);
+            }
+            atomicAdd((unsigned long long *)&t.scount[0], (unsigned long long)cnt);
+        }
+    } else
     /* warp-uniform trip count: every lane takes part in the reductions */
     for (ll base = (ll)blockIdx.x * blockDim.x; base < n; base += (ll)gridDim.x * blockDim.x) {
         const ll k = base + threadIdx.x;
-        ull lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
-        unsigned cnt = 0;
+        for (int c = 0; c < 3; c++) {
+            lo[c] = ~0ull;
+            hi[c] = 0ull;
+        }
+        cnt = 0;
         int sim = -1;
         if (k < n) {
             const double r = A.rad[k];
@@ -242,29 +282,42 @@ __global__ void __launch_bounds__(32) k_bh_segs(DevCtl *ctl, SimSegs seg, BhTree
 /* the collection whose run of sorted tree positions holds p (0 <= p < M) */
 __device__ __forceinline__ int bh_run_of(const BhTree &t, int nsims, ll p) { return nbg_sim_of(t.stree, nsims, p); }
 
-/* octant path of every tree body in its collection's cube; other bodies
- * get the largest key */
+/* a collection's root cube as a grid */
+__device__ __forceinline__ NbgOctGrid bh_grid(const BhTree &t, int s)
+{
+    double cx, cy, cz, half;
+    bh_root(t, s, cx, cy, cz, half);
+    return nbg_oct_grid(cx, cy, cz, half);
+}
+
+/* the path of the rare body near a cell's face */
+__device__ __noinline__ ull bh_path(double x, double y, double z, double cx, double cy, double cz, double half)
+{
+    return nbg_oct_path(x, y, z, cx, cy, cz, half);
+}
+
+/* Octant path of every tree body in its collection's cube; other bodies get the
+ * largest key.  The 21 levels' comparisons and centres are 170 FP64 operations a
+ * body, and the FP64 pipe bounds the pass; the cell of a 2^21 grid has the same bits unless the
+ * coordinate is within rounding of a cell's face, which takes 9 (and the path
+ * where it is): 49 -> 18 us at 131,072 bodies, 252 -> 38 us at 1,048,576. */
 __global__ void __launch_bounds__(BH_BLOCK) k_bh_keys(BodyArrays A, DevCtl *ctl, SimSegs seg, BhTree t, ull *keys,
                                                       unsigned *vals)
 {
     if (ctl->error) return;
     const ll n = ctl->n;
+    int sim = -1;
+    NbgOctGrid g;
     for (ll k = (ll)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (ll)gridDim.x * blockDim.x) {
         ull key = ~0ull;
         if (tree_body(A, k)) {
             const double x = A.x[k], y = A.y[k], z = A.z[k];
-            double cx, cy, cz, half;
-            bh_root(t, nbg_sim_of(seg.off, seg.nsims, k), cx, cy, cz, half);
-            key = 0;
-            for (int d = 0; d < BH_LEVELS; d++) {
-                const unsigned oct = (x >= cx ? 1u : 0u) | (y >= cy ? 2u : 0u) | (z >= cz ? 4u : 0u);
-                key = (key << 3) | oct;
-                const double q = half / 2;
-                cx = (oct & 1u) ? cx + q : cx - q;
-                cy = (oct & 2u) ? cy + q : cy - q;
-                cz = (oct & 4u) ? cz + q : cz - q;
-                half = half / 2;
+            const int s = nbg_sim_of(seg.off, seg.nsims, k);
+            if (s != sim) {
+                g = bh_grid(t, s);
+                sim = s;
             }
+            if (!nbg_oct_cell(g, x, y, z, key)) key = bh_path(x, y, z, g.cx, g.cy, g.cz, g.half);
         }
         keys[k] = key;
         vals[k] = (unsigned)k;
@@ -283,8 +336,17 @@ __device__ __forceinline__ unsigned bh_digit(const SimSegs &seg, ull key, unsign
     return (d >> (8 * simpass)) & 0xffu;
 }
 
+/* A pass is a histogram of each block's BH_RS_TILE keys (with the digits'
+ * totals, which all blocks add to), and a scatter.  Up to BH_RS_NARROW
+ * blocks, the histogram lies block by block and each block of the scatter adds
+ * up the rows of those before it; past that, the sum would grow with the square
+ * of the blocks, and a scan between the two turns the histogram, digit by
+ * digit, into offsets.  Small tiles, so 131,072 keys make 128 blocks, and no
+ * barrier between a block's keys: a pass over 131,072 takes 12.6 us with the scan
+ * (30.9 with tiles of 4,096 and a scan by one block), over 1,048,576 28.6 (63.8). */
 __global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_hist(DevCtl *ctl, SimSegs seg, const ull *keys,
-                                                          const unsigned *vals, int shift, int simpass, ll *hist)
+                                                          const unsigned *vals, int shift, int simpass, int wide,
+                                                          unsigned *hist, unsigned *digits)
 {
     __shared__ unsigned cnt[BH_RS_BINS];
     if (ctl->error) return;
@@ -292,100 +354,122 @@ __global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_hist(DevCtl *ctl, SimSegs
     const ll nb = (n + BH_RS_TILE - 1) / BH_RS_TILE;
     const ll b = blockIdx.x;
     if (b >= nb) return;
-    for (int d = threadIdx.x; d < BH_RS_BINS; d += BH_RS_BLOCK) cnt[d] = 0;
+    const int tid = threadIdx.x;
+    cnt[tid] = 0;
     __syncthreads();
+#pragma unroll
     for (int q = 0; q < BH_RS_ITEMS; q++) {
-        const ll k = b * BH_RS_TILE + (ll)q * BH_RS_BLOCK + threadIdx.x;
-        if (k < n) atomicAdd(&cnt[bh_digit(seg, keys[k], vals[k], shift, simpass)], 1u);
+        const ll k = b * BH_RS_TILE + (ll)q * BH_RS_BLOCK + tid;
+        if (k < n) atomicAdd(&cnt[bh_digit(seg, keys[k], simpass < 0 ? 0u : vals[k], shift, simpass)], 1u);
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < BH_RS_BINS; d += BH_RS_BLOCK) hist[(ll)d * nb + b] = cnt[d];
+    const unsigned c = cnt[tid];
+    hist[wide ? (ll)tid * nb + b : b * BH_RS_BINS + tid] = c;
+    if (c) atomicAdd(&digits[tid], c);
+}
+static_assert(BH_RS_BLOCK == BH_RS_BINS, "a thread per digit");
+
+/* thread d: the elements of the digits below d */
+__device__ __forceinline__ unsigned bh_digit_start(const unsigned *digits, unsigned *wtot)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned v = digits[threadIdx.x];
+    unsigned x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(FULL_MASK, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wtot[w] = x;
+    __syncthreads();
+    for (int u = 0; u < w; u++) x += wtot[u];
+    return x - v;
 }
 
-/* exclusive scan of the digit-major histogram (one block, four entries per
- * thread per round) */
-__global__ void __launch_bounds__(1024) k_bh_rs_scan(DevCtl *ctl, ll *hist)
+/* a warp to a digit's row of the histogram */
+__global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_scan(DevCtl *ctl, unsigned *hist, const unsigned *digits)
 {
-    __shared__ ll warp_tot[32];
+    __shared__ unsigned wtot[BH_RS_BLOCK / 32], start[BH_RS_BINS];
     if (ctl->error) return;
-    const ll n = ctl->n;
-    const ll total = ((n + BH_RS_TILE - 1) / BH_RS_TILE) * BH_RS_BINS;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    ll carry = 0;
-    for (ll c0 = 0; c0 < total; c0 += 4096) {
-        const ll c = c0 + (ll)threadIdx.x * 4;
-        ll v[4], sum = 0;
-        for (int q = 0; q < 4; q++) {
-            v[q] = c + q < total ? hist[c + q] : 0;
-            sum += v[q];
-        }
-        ll x = sum;
+    const ll nb = (ctl->n + BH_RS_TILE - 1) / BH_RS_TILE;
+    const int lane = threadIdx.x & 31, d = blockIdx.x * (BH_RS_BLOCK / 32) + (threadIdx.x >> 5);
+    start[threadIdx.x] = bh_digit_start(digits, wtot);
+    __syncthreads();
+    unsigned carry = start[d];
+    unsigned *row = hist + (ll)d * nb;
+    for (ll c = 0; c < nb; c += 32) {
+        const unsigned v = c + lane < nb ? row[c + lane] : 0u;
+        unsigned x = v;
         for (int o = 1; o < 32; o <<= 1) {
-            const ll y = __shfl_up_sync(FULL_MASK, x, o);
+            const unsigned y = __shfl_up_sync(FULL_MASK, x, o);
             if (lane >= o) x += y;
         }
-        if (lane == 31) warp_tot[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            ll t = warp_tot[lane];
-            for (int o = 1; o < 32; o <<= 1) {
-                const ll y = __shfl_up_sync(FULL_MASK, t, o);
-                if (lane >= o) t += y;
-            }
-            warp_tot[lane] = t;
-        }
-        __syncthreads();
-        ll ex = carry + x - sum + (w > 0 ? warp_tot[w - 1] : 0);
-        for (int q = 0; q < 4; q++) {
-            if (c + q < total) hist[c + q] = ex;
-            ex += v[q];
-        }
-        carry += warp_tot[31];
-        __syncthreads();
+        if (c + lane < nb) row[c + lane] = carry + x - v;
+        carry += __shfl_sync(FULL_MASK, x, 31);
     }
 }
 
 __global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_scatter(DevCtl *ctl, SimSegs seg, const ull *keys_in,
                                                              const unsigned *vals_in, ull *keys_out,
-                                                             unsigned *vals_out, int shift, int simpass,
-                                                             const ll *offs)
+                                                             unsigned *vals_out, int shift, int simpass, int wide,
+                                                             const unsigned *hist, const unsigned *digits)
 {
-    __shared__ ll base[BH_RS_BINS];
-    __shared__ unsigned wcnt[BH_RS_BLOCK / 32][BH_RS_BINS];
+    __shared__ unsigned wtot[BH_RS_BLOCK / 32], cnt[BH_RS_BLOCK / 32][BH_RS_BINS];
     if (ctl->error) return;
     const ll n = ctl->n;
     const ll nb = (n + BH_RS_TILE - 1) / BH_RS_TILE;
     const ll b = blockIdx.x;
     if (b >= nb) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int d = threadIdx.x; d < BH_RS_BINS; d += BH_RS_BLOCK) base[d] = offs[(ll)d * nb + b];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
+    /* a warp's keys are consecutive: its first, then 32 at a time */
+    const ll k0 = b * BH_RS_TILE + (ll)w * (32 * BH_RS_ITEMS) + lane;
+    ull key[BH_RS_ITEMS];
+    unsigned val[BH_RS_ITEMS], rank[BH_RS_ITEMS], dig[BH_RS_ITEMS];
+#pragma unroll
     for (int q = 0; q < BH_RS_ITEMS; q++) {
-        for (int d = threadIdx.x; d < BH_RS_BINS * (BH_RS_BLOCK / 32); d += BH_RS_BLOCK) (&wcnt[0][0])[d] = 0;
-        __syncthreads();
-        const ll k = b * BH_RS_TILE + (ll)q * BH_RS_BLOCK + threadIdx.x;
-        const bool ok = k < n;
-        const ull key = ok ? keys_in[k] : 0ull;
-        const unsigned val = ok ? vals_in[k] : 0u;
-        const unsigned d = ok ? bh_digit(seg, key, val, shift, simpass) : BH_RS_BINS;
-        const unsigned peers = __match_any_sync(FULL_MASK, d);
-        const unsigned rank = __popc(peers & lt);
-        if (ok && rank == 0) wcnt[w][d] = __popc(peers);
-        __syncthreads();
-        if (ok) {
-            ll pos = base[d] + rank;
-            for (int v = 0; v < w; v++) pos += wcnt[v][d];
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-        }
-        __syncthreads();
-        for (int dd = threadIdx.x; dd < BH_RS_BINS; dd += BH_RS_BLOCK) {
-            ll s = 0;
-            for (int v = 0; v < BH_RS_BLOCK / 32; v++) s += wcnt[v][dd];
-            base[dd] += s;
-        }
-        __syncthreads();
+        const bool ok = k0 + 32 * q < n;
+        key[q] = ok ? keys_in[k0 + 32 * q] : 0ull;
+        val[q] = ok ? vals_in[k0 + 32 * q] : 0u;
     }
+    /* where the block's elements of digit tid start */
+    unsigned at;
+    if (wide) {
+        at = hist[(ll)tid * nb + b];
+    } else {
+        at = bh_digit_start(digits, wtot);
+        const unsigned *h = hist + tid;
+#pragma unroll 8
+        for (int u = 0; u < (int)b; u++) at += h[u * BH_RS_BINS];
+    }
+    for (int c = tid; c < BH_RS_BINS * (BH_RS_BLOCK / 32); c += BH_RS_BLOCK) (&cnt[0][0])[c] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < BH_RS_ITEMS; q++) {
+        const bool ok = k0 + 32 * q < n;
+        const unsigned d = ok ? bh_digit(seg, key[q], val[q], shift, simpass) : BH_RS_BINS;
+        const unsigned peers = __match_any_sync(FULL_MASK, d);
+        const unsigned before = __popc(peers & lt);
+        const unsigned old = ok ? cnt[w][d] : 0u;
+        dig[q] = d;
+        rank[q] = old + before;
+        __syncwarp();
+        if (ok && before == 0) cnt[w][d] = old + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int u = 0; u < BH_RS_BLOCK / 32; u++) {
+        const unsigned c = cnt[u][tid];
+        cnt[u][tid] = at;
+        at += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < BH_RS_ITEMS; q++)
+        if (k0 + 32 * q < n) {
+            const unsigned pos = cnt[w][dig[q]] + rank[q];
+            keys_out[pos] = key[q];
+            vals_out[pos] = val[q];
+        }
 }
 
 /* ---- 3. nodes -------------------------------------------------------------- */
@@ -1794,6 +1878,7 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
     ALLOC(t.val[0], cap);
     ALLOC(t.val[1], cap);
     ALLOC(t.hist, nb * BH_RS_BINS);
+    ALLOC(t.digits, BH_RS_PASSES * BH_RS_BINS);
     ALLOC(t.base, cap + 1);
     ALLOC(t.blk, nblk);
     ALLOC(t.mass, node_cap);
@@ -1836,13 +1921,15 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
 
 void nbg_bh_free(BhTree &t)
 {
-    void *ps[] = {t.key[0], t.key[1], t.val[0], t.val[1], t.hist, t.base, t.blk, t.mass, t.mx, t.my,
+    void *ps[] = {t.key[0], t.key[1], t.val[0], t.val[1], t.hist, t.digits, t.base, t.blk, t.mass, t.mx, t.my,
                   t.mz, t.cx, t.cy, t.cz, t.half, t.skip, t.start,
                   t.end, t.first, t.parent, t.flags, t.fa, t.fb, t.rec, t.shalf, t.fc, t.fd, t.cbase, t.ccount, t.slot,
                   t.sbox, t.scount, t.stree, t.sroot, t.sgrp, t.sunit};
     for (void *p : ps) cudaFree(p);
     memset(&t, 0, sizeof t);
 }
+
+static int bh_sort_wide(ll cap) { return (cap + BH_RS_TILE - 1) / BH_RS_TILE > BH_RS_NARROW; }
 
 /* The force and collision pass of one cycle (the replacement of the pair
  * kernel): bounds, keys, sort, nodes, masses, forces (FP64, or the mixed
@@ -1863,14 +1950,15 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
     /* eight passes of the key, then (several collections) two of the
      * collection index: an even count, so the sorted keys and values end in
      * buffer 0 */
-    const int passes = seg.nsims > 1 ? 10 : 8;
+    const int passes = seg.nsims > 1 ? BH_RS_PASSES : 8, wide = bh_sort_wide(cap);
     int in = 0;
     for (int pass = 0; pass < passes; pass++) {
         const int shift = pass < 8 ? 8 * pass : 0, simpass = pass < 8 ? -1 : pass - 8;
-        k_bh_rs_hist<<<nb, BH_RS_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], shift, simpass, t.hist);
-        k_bh_rs_scan<<<1, 1024, 0, st>>>(ctl, t.hist);
+        unsigned *digits = t.digits + pass * BH_RS_BINS;
+        k_bh_rs_hist<<<nb, BH_RS_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], shift, simpass, wide, t.hist, digits);
+        if (wide) k_bh_rs_scan<<<BH_RS_BINS / (BH_RS_BLOCK / 32), BH_RS_BLOCK, 0, st>>>(ctl, t.hist, digits);
         k_bh_rs_scatter<<<nb, BH_RS_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], t.key[in ^ 1], t.val[in ^ 1],
-                                                   shift, simpass, t.hist);
+                                                   shift, simpass, wide, t.hist, digits);
         in ^= 1;
     }
     const int sb = (int)(cap / BH_SCAN_TILE + 1);
@@ -1908,8 +1996,8 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
 
 int nbg_bh_launches(const CycleBufs &cb, bool mixed)
 {
-    const int passes = cb.seg.nsims > 1 ? 10 : 8;
+    const int passes = cb.seg.nsims > 1 ? BH_RS_PASSES : 8;
     /* reset, bounds, segs, keys; the sort; count, top, scan, roots, nodes;
      * children, masses; prep, walk; suns, collisions */
-    return 4 + 3 * passes + 5 + 2 + 2 + 2;
+    return 4 + (2 + bh_sort_wide(cb.cap)) * passes + 5 + 2 + 2 + 2;
 }

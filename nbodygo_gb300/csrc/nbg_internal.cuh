@@ -199,7 +199,8 @@ __device__ __forceinline__ int nbg_sim_of(const ll *off, int nsims, ll k)
 struct BhTree {
     ull *key[2];        /* octant-path keys (radix ping-pong) */
     unsigned *val[2];   /* body index (ping-pong partner) */
-    ll *hist;           /* radix digit histogram */
+    unsigned *hist;     /* radix digit histogram */
+    unsigned *digits;   /* and each pass's digit totals */
     ll *base;           /* nodes starting at each sorted position, then their scan */
     ll *blk;            /* per-block sums of that scan */
     double *mass, *mx, *my, *mz, *cx, *cy, *cz, *half;
