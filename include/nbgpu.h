@@ -371,8 +371,9 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
 #define NBG_OPT_GRAPH_CYCLES 6 /* cycles captured in one CUDA graph (default 1) */
 /* shape of the mixed pair kernel, 0..NBG_MIX_SHAPES-1 (see nbg_autotune).  A
  * context that was neither given one nor tuned nor restored from a snapshot takes a
- * one-sided shape (6 for fewer than 32,768 bodies in all, 2 for more), or 15
- * (symmetric) when every loaded collection has 98,304 bodies or more and the j
+ * one-sided shape (6 when every loaded collection is below 32,768 bodies, else
+ * 2), or 15 (symmetric) when every collection has 49,152 bodies or more, they
+ * make as many pairs of 512-body blocks as one of 98,304 does, and the j
  * partials fit in an eighth of the device's memory. */
 #define NBG_OPT_MIX_SHAPE 7
 #define NBG_MIX_SHAPES 19

@@ -419,36 +419,46 @@ __host__ __device__ __forceinline__ unsigned nbg_hilbert(unsigned x, unsigned y,
 #define NBG_MIX_K 4
 #define NBG_MIX_ITILE (NBG_MIX_BLOCK * NBG_MIX_K)
 
-/* The shape of a context that was not given one: one-sided, 256 bodies a tile,
- * with j tiles of 256 bodies (shape 2) or, for few bodies, of 128 (shape 6:
- * shorter careful passes; the longer tiles are 5% faster once they fill the
- * chip).  Shapes 0 / 2 / 6, pair pass in us: Plummer 2,000 bodies 110 / 97 /
- * 97, 20,000 424 / 227 / 202, 50,000 1,053 / 1,009 / 1,012, 131,072 6,652 /
- * 6,351 / 6,675.  Or the symmetric kernel when every collection has NBG_MIX_SYM_MIN_N bodies.  Fewer make too few block pairs to share
- * evenly, and the block pairs around a large body take longest: one-sided
- * against symmetric pair pass, in ms, for a uniform ball / a disk around a
- * star, 1.65 / 1.84 and 1.54 / 2.29 at 65,536 bodies, 3.61 / 3.74 and 2.84 /
+/* The shape of a context that was not given one.
+ *
+ * One-sided, 256 bodies a tile: with j tiles of 128 bodies (shape 6: shorter
+ * careful passes) for collections below NBG_MIX_FEW_N, of 256 (shape 2: 5%
+ * faster once near pairs are few) otherwise.  Shapes 0 / 2 / 6, pair pass in us:
+ * Plummer 2,000 bodies 110 / 97 / 97, 20,000 424 / 227 / 202, 50,000 1,053 /
+ * 1,009 / 1,012, 131,072 6,652 / 6,351 / 6,675; shapes 2 / 6, 512 spheres of 2,048
+ * 3,886 / 3,049, 128 of 8,192 3,928 / 3,760, 48 of 16,384 5,127 / 5,208.
+ *
+ * The symmetric kernel when every collection has NBG_MIX_SYM_MIN_N bodies (in
+ * smaller ones most block pairs hold near pairs: 128 Plummer spheres of 8,192
+ * take 6,168 us for 3,928 one-sided, 4 of 50,000 3,249 for 3,819) and there
+ * are NBG_MIX_SYM_MIN_UNITS block pairs in all, as one collection of 98,304 makes
+ * (fewer share unevenly, and those around a large body take longest).
+ * One-sided against symmetric, in ms, for a uniform ball / a disk around a
+ * star: 1.65 / 1.84 and 1.54 / 2.29 at 65,536 bodies, 3.61 / 3.74 and 2.84 /
  * 3.85 at 98,304, 6.34 / 6.45 and 4.91 / 5.68 at 131,072, 99.9 / 86.4 and
- * 75.4 / 66.1 at 524,288.  The symmetric kernel's j partials grow with
- * the square of the body count (units: block pairs, 6 KB each); more than an
- * eighth of the device's memory is not taken unasked. */
+ * 75.4 / 66.1 at 524,288.  Its j partials grow with the square of the body
+ * count (6 KB a block pair); more than an eighth of the device's memory is not
+ * taken unasked. */
 #define NBG_MIX_ONE_SIDED 2
 #define NBG_MIX_ONE_SIDED_FEW 6
 #define NBG_MIX_FEW_N 32768
-#define NBG_MIX_SYM_MIN_N 98304
+#define NBG_MIX_SYM_MIN_N 49152
+#define NBG_MIX_SYM_MIN_UNITS 18528
 static inline int nbg_default_shape(int nsims, const ll *counts, unsigned long long device_bytes)
 {
     unsigned long long units = 0;
-    ll n = 0;
-    for (int s = 0; s < nsims; s++) n += counts[s];
-    if (n < NBG_MIX_FEW_N) return NBG_MIX_ONE_SIDED_FEW;
+    ll least = 0, most = 0;
     for (int s = 0; s < nsims; s++) {
-        if (counts[s] < NBG_MIX_SYM_MIN_N) return NBG_MIX_ONE_SIDED;
+        least = s == 0 || counts[s] < least ? counts[s] : least;
+        most = counts[s] > most ? counts[s] : most;
         const unsigned long long T = ((unsigned long long)counts[s] + NBG_MIX_ITILE - 1) / NBG_MIX_ITILE;
         units += T * (T + 1) / 2;
     }
     const unsigned long long unit_bytes = 3ull * NBG_MIX_ITILE * sizeof(float);
-    return (units + units / 4) > device_bytes / 8 / unit_bytes ? NBG_MIX_ONE_SIDED : NBG_MIX_SYM;
+    if (least >= NBG_MIX_SYM_MIN_N && units >= NBG_MIX_SYM_MIN_UNITS &&
+        units + units / 4 <= device_bytes / 8 / unit_bytes)
+        return NBG_MIX_SYM;
+    return most < NBG_MIX_FEW_N ? NBG_MIX_ONE_SIDED_FEW : NBG_MIX_ONE_SIDED;
 }
 #define NBG_MIX_JT 256
 

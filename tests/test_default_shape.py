@@ -43,7 +43,7 @@ def run(b, shape=None, first=None):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,shape", [(3000, 6), (32767, 6), (32768, 2), (MIN_N - 1, 2), (MIN_N, A.MIX_SYM)])
+@pytest.mark.parametrize("n,shape", [(3000, 6), (32767, 6), (32768, 2), (MIN_N - 512, 2), (MIN_N, A.MIX_SYM)])
 def test_default_is_the_rules_shape(n, shape):
     b = W.uniform_ball(n)
     small, large = W.uniform_ball(2000), W.uniform_ball(MIN_N + 5)
