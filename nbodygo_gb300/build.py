@@ -36,7 +36,7 @@ UNITS = {
     "nbg_api.cu": [],
     "nbg_noalloc.cu": [],
 }
-HEADERS = ["nbg_internal.cuh", "nbg_exact.h", "nbg_octant.h", "nbg_math.h", "nbg_shared.h"]
+HEADERS = ["nbg_internal.cuh", "nbg_exact.h", "nbg_octant.h", "nbg_radix.cuh", "nbg_math.h", "nbg_shared.h"]
 
 
 def _nvcc():

@@ -61,17 +61,13 @@
 #include "nbg_internal.cuh"
 #include "nbg_math.h"
 #include "nbg_octant.h"
+#include "nbg_radix.cuh"
 #include "nbg_shared.h"
 
 #define BH_THETA 0.3
 #define BH_SOFTENING 1e-4
 #define BH_LEVELS NBG_OCT_LEVELS
 #define BH_BLOCK 256
-#define BH_RS_BLOCK 256
-#define BH_RS_ITEMS 4
-#define BH_RS_TILE (BH_RS_BLOCK * BH_RS_ITEMS)
-#define BH_RS_BINS 256
-#define BH_RS_NARROW 192 /* most blocks whose scatter sums the histogram itself */
 #define BH_RS_PASSES 10
 #define BH_SCAN_BLOCK 1024
 #define BH_SCAN_ITEMS 4
@@ -128,7 +124,7 @@ __device__ __forceinline__ void bh_root(const BhTree &t, int s, double &cx, doub
 __global__ void __launch_bounds__(1024) k_bh_reset(DevCtl *ctl, SimSegs seg, BhTree t)
 {
     if (ctl->error) return;
-    for (int d = threadIdx.x; d < BH_RS_PASSES * BH_RS_BINS; d += blockDim.x) t.digits[d] = 0;
+    for (int d = threadIdx.x; d < BH_RS_PASSES * RX_BINS; d += blockDim.x) t.digits[d] = 0;
     for (int s = threadIdx.x; s < seg.nsims; s += blockDim.x) {
         ull *b = t.sbox + 6 * (ll)s;
         for (int c = 0; c < 3; c++) {
@@ -336,140 +332,31 @@ __device__ __forceinline__ unsigned bh_digit(const SimSegs &seg, ull key, unsign
     return (d >> (8 * simpass)) & 0xffu;
 }
 
-/* A pass is a histogram of each block's BH_RS_TILE keys (with the digits'
- * totals, which all blocks add to), and a scatter.  Up to BH_RS_NARROW
- * blocks, the histogram lies block by block and each block of the scatter adds
- * up the rows of those before it; past that, the sum would grow with the square
- * of the blocks, and a scan between the two turns the histogram, digit by
- * digit, into offsets.  Small tiles, so 131,072 keys make 128 blocks, and no
- * barrier between a block's keys: a pass over 131,072 takes 12.6 us with the scan
- * (30.9 with tiles of 4,096 and a scan by one block), over 1,048,576 28.6 (63.8). */
-__global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_hist(DevCtl *ctl, SimSegs seg, const ull *keys,
-                                                          const unsigned *vals, int shift, int simpass, int wide,
-                                                          unsigned *hist, unsigned *digits)
+/* (nbg_radix.cuh; a pass over 131,072 keys takes 12.6 us with the scan, 30.9 with
+ * tiles of 4,096 and a scan by one block, over 1,048,576 28.6 and 63.8) */
+__global__ void __launch_bounds__(RX_BLOCK) k_bh_rs_hist(DevCtl *ctl, SimSegs seg, const ull *keys,
+                                                       const unsigned *vals, int shift, int simpass, int wide,
+                                                       unsigned *hist, unsigned *digits)
 {
-    __shared__ unsigned cnt[BH_RS_BINS];
     if (ctl->error) return;
-    const ll n = ctl->n;
-    const ll nb = (n + BH_RS_TILE - 1) / BH_RS_TILE;
-    const ll b = blockIdx.x;
-    if (b >= nb) return;
-    const int tid = threadIdx.x;
-    cnt[tid] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < BH_RS_ITEMS; q++) {
-        const ll k = b * BH_RS_TILE + (ll)q * BH_RS_BLOCK + tid;
-        if (k < n) atomicAdd(&cnt[bh_digit(seg, keys[k], simpass < 0 ? 0u : vals[k], shift, simpass)], 1u);
-    }
-    __syncthreads();
-    const unsigned c = cnt[tid];
-    hist[wide ? (ll)tid * nb + b : b * BH_RS_BINS + tid] = c;
-    if (c) atomicAdd(&digits[tid], c);
-}
-static_assert(BH_RS_BLOCK == BH_RS_BINS, "a thread per digit");
-
-/* thread d: the elements of the digits below d */
-__device__ __forceinline__ unsigned bh_digit_start(const unsigned *digits, unsigned *wtot)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned v = digits[threadIdx.x];
-    unsigned x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(FULL_MASK, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wtot[w] = x;
-    __syncthreads();
-    for (int u = 0; u < w; u++) x += wtot[u];
-    return x - v;
+    rx_hist(ctl->n, wide, hist, digits,
+            [&](ll k) { return bh_digit(seg, keys[k], simpass < 0 ? 0u : vals[k], shift, simpass); });
 }
 
-/* a warp to a digit's row of the histogram */
-__global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_scan(DevCtl *ctl, unsigned *hist, const unsigned *digits)
+__global__ void __launch_bounds__(RX_BLOCK) k_bh_rs_scan(DevCtl *ctl, unsigned *hist, const unsigned *digits)
 {
-    __shared__ unsigned wtot[BH_RS_BLOCK / 32], start[BH_RS_BINS];
     if (ctl->error) return;
-    const ll nb = (ctl->n + BH_RS_TILE - 1) / BH_RS_TILE;
-    const int lane = threadIdx.x & 31, d = blockIdx.x * (BH_RS_BLOCK / 32) + (threadIdx.x >> 5);
-    start[threadIdx.x] = bh_digit_start(digits, wtot);
-    __syncthreads();
-    unsigned carry = start[d];
-    unsigned *row = hist + (ll)d * nb;
-    for (ll c = 0; c < nb; c += 32) {
-        const unsigned v = c + lane < nb ? row[c + lane] : 0u;
-        unsigned x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(FULL_MASK, x, o);
-            if (lane >= o) x += y;
-        }
-        if (c + lane < nb) row[c + lane] = carry + x - v;
-        carry += __shfl_sync(FULL_MASK, x, 31);
-    }
+    rx_scan(ctl->n, hist, digits);
 }
 
-__global__ void __launch_bounds__(BH_RS_BLOCK) k_bh_rs_scatter(DevCtl *ctl, SimSegs seg, const ull *keys_in,
-                                                             const unsigned *vals_in, ull *keys_out,
-                                                             unsigned *vals_out, int shift, int simpass, int wide,
-                                                             const unsigned *hist, const unsigned *digits)
+__global__ void __launch_bounds__(RX_BLOCK) k_bh_rs_scatter(DevCtl *ctl, SimSegs seg, const ull *keys_in,
+                                                          const unsigned *vals_in, ull *keys_out, unsigned *vals_out,
+                                                          int shift, int simpass, int wide, const unsigned *hist,
+                                                          const unsigned *digits)
 {
-    __shared__ unsigned wtot[BH_RS_BLOCK / 32], cnt[BH_RS_BLOCK / 32][BH_RS_BINS];
     if (ctl->error) return;
-    const ll n = ctl->n;
-    const ll nb = (n + BH_RS_TILE - 1) / BH_RS_TILE;
-    const ll b = blockIdx.x;
-    if (b >= nb) return;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    /* a warp's keys are consecutive: its first, then 32 at a time */
-    const ll k0 = b * BH_RS_TILE + (ll)w * (32 * BH_RS_ITEMS) + lane;
-    ull key[BH_RS_ITEMS];
-    unsigned val[BH_RS_ITEMS], rank[BH_RS_ITEMS], dig[BH_RS_ITEMS];
-#pragma unroll
-    for (int q = 0; q < BH_RS_ITEMS; q++) {
-        const bool ok = k0 + 32 * q < n;
-        key[q] = ok ? keys_in[k0 + 32 * q] : 0ull;
-        val[q] = ok ? vals_in[k0 + 32 * q] : 0u;
-    }
-    /* where the block's elements of digit tid start */
-    unsigned at;
-    if (wide) {
-        at = hist[(ll)tid * nb + b];
-    } else {
-        at = bh_digit_start(digits, wtot);
-        const unsigned *h = hist + tid;
-#pragma unroll 8
-        for (int u = 0; u < (int)b; u++) at += h[u * BH_RS_BINS];
-    }
-    for (int c = tid; c < BH_RS_BINS * (BH_RS_BLOCK / 32); c += BH_RS_BLOCK) (&cnt[0][0])[c] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < BH_RS_ITEMS; q++) {
-        const bool ok = k0 + 32 * q < n;
-        const unsigned d = ok ? bh_digit(seg, key[q], val[q], shift, simpass) : BH_RS_BINS;
-        const unsigned peers = __match_any_sync(FULL_MASK, d);
-        const unsigned before = __popc(peers & lt);
-        const unsigned old = ok ? cnt[w][d] : 0u;
-        dig[q] = d;
-        rank[q] = old + before;
-        __syncwarp();
-        if (ok && before == 0) cnt[w][d] = old + __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int u = 0; u < BH_RS_BLOCK / 32; u++) {
-        const unsigned c = cnt[u][tid];
-        cnt[u][tid] = at;
-        at += c;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < BH_RS_ITEMS; q++)
-        if (k0 + 32 * q < n) {
-            const unsigned pos = cnt[w][dig[q]] + rank[q];
-            keys_out[pos] = key[q];
-            vals_out[pos] = val[q];
-        }
+    rx_scatter(ctl->n, wide, keys_in, vals_in, keys_out, vals_out, hist, digits,
+               [&](ull key, unsigned val) { return bh_digit(seg, key, val, shift, simpass); });
 }
 
 /* ---- 3. nodes -------------------------------------------------------------- */
@@ -1869,7 +1756,7 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_collide(BodyArrays A, DevCtl *c
 int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
 {
     nbg_bh_free(t);
-    const ll nb = (cap + BH_RS_TILE - 1) / BH_RS_TILE;
+    const ll nb = rx_blocks(cap);
     const ll nblk = cap / BH_SCAN_TILE + 2;
     bool ok = true;
 #define ALLOC(p, cnt) ok = ok && cudaMalloc((void **)&(p), (size_t)(cnt) * sizeof(*(p))) == cudaSuccess
@@ -1877,8 +1764,8 @@ int nbg_bh_alloc(BhTree &t, ll cap, ll node_cap)
     ALLOC(t.key[1], cap);
     ALLOC(t.val[0], cap);
     ALLOC(t.val[1], cap);
-    ALLOC(t.hist, nb * BH_RS_BINS);
-    ALLOC(t.digits, BH_RS_PASSES * BH_RS_BINS);
+    ALLOC(t.hist, nb * RX_BINS);
+    ALLOC(t.digits, BH_RS_PASSES * RX_BINS);
     ALLOC(t.base, cap + 1);
     ALLOC(t.blk, nblk);
     ALLOC(t.mass, node_cap);
@@ -1929,8 +1816,6 @@ void nbg_bh_free(BhTree &t)
     memset(&t, 0, sizeof t);
 }
 
-static int bh_sort_wide(ll cap) { return (cap + BH_RS_TILE - 1) / BH_RS_TILE > BH_RS_NARROW; }
-
 /* The force and collision pass of one cycle (the replacement of the pair
  * kernel): bounds, keys, sort, nodes, masses, forces (FP64, or the mixed
  * walk), suns, collisions. */
@@ -1946,18 +1831,18 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
     k_bh_bounds<<<g, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t);
     k_bh_segs<<<1, 32, 0, st>>>(ctl, seg, t);
     k_bh_keys<<<g, BH_BLOCK, 0, st>>>(cb.a, ctl, seg, t, t.key[0], t.val[0]);
-    const int nb = (int)((cap + BH_RS_TILE - 1) / BH_RS_TILE);
+    const int nb = (int)rx_blocks(cap);
     /* eight passes of the key, then (several collections) two of the
      * collection index: an even count, so the sorted keys and values end in
      * buffer 0 */
-    const int passes = seg.nsims > 1 ? BH_RS_PASSES : 8, wide = bh_sort_wide(cap);
+    const int passes = seg.nsims > 1 ? BH_RS_PASSES : 8, wide = rx_wide(cap);
     int in = 0;
     for (int pass = 0; pass < passes; pass++) {
         const int shift = pass < 8 ? 8 * pass : 0, simpass = pass < 8 ? -1 : pass - 8;
-        unsigned *digits = t.digits + pass * BH_RS_BINS;
-        k_bh_rs_hist<<<nb, BH_RS_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], shift, simpass, wide, t.hist, digits);
-        if (wide) k_bh_rs_scan<<<BH_RS_BINS / (BH_RS_BLOCK / 32), BH_RS_BLOCK, 0, st>>>(ctl, t.hist, digits);
-        k_bh_rs_scatter<<<nb, BH_RS_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], t.key[in ^ 1], t.val[in ^ 1],
+        unsigned *digits = t.digits + pass * RX_BINS;
+        k_bh_rs_hist<<<nb, RX_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], shift, simpass, wide, t.hist, digits);
+        if (wide) k_bh_rs_scan<<<RX_BINS / RX_WARPS, RX_BLOCK, 0, st>>>(ctl, t.hist, digits);
+        k_bh_rs_scatter<<<nb, RX_BLOCK, 0, st>>>(ctl, seg, t.key[in], t.val[in], t.key[in ^ 1], t.val[in ^ 1],
                                                    shift, simpass, wide, t.hist, digits);
         in ^= 1;
     }
@@ -1999,5 +1884,5 @@ int nbg_bh_launches(const CycleBufs &cb, bool mixed)
     const int passes = cb.seg.nsims > 1 ? BH_RS_PASSES : 8;
     /* reset, bounds, segs, keys; the sort; count, top, scan, roots, nodes;
      * children, masses; prep, walk; suns, collisions */
-    return 4 + (2 + bh_sort_wide(cb.cap)) * passes + 5 + 2 + 2 + 2;
+    return 4 + (2 + rx_wide(cb.cap)) * passes + 5 + 2 + 2 + 2;
 }

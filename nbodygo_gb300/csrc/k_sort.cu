@@ -21,6 +21,7 @@
  * Bodies with a non-finite position or NaN radius sort last (key 2^30).
  */
 #include "nbg_internal.cuh"
+#include "nbg_radix.cuh"
 
 #define RS_BLOCK 256
 #define RS_ITEMS 16
@@ -34,7 +35,8 @@ __device__ __forceinline__ unsigned quant10(float x, float inv_span)
     return (unsigned)t;
 }
 
-/* Keys of the bodies 0..n-1 and the identity permutation.  One sim: a 30-bit
+/* Keys of the bodies 0..n-1 and the identity permutation (and no digits
+ * counted).  One sim: a 30-bit
  * Hilbert key over [-x_max, x_max]^3.  Several sims: the sim index in the top
  * 11 bits and a 21-bit Hilbert key over the sim's own box, so every sim keeps
  * its range of positions and is ordered inside it. */
@@ -59,30 +61,55 @@ __device__ __forceinline__ unsigned order_key(const BodyArrays &A, const DevCtl 
     return ((unsigned)sim << 21) | m;
 }
 
-__global__ void k_order_keys(BodyArrays A, DevCtl *ctl, SimSegs seg, unsigned *keys, unsigned *vals)
+__global__ void k_order_keys(BodyArrays A, DevCtl *ctl, SimSegs seg, unsigned *keys, unsigned *vals, unsigned *digits)
 {
     if (ctl->error || !ctl->sort_now) return;
     const ll n = ctl->n;
+    if (blockIdx.x == 0)
+        for (int d = threadIdx.x; d < 4 * RX_BINS; d += blockDim.x) digits[d] = 0;
     for (ll k = (ll)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (ll)gridDim.x * blockDim.x) {
         keys[k] = order_key(A, ctl, seg, k);
         vals[k] = (unsigned)k;
     }
 }
 
-/* What a radix pass sorts.  RS_ORDER: the bodies' Hilbert keys (32-bit,
- * with the permutation as values), in cycles that sort.  RS_EVENTS: the
+/* One pass over the Hilbert keys (nbg_radix.cuh), with the permutation as
+ * values, in cycles that sort.  20,011 bodies make 20 blocks, where tiles of
+ * 4,096 made 5: 23.5 -> 10.3 us a pass under the profiler. */
+__global__ void __launch_bounds__(RX_BLOCK) k_order_hist(DevCtl *ctl, const unsigned *keys, int shift, int wide,
+                                                         unsigned *hist, unsigned *digits)
+{
+    if (ctl->error || !ctl->sort_now) return;
+    rx_hist(ctl->n, wide, hist, digits, [&](ll k) { return (keys[k] >> shift) & 0xffu; });
+}
+
+__global__ void __launch_bounds__(RX_BLOCK) k_order_scan(DevCtl *ctl, unsigned *hist, const unsigned *digits)
+{
+    if (ctl->error || !ctl->sort_now) return;
+    rx_scan(ctl->n, hist, digits);
+}
+
+__global__ void __launch_bounds__(RX_BLOCK) k_order_scatter(DevCtl *ctl, const unsigned *keys_in,
+                                                            const unsigned *vals_in, unsigned *keys_out,
+                                                            unsigned *vals_out, int shift, int wide,
+                                                            const unsigned *hist, const unsigned *digits)
+{
+    if (ctl->error || !ctl->sort_now) return;
+    rx_scatter(ctl->n, wide, keys_in, vals_in, keys_out, vals_out, hist, digits,
+               [&](unsigned key, unsigned) { return (key >> shift) & 0xffu; });
+}
+
+/* What a radix pass of the kernels below sorts.  RS_EVENTS: the
  * detected events' 64-bit keys i<<32 | j<<2 | type, when there are more than
  * the one-block sort of k_cycle.cu holds.  The count comes from the control
  * block, so one captured graph serves every count: passes with nothing to
  * sort return at once. */
-#define RS_ORDER 0
 #define RS_EVENTS 1
 #define RS_INCIDENCES 2 /* two (body, event) keys per event, for the resolution's links */
 
 __device__ __forceinline__ ll rs_count(const DevCtl *ctl, int what)
 {
     if (ctl->error) return 0;
-    if (what == RS_ORDER) return ctl->sort_now ? ctl->n : 0;
     if (ctl->ev_count <= NBG_EV_BLOCK_SORT) return 0;
     return what == RS_EVENTS ? ctl->ev_count : 2 * ctl->ev_count;
 }
@@ -204,63 +231,6 @@ __global__ void __launch_bounds__(1024) k_rs_scan_fin(DevCtl *ctl, int what, ll 
     }
 }
 
-/* The histogram and its scan in one launch, for histograms of at most
- * one scan chunk: the block that arrives last scans them all.  The order of
- * up to 131,072 bodies takes 9 launches in place of 21 (20,011 bodies, mean of
- * a cycle that sorts and three that keep their order: 64 us against 101); a
- * longer histogram would leave the last block's 256 threads a scan of more than
- * 32 entries each, and keeps its three launches. */
-template <typename K>
-__global__ void __launch_bounds__(RS_BLOCK) k_rs_hist_scan(DevCtl *ctl, int what, const K *keys, int shift, ll *hist)
-{
-    __shared__ unsigned cnt[RS_BINS];
-    __shared__ ll wtot[RS_BLOCK / 32];
-    __shared__ unsigned s_last;
-    const ll n = rs_count(ctl, what);
-    if (n == 0) return;
-    const ll nb = (n + RS_TILE - 1) / RS_TILE;
-    const ll b = blockIdx.x;
-    if (b >= nb) return;
-    for (int d = threadIdx.x; d < RS_BINS; d += RS_BLOCK) cnt[d] = 0;
-    __syncthreads();
-    const ll base = b * RS_TILE;
-    for (int q = 0; q < RS_ITEMS; q++) {
-        ll k = base + (ll)q * RS_BLOCK + threadIdx.x;
-        if (k < n) atomicAdd(&cnt[(unsigned)(keys[k] >> shift) & 0xffu], 1u);
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < RS_BINS; d += RS_BLOCK) hist[(ll)d * nb + b] = cnt[d];
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_last = atomicAdd(&ctl->ticket, 1u) == (unsigned)nb - 1u ? 1u : 0u;
-        if (s_last) ctl->ticket = 0;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    /* thread d takes digit d's nb entries */
-    ll *row = hist + (ll)threadIdx.x * nb;
-    ll s = 0;
-    for (ll q = 0; q < nb; q++) s += __ldcg(&row[q]);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    ll x = s;
-    for (int o = 1; o < 32; o <<= 1) {
-        const ll y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wtot[w] = x;
-    __syncthreads();
-    ll ex = x - s;
-    for (int v = 0; v < w; v++) ex += wtot[v];
-    for (ll q = 0; q < nb; q++) {
-        const ll v = __ldcg(&row[q]);
-        row[q] = ex;
-        ex += v;
-    }
-}
-static_assert(RS_BLOCK == RS_BINS, "a thread per digit");
-
 /* stable scatter: element order within a block is kept per digit (vals
  * NULL: keys only) */
 template <typename K>
@@ -304,6 +274,9 @@ __global__ void __launch_bounds__(RS_BLOCK) k_rs_scatter(DevCtl *ctl, int what, 
         __syncthreads();
     }
 }
+
+/* the order's scratch: four passes' digit totals, and a histogram */
+ll nbg_order_scratch(ll cap) { return 4 * RX_BINS + rx_blocks(cap) * RX_BINS; }
 
 /* the histogram plus its chunk sums */
 ll nbg_sort_scratch_hist(ll cap)
@@ -400,21 +373,15 @@ void nbg_launch_spatial_sort(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
         return;
     }
     const int g = nbg_flat_grid(cb, cb.cap);
-    k_order_keys<<<g, 256, 0, st>>>(cb.a, ctl, cb.seg, cb.skey[0], cb.perm);
-    const int nb = (int)((cb.cap + RS_TILE - 1) / RS_TILE);
-    const int nchunk = (int)(((ll)nb * RS_BINS + RS_SCAN_CHUNK - 1) / RS_SCAN_CHUNK);
+    k_order_keys<<<g, 256, 0, st>>>(cb.a, ctl, cb.seg, cb.skey[0], cb.perm, cb.shist);
+    const int nb = (int)rx_blocks(cb.cap), wide = rx_wide(cb.cap);
     unsigned *kin = cb.skey[0], *vin = cb.perm, *kout = cb.skey[1], *vout = cb.sval;
     for (int pass = 0; pass < 4; pass++) {
         const int shift = 8 * pass;
-        if (nchunk == 1) {
-            k_rs_hist_scan<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, shift, cb.shist);
-        } else {
-            k_rs_hist<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, shift, cb.shist);
-            k_rs_scan_part<<<nchunk, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
-            k_rs_scan_top<<<1, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
-            k_rs_scan_fin<<<nchunk, 1024, 0, st>>>(ctl, RS_ORDER, cb.shist);
-        }
-        k_rs_scatter<unsigned><<<nb, RS_BLOCK, 0, st>>>(ctl, RS_ORDER, kin, vin, kout, vout, shift, cb.shist);
+        unsigned *digits = cb.shist + pass * RX_BINS, *hist = cb.shist + 4 * RX_BINS;
+        k_order_hist<<<nb, RX_BLOCK, 0, st>>>(ctl, kin, shift, wide, hist, digits);
+        if (wide) k_order_scan<<<RX_BINS / RX_WARPS, RX_BLOCK, 0, st>>>(ctl, hist, digits);
+        k_order_scatter<<<nb, RX_BLOCK, 0, st>>>(ctl, kin, vin, kout, vout, shift, wide, hist, digits);
         unsigned *t = kin;
         kin = kout;
         kout = t;
@@ -428,8 +395,7 @@ void nbg_launch_spatial_sort(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
 int nbg_spatial_sort_launches(const CycleBufs &cb)
 {
     if (cb.cap <= RSS_MAX) return 1;
-    const ll hist = ((cb.cap + RS_TILE - 1) / RS_TILE) * RS_BINS;
-    return 1 + 4 * (hist <= RS_SCAN_CHUNK ? 2 : 5);
+    return 1 + 4 * (2 + rx_wide(cb.cap));
 }
 
 /* Events beyond the one-block sort: a stable LSD radix sort of their keys

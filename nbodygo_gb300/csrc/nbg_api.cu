@@ -371,7 +371,7 @@ static int ensure_cap(nbg_ctx *ctx, ll need, ll keep)
     CAP_ALLOC(ctx->cb.sval, cap * sizeof(unsigned));
     CAP_ALLOC(ctx->cb.skey[0], cap * sizeof(unsigned));
     CAP_ALLOC(ctx->cb.skey[1], cap * sizeof(unsigned));
-    CAP_ALLOC(ctx->cb.shist, nbg_sort_scratch_hist(cap) * sizeof(ll));
+    CAP_ALLOC(ctx->cb.shist, nbg_order_scratch(cap) * sizeof(unsigned));
 #undef CAP_ALLOC
     if (e != cudaSuccess) {
         const std::string m = "buffers for " + std::to_string(cap) + " bodies: " + cudaGetErrorString(e) +

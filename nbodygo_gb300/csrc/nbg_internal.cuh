@@ -265,7 +265,7 @@ struct CycleBufs {
     unsigned *perm;     /* sorted position -> body index */
     unsigned *skey[2];  /* radix-sort keys (ping-pong) */
     unsigned *sval;     /* radix-sort values (ping-pong partner of perm) */
-    ll *shist;          /* radix-sort digit histogram / offsets */
+    unsigned *shist;    /* the spatial order's digit totals and histogram (nbg_order_scratch) */
     ll part_doubles;    /* size of part */
     int work_cap;       /* most CTAs the mixed pair work is divided among (0 = slots) */
     int slots;          /* resident CTAs of the mixed kernel on this device */
@@ -523,6 +523,7 @@ void nbg_launch_event_radix(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
 ull *nbg_launch_incidence_radix(const CycleBufs &cb, DevCtl *ctl, int bits, cudaStream_t st);
 int nbg_event_radix_launches(const CycleBufs &cb);
 ll nbg_sort_scratch_hist(ll cap);
+ll nbg_order_scratch(ll cap);
 
 /* k_probe.cu */
 int nbg_run_probes(int device, double *fp32, double *fp64, double *mhz);

@@ -22,6 +22,7 @@
 #include <string>
 
 #include "nbg_internal.cuh"
+#include "nbg_radix.cuh"
 
 /* partial sums: 786,432 doubles, 512 slots of a 512-body i-tile; a 65,536-body
  * collection has 128 i-tiles, which leaves room for 385 CTAs */
@@ -41,10 +42,9 @@ static constexpr size_t OFF_SVAL = OFF_PERM + align256((size_t)NBG_NOALLOC_MAX_B
 static constexpr size_t OFF_KEY0 = OFF_SVAL + align256((size_t)NBG_NOALLOC_MAX_BODIES * 4);
 static constexpr size_t OFF_KEY1 = OFF_KEY0 + align256((size_t)NBG_NOALLOC_MAX_BODIES * 4);
 static constexpr size_t OFF_HIST = OFF_KEY1 + align256((size_t)NBG_NOALLOC_MAX_BODIES * 4);
-/* radix-sort histogram: 256 digits per 4096-body block, then one sum per
- * 8192-entry chunk of it */
-static constexpr size_t HIST_ENTRIES = (size_t)((NBG_NOALLOC_MAX_BODIES + 4095) / 4096) * 256;
-static constexpr size_t HIST_BYTES = (HIST_ENTRIES + (HIST_ENTRIES + 8191) / 8192) * 8;
+/* the order's digit totals and its histogram, 256 digits per RX_TILE bodies */
+static constexpr size_t HIST_BYTES =
+    (4 * RX_BINS + (size_t)((NBG_NOALLOC_MAX_BODIES + RX_TILE - 1) / RX_TILE) * RX_BINS) * 4;
 /* the per-sim layout arrays of one collection */
 static constexpr size_t OFF_SEG = OFF_HIST + align256(HIST_BYTES);
 static constexpr size_t TOTAL_BYTES = OFF_SEG + align256(NBG_SEG_BYTES(1));
@@ -171,7 +171,7 @@ extern "C" int nbg_forces_mixed_noalloc(const double *x, const double *y, const 
     cb.sval = (unsigned *)(base + OFF_SVAL);
     cb.skey[0] = (unsigned *)(base + OFF_KEY0);
     cb.skey[1] = (unsigned *)(base + OFF_KEY1);
-    cb.shist = (ll *)(base + OFF_HIST);
+    cb.shist = (unsigned *)(base + OFF_HIST);
     cb.ev_keys = nullptr; /* events are discarded */
     cb.ev_cap = 0;
     cb.part_doubles = NOALLOC_PART_DOUBLES;
