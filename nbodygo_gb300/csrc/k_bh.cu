@@ -572,8 +572,8 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_nodes(DevCtl *ctl, SimSegs seg,
  * the children in their order: an FP64 add costs the same for one lane as for
  * 32, and one lane a node would spend four times as many.  (The centres of mass
  * are divided out with every lane busy, in the preparation of the walks.)  One
- * launch where each of 22 levels' launches read every node's level: 194 -> 47 us
- * for 131,072 Plummer bodies, 785 -> 210 us for 1,048,576 uniform ones. */
+ * launch where each of 22 levels' launches read every node's level: 290 -> 71 us
+ * for 131,072 Plummer bodies, 785 -> 313 us for 1,000,003 uniform ones. */
 __global__ void __launch_bounds__(BH_BLOCK) k_bh_mass(BodyArrays A, DevCtl *ctl, const unsigned *vals, BhTree t)
 {
     if (ctl->error) return;
@@ -1125,8 +1125,8 @@ __global__ void __launch_bounds__(BHW_BLOCK, 5) k_bh_force(const __grid_constant
  *
  * A walk that took one node at a time for the whole warp was bound by the
  * latency of its node loads (issue slots 25 % busy).  The walk of a 131,072-
- * body Plummer sphere went from 5.0 to 1.56 ms, of 10^6 uniform bodies from
- * 20.3 to 7.3 ms.  What bounds it now is issue and, with a group to a warp,
+ * body Plummer sphere went from 5.0 to 1.54 ms, of 10^6 uniform bodies from
+ * 20.3 to 7.2 ms.  What bounds it now is issue and, with a group to a warp,
  * groups of uneven cost: 263,000 instructions a group before the lists were
  * split into far and near ones, 60 % of them in the sums. */
 /* every node's record for the walk, in its slot */

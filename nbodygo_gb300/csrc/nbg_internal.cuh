@@ -301,7 +301,7 @@ struct MixVariantInfo {
 };
 #define NBG_MIX_VARIANTS NBG_MIX_SHAPES
 /* the symmetric kernel (each unordered pair once, k_pair_sym): shapes 15
- * and 16 (registers capped for 4 and 5 CTAs per SM) */
+ * and 16 (registers capped for 3 and 4 CTAs per SM) */
 #define NBG_MIX_SYM 15
 __host__ __device__ __forceinline__ bool nbg_mix_is_sym(int variant)
 {
