@@ -372,7 +372,7 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
 /* shape of the mixed pair kernel, 0..NBG_MIX_SHAPES-1 (see nbg_autotune).  A
  * context that was neither given one nor tuned nor restored from a snapshot takes a
  * one-sided shape (6 when every loaded collection is below 32,768 bodies, else
- * 2), or 15 (symmetric) when every collection has 49,152 bodies or more, they
+ * 2), or 15 (symmetric) when every collection has 24,576 bodies or more, they
  * make as many pairs of 512-body blocks as one of 98,304 does, and the j
  * partials fit in an eighth of the device's memory. */
 #define NBG_OPT_MIX_SHAPE 7

@@ -430,7 +430,9 @@ __host__ __device__ __forceinline__ unsigned nbg_hilbert(unsigned x, unsigned y,
  *
  * The symmetric kernel when every collection has NBG_MIX_SYM_MIN_N bodies (in
  * smaller ones most block pairs hold near pairs: 128 Plummer spheres of 8,192
- * take 6,168 us for 3,928 one-sided, 4 of 50,000 3,249 for 3,819) and there
+ * take 6,168 us for 3,928 one-sided, 40 of 20,000 6,846 for 6,276, 30 of 24,000
+ * 6,160 for 6,676, 4 of 50,000 3,249 for 3,819; 200 of 256 to 32,768 8,843 for
+ * 8,311) and there
  * are NBG_MIX_SYM_MIN_UNITS block pairs in all, as one collection of 98,304 makes
  * (fewer share unevenly, and those around a large body take longest).
  * One-sided against symmetric, in ms, for a uniform ball / a disk around a
@@ -442,7 +444,7 @@ __host__ __device__ __forceinline__ unsigned nbg_hilbert(unsigned x, unsigned y,
 #define NBG_MIX_ONE_SIDED 2
 #define NBG_MIX_ONE_SIDED_FEW 6
 #define NBG_MIX_FEW_N 32768
-#define NBG_MIX_SYM_MIN_N 49152
+#define NBG_MIX_SYM_MIN_N 24576
 #define NBG_MIX_SYM_MIN_UNITS 18528
 static inline int nbg_default_shape(int nsims, const ll *counts, unsigned long long device_bytes)
 {

@@ -33,13 +33,13 @@ int main()
     want(3, mixed, big, NBG_MIX_ONE_SIDED);
     want(2, small, big, NBG_MIX_ONE_SIDED);
     // every unit counts: collections that are too few alone, and that fit alone
-    static ll some[4], many[64], batch[1000];
+    static ll some[16], many[64], batch[1000];
     for (ll &c : some) c = k;
     for (ll &c : many) c = 1 << 18;
-    for (ll &c : batch) c = NBG_MIX_FEW_N - 1;
-    want(1, some, big, NBG_MIX_ONE_SIDED);
-    want(3, some, big, NBG_MIX_ONE_SIDED);
-    want(4, some, big, NBG_MIX_SYM);
+    for (ll &c : batch) c = NBG_MIX_SYM_MIN_N - 1;
+    want(1, some, big, NBG_MIX_ONE_SIDED_FEW);
+    want(15, some, big, NBG_MIX_ONE_SIDED_FEW);
+    want(16, some, big, NBG_MIX_SYM);
     want(1, many, big, NBG_MIX_SYM);
     want(64, many, big, NBG_MIX_ONE_SIDED);
     want(1000, batch, big, NBG_MIX_ONE_SIDED_FEW);
