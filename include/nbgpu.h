@@ -432,7 +432,7 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value);
  * threads per CTA x i-bodies per thread, j per shared-memory tile, unroll,
  * CTAs per SM, in three kinds: sums in registers (R), sums in shared memory
  * (S), and shared memory with two j-tile buffers filled a tile ahead (D):
- *   0: R 128x4, 256, 2, 3 (default)  1: R 128x4, 256, 1, 3  2: R 128x2, 256, 2, 4
+ *   0: R 128x4, 256, 2, 3            1: R 128x4, 256, 1, 3  2: R 128x2, 256, 2, 4
  *   3: R 256x2, 256, 2, 2            4: R 128x4, 512, 2, 3  5: R 64x4, 256, 2, 6
  *   6: R 128x2, 128, 4, 4            7: S 128x2, 256, 2, 5  8: S 128x3, 256, 2, 4
  *   9: S 128x4, 256, 2, 4           10: S 128x4, 128, 4, 4 11: D 128x2, 128, 4, 4

@@ -577,7 +577,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(ull *bar, unsigned parity)
  * event keys. */
 template <int BLOCK, int K, int JT, int UNROLL, int MINB, bool SF, bool DB, bool BULK>
 __global__ void __launch_bounds__(BLOCK, MINB)
-k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi, const float4 *__restrict__ jlo,
+k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi,
+             const float4 *__restrict__ jlo,
              const float4 *__restrict__ tile_c, const float4 *__restrict__ iprep, const unsigned *__restrict__ perm,
              double *__restrict__ part, ull *ev_keys, ll ev_cap)
 {
@@ -1018,7 +1019,7 @@ __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A
 #define SYM_JP (SYM_B / 2)    /* j pairs per block */
 #define SYM_NSUB (SYM_B / 64) /* 64-j sub-blocks a warp rotates through */
 #define SYM_FOLD 4            /* sub-blocks between folds of the i-sums */
-static_assert(SYM_B == NBG_MIX_ITILE, "blocks are the i-tiles of the default shape");
+static_assert(SYM_B == NBG_MIX_ITILE, "blocks are the i-tiles that sums and j partials are sized by");
 static_assert(SYM_NSUB % SYM_FOLD == 0, "whole folds per unit");
 
 /* first unit of row a in a collection of T blocks (rows a .. T-1 wide) */
@@ -1108,7 +1109,8 @@ struct SymNear {
 
 template <int MINB>
 __global__ void __launch_bounds__(SYM_THREADS, MINB)
-k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi, const float4 *__restrict__ jlo,
+k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jhi,
+           const float4 *__restrict__ jlo,
            const float4 *__restrict__ tile_c, const float2 *__restrict__ tile_r, const float4 *__restrict__ iprep,
            const unsigned *__restrict__ perm, double *__restrict__ part, float *__restrict__ jpart, ull *ev_keys,
            ll ev_cap)

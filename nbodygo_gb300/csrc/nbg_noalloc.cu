@@ -176,7 +176,7 @@ extern "C" int nbg_forces_mixed_noalloc(const double *x, const double *y, const 
     cb.ev_cap = 0;
     cb.part_doubles = NOALLOC_PART_DOUBLES;
     cb.work_cap = 0;
-    cb.mix_variant = 0; /* the default shape: 512-body i-tiles */
+    cb.mix_variant = 0; /* 512-body i-tiles, which the scratch is sized for */
     cb.itile = NBG_MIX_ITILE;
     cb.slots = nbg_mixed_slots(dev, 0);
     if (cudaDeviceGetAttribute(&cb.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || cb.sms < 1)
