@@ -460,7 +460,9 @@ __device__ __forceinline__ void near_pair(const BodyArrays &A, DevCtl *ctl, ull 
     two_sum_add(t.hz, t.lz, s * dz);
 }
 
-/* The careful pass over one j tile (jpv j pairs in sA, sB from position jt)
+/* The careful pass over one j tile (jn bodies in sA, sB from position jt; the
+ * tile is filled up with sentinels, which a large enough threshold takes in
+ * too, and whose positions may hold another collection's body or none)
  * for body p, which met a near pair in it (its own body, in its own tile):
  * the fast pass again, four j at a time, with each near pair taken out of
  * the packed sum (moved so far away that its term is zero) and added exactly
@@ -474,13 +476,13 @@ __device__ __forceinline__ void near_pair(const BodyArrays &A, DevCtl *ctl, ull 
 __device__ __noinline__ TileSum careful_tile(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
                                              const unsigned *__restrict__ perm, const float4 *__restrict__ jhi,
                                              const float4 *__restrict__ jlo, const float4 *sA, const float4 *sB,
-                                             int jpv, ll jt, ll p, float nx, float ny, float nz, float thk)
+                                             int jn, ll jt, ll p, float nx, float ny, float nz, float thk)
 {
     TileSum mine = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float4 hi_i = jhi[p], lo_i = jlo[p];
     float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
 #pragma unroll 1
-    for (int pp = 0; pp < jpv; pp += 2) {
+    for (int pp = 0; 2 * pp < jn; pp += 2) {
         float2 dx[2], dy[2], dz[2], r2[2], mj[2];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -496,15 +498,15 @@ __device__ __noinline__ TileSum careful_tile(const BodyArrays &A, DevCtl *ctl, u
         unsigned hit = (r2[0].x < thk ? 1u : 0u) | (r2[0].y < thk ? 2u : 0u) | (r2[1].x < thk ? 4u : 0u) |
                        (r2[1].y < thk ? 8u : 0u);
         if (hit) {
+            if (jn - 2 * pp < 4) hit &= (1u << (jn - 2 * pp)) - 1u; /* no sentinels */
             if (hit & 1u) r2[0].x = FAR_R2;
             if (hit & 2u) r2[0].y = FAR_R2;
             if (hit & 4u) r2[1].x = FAR_R2;
             if (hit & 8u) r2[1].y = FAR_R2;
-            do {
+            for (; hit; hit &= hit - 1u) {
                 const ll q = jt + 2 * pp + __ffs(hit) - 1;
-                hit &= hit - 1u;
                 if (q != p) near_pair(A, ctl, ev_keys, ev_cap, perm, p, q, hi_i, lo_i, jhi[q], jlo[q], mine);
-            } while (hit);
+            }
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -797,10 +799,8 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
                 ax[k] = ay[k] = az[k] = make_float2(0.f, 0.f);
                 mn[k] = 3.0e38f;
             }
-            /* the j pairs this tile holds (a segment's last tile is short) */
-            /* j pairs of this tile that hold bodies: JP, except in a
-             * segment's short last tile */
-            const int jpv = je - jt >= JT ? JP : (int)((je - jt + 1) / 2);
+            /* bodies of this tile: JT, except in a segment's short last tile */
+            const int jn = je - jt >= JT ? JT : (int)(je - jt);
             auto pair_step = [&](int pp) {
                 const float4 a = sA[pp], b = sB[pp];
                 const float2 xj = make_float2(a.x, a.y), yj = make_float2(a.z, a.w);
@@ -826,12 +826,12 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
             /* a full tile keeps a constant trip count for the unroller; a short
              * one runs on to a multiple of four pairs (the rest of the tile
              * holds sentinels, whose terms are zero) */
-            if (jpv == JP) {
+            if (jn == JT) {
 #pragma unroll UNROLL
                 for (int pp = 0; pp < JP; pp++) pair_step(pp);
             } else {
 #pragma unroll 1
-                for (int pp = 0; pp < jpv; pp += 4) {
+                for (int pp = 0; 2 * pp < jn; pp += 4) {
                     pair_step(pp);
                     pair_step(pp + 1);
                     pair_step(pp + 2);
@@ -843,7 +843,7 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
                 const float thk = THR(k);
                 float tx = ax[k].x + ax[k].y, ty = ay[k].x + ay[k].y, tz = az[k].x + az[k].y;
                 if (mn[k] < thk) {
-                    const TileSum t = careful_tile(A, ctl, ev_keys, ev_cap, perm, jhi, jlo, sA, sB, jpv, jt,
+                    const TileSum t = careful_tile(A, ctl, ev_keys, ev_cap, perm, jhi, jlo, sA, sB, jn, jt,
                                                    ibase + (ll)k * BLOCK + tid, nx[k].x, ny[k].x, nz[k].x, thk);
                     tx = t.hx;
                     ty = t.hy;
