@@ -65,6 +65,7 @@
 #include "nbg_shared.h"
 
 #define BH_THETA 0.3
+#define BH_FLT_MAX 3.402823466e38f
 #define BH_SOFTENING 1e-4
 #define BH_LEVELS NBG_OCT_LEVELS
 #define BH_BLOCK 256
@@ -85,6 +86,7 @@
 #endif
 #define BH_F_LEAF 1u
 #define BH_F_NAN_CM 2u
+#define BH_F_FAR_OUT 8u /* mixed walk: a one-body leaf past FP32's range */
 #define FULL_MASK 0xffffffffu
 
 /* order-preserving integer image of a double (for atomicMin / atomicMax) */
@@ -1160,11 +1162,18 @@ __global__ void __launch_bounds__(BH_BLOCK) k_bh_prep_mixed(BodyArrays A, DevCtl
             const double o = 2 * t.half[id] / BH_THETA;
             b.w = (float)(o * o);
         }
+        /* A centre of mass past FP32's range (or with an infinite moment or
+         * mass) is at no distance from any body: the acceptance test opens the
+         * node for every one, and a leaf's term is NaN.  Flagged here, so that
+         * the walk neither bounds the distance nor adds the term for bodies
+         * that accepted an ancestor. */
+        unsigned fl = bh_walk_flags(A, t, id);
+        if (!(fabsf(a.x) <= BH_FLT_MAX && fabsf(a.y) <= BH_FLT_MAX && fabsf(a.z) <= BH_FLT_MAX))
+            fl |= (fl & BH_F_LEAF) ? BH_F_FAR_OUT : BH_F_NAN_CM;
         const int slot = t.slot[id];
         t.fa[slot] = a;
         t.fb[slot] = b;
-        t.fc[slot] = make_int4(t.cbase[id], (int)t.ccount[id] | ((int)bh_walk_flags(A, t, id) << 8), t.start[id],
-                               t.end[id]);
+        t.fc[slot] = make_int4(t.cbase[id], (int)t.ccount[id] | ((int)fl << 8), t.start[id], t.end[id]);
     }
 }
 
@@ -1185,8 +1194,8 @@ __device__ __forceinline__ float bh_rsqrt(float x)
     return y;
 }
 
-/* the terms of a leaf at the deepest level holding bodies [s, e) (rare; kept
- * out of the walk's registers) */
+/* the terms of a leaf at the deepest level holding bodies [s, e), or of one
+ * body past FP32's range (rare; kept out of the walk's registers) */
 __device__ __noinline__ int bucket_terms(const BodyArrays &A, const unsigned *vals, int s, int e, unsigned k, float xh,
                                          float yh, float zh, float xl, float yl, float zl, float soft2, double mroot,
                                          float &ax, float &ay, float &az)
@@ -1196,6 +1205,10 @@ __device__ __noinline__ int bucket_terms(const BodyArrays &A, const unsigned *va
         const unsigned j = vals[q];
         const double mj = A.m[j];
         if (j == k || mj == 0) continue;
+        if (e - s == 1) {
+            ax = ay = az = __int_as_float(0x7fc00000);
+            return 1;
+        }
         const float ex = (float)(A.x[j] - (double)xh - (double)xl);
         const float ey = (float)(A.y[j] - (double)yh - (double)yl);
         const float ez = (float)(A.z[j] - (double)zh - (double)zl);
@@ -1481,7 +1494,10 @@ __global__ void __launch_bounds__(BHW_BLOCK, MINB) k_bh_force_mixed(const __grid
                     w.stack[top - 1 - lane] = make_uint2(en.x + (unsigned)(take - x), en.y);
                     w.run[top - 1 - lane] = (unsigned char)(x + rn - take);
                 }
-                top -= __popc(__ballot_sync(FULL_MASK, rn > 0 && x + rn <= take));
+                /* runs of no nodes go too: a body past FP32's range, whose
+                 * distances are NaN, opens accepted nodes, which have no
+                 * children here */
+                top -= __popc(__ballot_sync(FULL_MASK, lane < top && x + rn <= take));
             }
             if (cf >= 32) flush(); /* while those loads are in flight */
             bool isfar = false;
@@ -1496,7 +1512,7 @@ __global__ void __launch_bounds__(BHW_BLOCK, MINB) k_bh_force_mixed(const __grid
                 if (na.w == 0.f) {
                     cls = BHW_DROP; /* nothing with mass below: skipped by every body */
                 } else if (fl & BH_F_LEAF) {
-                    cls = e - s > 1 ? BHW_BUCKET : BHW_ACCEPT;
+                    cls = e - s > 1 || (fl & BH_F_FAR_OUT) ? BHW_BUCKET : BHW_ACCEPT;
                     /* a one-body leaf holds sorted position s: not for itself */
                     if (cls == BHW_ACCEPT && s >= p0 && s < p0 + 32) mask &= ~(1u << (int)(s - p0));
                 } else if (fl & BH_F_NAN_CM) {
@@ -1563,7 +1579,8 @@ __global__ void __launch_bounds__(BHW_BLOCK, MINB) k_bh_force_mixed(const __grid
                 }
                 cm += __popc(mm);
             }
-            /* a leaf at the deepest level holding several bodies */
+            /* a leaf at the deepest level holding several bodies, or one past
+             * FP32's range */
             for (unsigned bm = __ballot_sync(FULL_MASK, cls == BHW_BUCKET && (dealt || wi == 0)); bm; bm &= bm - 1u) {
                 const int src = __ffs(bm) - 1;
                 const unsigned mk = __shfl_sync(FULL_MASK, mask, src);
