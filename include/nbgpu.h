@@ -420,6 +420,9 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
    is left with no bodies (one empty collection, no staged adds); it stays
    usable, and the next load allocates again.  The hook clears itself. */
 #define NBG_OPT_TEST_FAIL_GROWTH 15
+/* test hook for the symmetric kernel's j partials: while 1, they do not
+   grow, as on a device without room for them; 0 (default) turns it off. */
+#define NBG_OPT_TEST_FAIL_JPART 16
 #define NBG_OPT_NEAR_PPM 5   /* mixed: pairs closer than (value * 1e-6) x the i-body's
                                 distance from its tile origin take the near-pair
                                 pass: the exact hi/lo difference, FP64 for a

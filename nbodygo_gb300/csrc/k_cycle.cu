@@ -1837,21 +1837,23 @@ static int scan_grid(ll cap) { return (int)((cap + NBG_SCAN_TILE - 1) / NBG_SCAN
 /* whether one block of each cycle kernel covers the collections */
 static bool small_cycle(const CycleBufs &cb) { return cb.cap <= NBG_SCAN_TILE; }
 
-void nbg_launch_begin(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
+/* direct: the mixed direct sum follows, whose symmetric kernel needs its j
+ * partials; no other force pass reads them, whatever the shape */
+void nbg_launch_begin(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool direct)
 {
     k_begin<<<1, NBG_SCAN_BLOCK, 0, st>>>(ctl, cb.seg, cb.slots, cb.work_cap, cb.itile > 0 ? cb.itile : NBG_MIX_ITILE,
-                                          cb.part_doubles, nbg_mix_is_sym(cb.mix_variant), cb.jpart_units);
+                                          cb.part_doubles, direct && nbg_mix_is_sym(cb.mix_variant), cb.jpart_units);
 }
 
-void nbg_launch_begin_cycle(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
+void nbg_launch_begin_cycle(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool direct)
 {
     if (small_cycle(cb)) {
         k_begin_small<<<1, NBG_SCAN_BLOCK, 0, st>>>(
             cb.a, ctl, cb.seg, cb.slots, cb.work_cap, cb.itile > 0 ? cb.itile : NBG_MIX_ITILE, cb.part_doubles,
-            nbg_mix_is_sym(cb.mix_variant), cb.jpart_units, cb.blk_sum, cb.blk_off, cb.cap, cb.frag_cap);
+            direct && nbg_mix_is_sym(cb.mix_variant), cb.jpart_units, cb.blk_sum, cb.blk_off, cb.cap, cb.frag_cap);
         return;
     }
-    nbg_launch_begin(cb, ctl, st);
+    nbg_launch_begin(cb, ctl, st, direct);
     k_frag_count<<<scan_grid(cb.cap), NBG_SCAN_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.blk_sum, cb.blk_off, cb.cap,
                                                                cb.frag_cap);
 }

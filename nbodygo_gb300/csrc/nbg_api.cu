@@ -94,6 +94,7 @@ struct nbg_ctx {
     int ev_sort_mode = 0; /* NBG_OPT_EVENT_SORT */
     int ev_radix_auto = 0; /* automatic choice for the next call */
     bool test_fail_growth = false; /* NBG_OPT_TEST_FAIL_GROWTH: the next growth fails */
+    bool test_fail_jpart = false;  /* NBG_OPT_TEST_FAIL_JPART: the j partials do not grow */
     cudaEvent_t win[2] = {nullptr, nullptr}; /* the last two launches in flight */
 };
 
@@ -447,6 +448,15 @@ extern "C" {
 static int select_variant(nbg_ctx *ctx, int v);
 }
 
+static void drop_jpart(nbg_ctx *ctx)
+{
+    if (!ctx->cb.jpart) return;
+    cudaFree(ctx->cb.jpart); /* waits for the device */
+    ctx->cb.jpart = nullptr;
+    ctx->cb.jpart_units = 0;
+    invalidate_graph(ctx);
+}
+
 /* the symmetric mixed kernel's j-partial slots: at least `need` units (with
  * a quarter to spare, as collections grow by fragments and adds) */
 static int ensure_jpart(nbg_ctx *ctx, ll need)
@@ -454,13 +464,11 @@ static int ensure_jpart(nbg_ctx *ctx, ll need)
     if (need <= ctx->cb.jpart_units) return NBG_OK;
     const ll units = need + need / 4 + 16;
     const size_t bytes = (size_t)units * 3 * NBG_MIX_ITILE * sizeof(float);
-    cudaFree(ctx->cb.jpart);
-    ctx->cb.jpart = nullptr;
-    ctx->cb.jpart_units = 0;
+    drop_jpart(ctx);
     /* the slots grow with the square of the body count (13 GB at 2^20
      * bodies): past half of the free device memory the shape is refused */
     size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b / 2)
+    if (ctx->test_fail_jpart || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > free_b / 2))
         return fail(ctx, NBG_E_CUDA, "the symmetric kernel's j partials would take over half of the free device memory");
     CK(cudaMalloc((void **)&ctx->cb.jpart, bytes));
     ctx->cb.jpart_units = units;
@@ -1013,6 +1021,7 @@ int nbg_set_collections(nbg_ctx *ctx, int64_t nsims, const int64_t *counts, cons
     if (!ctx->shape_given) {
         const int v = nbg_default_shape((int)nsims, (const ll *)counts, ctx->device_bytes);
         if (v != ctx->cb.mix_variant && (rc = select_variant(ctx, v)) != NBG_OK) return rc;
+        if (!nbg_mix_is_sym(v)) drop_jpart(ctx);
     }
     k_set_loaded<<<1, 1, 0, ctx->st>>>(ctx->ctl, n);
     CK(cudaGetLastError());
@@ -1558,12 +1567,13 @@ static void launch_cycle(nbg_ctx *ctx, int precision, long ev_base)
     const CycleBufs &cb = ctx->cb;
     cudaStream_t st = ctx->st;
     if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base), st);
-    nbg_launch_begin_cycle(cb, ctx->ctl, st);
+    const bool mixed = precision == NBG_PRECISION_MIXED;
+    nbg_launch_begin_cycle(cb, ctx->ctl, st, !cb.bh && mixed);
     if (cb.bh) {
         if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 1), st);
-        nbg_launch_bh(cb, ctx->ctl, st, precision == NBG_PRECISION_MIXED);
+        nbg_launch_bh(cb, ctx->ctl, st, mixed);
         if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 2), st);
-    } else if (precision == NBG_PRECISION_MIXED) {
+    } else if (mixed) {
         nbg_launch_mixed_prep(cb, ctx->ctl, st);
         if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 1), st);
         nbg_launch_mixed_pair(cb, ctx->ctl, st);
@@ -1575,12 +1585,11 @@ static void launch_cycle(nbg_ctx *ctx, int precision, long ev_base)
         if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 2), st);
     }
     /* the mixed direct path keeps its Hilbert order through compaction */
-    nbg_launch_after_pair(cb, ctx->ctl, st, !cb.bh && precision == NBG_PRECISION_MIXED);
+    nbg_launch_after_pair(cb, ctx->ctl, st, !cb.bh && mixed);
     if (ev_base >= 0) cudaEventRecord(get_event(ctx, (size_t)ev_base + 3), st);
     /* the cycle's own, and the force pass: the plain pair kernel, or what
      * the mixed form and Barnes-Hut count (the sort's launches return at once
      * in cycles that keep the order) */
-    const bool mixed = precision == NBG_PRECISION_MIXED;
     ctx->launches_per_cycle = nbg_cycle_launches(cb, !cb.bh && mixed) +
                               (cb.ev_radix ? nbg_event_radix_launches(cb) : 0) +
                               (cb.bh ? nbg_bh_launches(cb, mixed) : mixed ? nbg_mixed_launches(cb) : 1) + (cb.ring_head ? 1 : 0);
@@ -1802,30 +1811,23 @@ int nbg_cancel(nbg_ctx *ctx)
     return NBG_OK;
 }
 
-int nbg_force_pass(nbg_ctx *ctx)
+/* One force pass of the context's form (nbg_force_pass), or of the mixed
+ * direct sum whatever the form (nbg_autotune), with the buffers it needs. */
+static int force_pass(nbg_ctx *ctx, bool direct)
 {
-    NvtxRange nvtx("nbg_force_pass");
-    if (!ctx) return NBG_E_ARG;
-    if (ctx->cb.seg.nsims < 1) return fail(ctx, NBG_E_STATE, "no collection is loaded (a segment allocation failed)");
-    CK(cudaSetDevice(ctx->device));
-    {
-        /* the octree's buffers exist (a failed allocation leaves none) */
-        int rc;
-        if (ctx->cb.bh && (rc = ensure_bh(ctx, 0)) != NBG_OK) return rc;
-    }
     for (int attempt = 0;; attempt++) {
         int z = 0;
         CK(cudaMemcpyAsync(&ctx->ctl->error, &z, sizeof z, cudaMemcpyHostToDevice, ctx->st));
         /* a retry follows a buffer k_begin found short (partial-sum or
          * j-partial slots) or the octree's (Barnes-Hut, which keeps no spatial
          * order): no kernel after k_begin ran, so the order stands */
-        nbg_launch_begin(ctx->cb, ctx->ctl, ctx->st);
-        if (ctx->cb.bh) {
-            nbg_launch_bh(ctx->cb, ctx->ctl, ctx->st, ctx->precision == NBG_PRECISION_MIXED);
-        } else if (ctx->precision == NBG_PRECISION_MIXED) {
+        nbg_launch_begin(ctx->cb, ctx->ctl, ctx->st, direct);
+        if (direct) {
             nbg_launch_mixed_prep(ctx->cb, ctx->ctl, ctx->st);
             nbg_launch_mixed_pair(ctx->cb, ctx->ctl, ctx->st);
             nbg_launch_mixed_out(ctx->cb, ctx->ctl, ctx->st);
+        } else if (ctx->cb.bh) {
+            nbg_launch_bh(ctx->cb, ctx->ctl, ctx->st, ctx->precision == NBG_PRECISION_MIXED);
         } else {
             nbg_launch_pair_fp64(ctx->cb, ctx->ctl, ctx->st);
         }
@@ -1847,6 +1849,17 @@ int nbg_force_pass(nbg_ctx *ctx)
     }
 }
 
+int nbg_force_pass(nbg_ctx *ctx)
+{
+    NvtxRange nvtx("nbg_force_pass");
+    if (!ctx) return NBG_E_ARG;
+    if (ctx->cb.seg.nsims < 1) return fail(ctx, NBG_E_STATE, "no collection is loaded (a segment allocation failed)");
+    CK(cudaSetDevice(ctx->device));
+    /* the octree's buffers exist (a failed allocation leaves none) */
+    const int rc = ctx->cb.bh ? ensure_bh(ctx, 0) : NBG_OK;
+    return rc != NBG_OK ? rc : force_pass(ctx, !ctx->cb.bh && ctx->precision == NBG_PRECISION_MIXED);
+}
+
 static int select_variant(nbg_ctx *ctx, int v)
 {
     if (v < 0 || v >= NBG_MIX_VARIANTS) return fail(ctx, NBG_E_ARG, "unknown kernel shape");
@@ -1865,7 +1878,7 @@ static int time_mixed_pair(nbg_ctx *ctx, float *ms)
     cudaEvent_t e0 = get_event(ctx, 0), e1 = get_event(ctx, 1);
     int z = 0;
     CK(cudaMemcpyAsync(&ctx->ctl->error, &z, sizeof z, cudaMemcpyHostToDevice, ctx->st));
-    nbg_launch_begin(ctx->cb, ctx->ctl, ctx->st);
+    nbg_launch_begin(ctx->cb, ctx->ctl, ctx->st, true);
     nbg_launch_mixed_prep(ctx->cb, ctx->ctl, ctx->st);
     CK(cudaEventRecord(e0, ctx->st));
     nbg_launch_mixed_pair(ctx->cb, ctx->ctl, ctx->st);
@@ -1928,7 +1941,7 @@ int nbg_autotune(nbg_ctx *ctx, const char *cache_path, int *variant, double *bes
             if ((rc = select_variant(ctx, v)) != NBG_OK) return rc;
             /* one untimed force pass grows the buffers this shape needs; a
              * symmetric shape whose j partials do not fit is passed over */
-            if ((rc = nbg_force_pass(ctx)) != NBG_OK) {
+            if ((rc = force_pass(ctx, true)) != NBG_OK) {
                 if (nbg_mix_is_sym(v) && rc == NBG_E_CUDA) {
                     cudaGetLastError();
                     continue;
@@ -1958,14 +1971,7 @@ int nbg_autotune(nbg_ctx *ctx, const char *cache_path, int *variant, double *bes
     }
     if ((rc = select_variant(ctx, best)) != NBG_OK) return rc;
     ctx->shape_given = 1;
-    if (!nbg_mix_is_sym(best) && ctx->cb.jpart) {
-        /* a one-sided shape won: the symmetric kernel's slots go */
-        CK(cudaStreamSynchronize(ctx->st));
-        cudaFree(ctx->cb.jpart);
-        ctx->cb.jpart = nullptr;
-        ctx->cb.jpart_units = 0;
-        invalidate_graph(ctx);
-    }
+    if (!nbg_mix_is_sym(best)) drop_jpart(ctx);
     if (variant) *variant = best;
     if (best_ms) *best_ms = best_t;
     return NBG_OK;
@@ -2148,6 +2154,10 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value)
     case NBG_OPT_TEST_FAIL_GROWTH:
         if (value < 0 || value > 1) return fail(ctx, NBG_E_ARG, "growth-failure hook must be 0 or 1");
         ctx->test_fail_growth = value != 0;
+        return NBG_OK;
+    case NBG_OPT_TEST_FAIL_JPART:
+        if (value < 0 || value > 1) return fail(ctx, NBG_E_ARG, "j-partial failure hook must be 0 or 1");
+        ctx->test_fail_jpart = value != 0;
         return NBG_OK;
     case NBG_OPT_STEP_DEADLINE_MS:
         if (value < 0 || value > ((ll)1 << 40)) return fail(ctx, NBG_E_ARG, "deadline must be 0..2^40 ms");

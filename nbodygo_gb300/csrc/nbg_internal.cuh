@@ -493,9 +493,9 @@ void nbg_launch_bh(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool mixed
 int nbg_bh_launches(const CycleBufs &cb, bool mixed); /* kernels nbg_launch_bh launches */
 
 /* k_cycle.cu (compiled with --fmad=false) */
-void nbg_launch_begin(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
+void nbg_launch_begin(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool direct);
 /* the start of a whole cycle: begin, and the fragments it emits */
-void nbg_launch_begin_cycle(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
+void nbg_launch_begin_cycle(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool direct);
 int nbg_cycle_launches(const CycleBufs &cb, bool carry_order);
 void nbg_launch_pair_fp64(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st);
 void nbg_launch_after_pair(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st, bool carry_order);

@@ -1,0 +1,57 @@
+"""The symmetric kernel's j partials: asked for by the mixed direct sum alone,
+whatever shape a context of another form has, and given back when the default
+shape of a load is one-sided.  The failure hook stands in for a device without
+room for them."""
+import pytest
+
+from nbodygo_gb300 import _abi as A
+from nbodygo_gb300 import workloads as W
+from nbodygo_gb300.api import NbgError, Simulation
+
+pytestmark = pytest.mark.gpu
+
+
+def free_bytes():
+    torch = pytest.importorskip("torch")
+    return torch.cuda.mem_get_info(0)[0]
+
+
+@pytest.mark.parametrize("n", [3000, 6000])
+@pytest.mark.parametrize("prec,bh", [("fp64", 0), ("fp64", 1), ("mixed", 1), ("mixed", 0)])
+def test_only_the_direct_sum_asks(prec, bh, n):
+    with Simulation(prec, capacity=n) as s:
+        s.set_option(A.OPT_BARNES_HUT, bh)
+        s.set_option(A.OPT_MIX_SHAPE, A.MIX_SYM)
+        s.set_option(A.OPT_TEST_FAIL_JPART, 1)
+        s.set_bodies(W.plummer(n=n, seed=1))
+        if prec == "mixed" and not bh:
+            for call in (s.force_pass, lambda: s.step(1e-3, 1.0, 1)):
+                with pytest.raises(NbgError):
+                    call()
+            s.set_option(A.OPT_TEST_FAIL_JPART, 0)
+        s.force_pass()
+        assert s.step(1e-3, 1.0, 2)["steps_done"] == 2
+
+
+def test_an_octree_context_takes_no_memory_for_them():
+    b = W.uniform_ball(200000)  # 76,636 block pairs: 589 MB with the quarter to spare
+    with Simulation("mixed", capacity=200001) as s:
+        s.set_option(A.OPT_BARNES_HUT, 1)
+        s.set_bodies(b)
+        before = free_bytes()
+        s.step(1e-5, 1.0, 1)
+        assert before - free_bytes() < 300 << 20
+
+
+def test_a_one_sided_default_gives_them_back():
+    with Simulation("mixed", capacity=98305) as s:
+        s.set_bodies(W.uniform_ball(98304))  # 18,528 block pairs: 142 MB
+        before = free_bytes()
+        s.step(1e-5, 1.0, 1)
+        held = before - free_bytes()
+        assert held > 100 << 20
+        s.set_bodies(W.uniform_ball(3000))
+        assert before - free_bytes() < held - (100 << 20)
+        s.step(1e-5, 1.0, 1)
+        s.set_bodies(W.uniform_ball(98304))
+        assert s.step(1e-5, 1.0, 2)["steps_done"] == 2
