@@ -1812,8 +1812,10 @@ int nbg_cancel(nbg_ctx *ctx)
 }
 
 /* One force pass of the context's form (nbg_force_pass), or of the mixed
- * direct sum whatever the form (nbg_autotune), with the buffers it needs. */
-static int force_pass(nbg_ctx *ctx, bool direct)
+ * direct sum whatever the form (nbg_autotune), with the buffers it needs.
+ * keep_shape: j partials that do not fit are an error, also for a shape that
+ * was not asked for. */
+static int force_pass(nbg_ctx *ctx, bool direct, bool keep_shape)
 {
     for (int attempt = 0;; attempt++) {
         int z = 0;
@@ -1840,6 +1842,7 @@ static int force_pass(nbg_ctx *ctx, bool direct)
             /* a buffer of the force pass was short: grow it, run again */
             rc = h->error_what == 4 ? ensure_part(ctx, h->error_need)
                  : h->error_what == 5 ? ensure_bh(ctx, h->error_need)
+                 : keep_shape         ? ensure_jpart(ctx, h->error_need)
                                       : grow_jpart(ctx, h->error_need);
             if (rc != NBG_OK) return rc;
             continue;
@@ -1857,7 +1860,7 @@ int nbg_force_pass(nbg_ctx *ctx)
     CK(cudaSetDevice(ctx->device));
     /* the octree's buffers exist (a failed allocation leaves none) */
     const int rc = ctx->cb.bh ? ensure_bh(ctx, 0) : NBG_OK;
-    return rc != NBG_OK ? rc : force_pass(ctx, !ctx->cb.bh && ctx->precision == NBG_PRECISION_MIXED);
+    return rc != NBG_OK ? rc : force_pass(ctx, !ctx->cb.bh && ctx->precision == NBG_PRECISION_MIXED, false);
 }
 
 static int select_variant(nbg_ctx *ctx, int v)
@@ -1941,7 +1944,7 @@ int nbg_autotune(nbg_ctx *ctx, const char *cache_path, int *variant, double *bes
             if ((rc = select_variant(ctx, v)) != NBG_OK) return rc;
             /* one untimed force pass grows the buffers this shape needs; a
              * symmetric shape whose j partials do not fit is passed over */
-            if ((rc = force_pass(ctx, true)) != NBG_OK) {
+            if ((rc = force_pass(ctx, true, true)) != NBG_OK) {
                 if (nbg_mix_is_sym(v) && rc == NBG_E_CUDA) {
                     cudaGetLastError();
                     continue;

@@ -55,3 +55,19 @@ def test_a_one_sided_default_gives_them_back():
         s.step(1e-5, 1.0, 1)
         s.set_bodies(W.uniform_ball(98304))
         assert s.step(1e-5, 1.0, 2)["steps_done"] == 2
+
+
+@pytest.mark.parametrize("n", [45000, 65536, 81920])
+def test_autotune_passes_over_a_shape_without_room(n, tmp_path):
+    """Sizes where the one-sided shape that would run in a symmetric one's
+    place is among the fastest, so a time recorded under the wrong name is
+    chosen in most of the tries."""
+    for k in range(4):
+        cache = str(tmp_path / f"cache{k}")
+        with Simulation("mixed", capacity=n) as s:
+            s.set_option(A.OPT_TEST_FAIL_JPART, 1)
+            s.set_bodies(W.plummer(n=n, seed=1))
+            shape = s.autotune(cache)[0]
+            assert shape not in (A.MIX_SYM, A.MIX_SYM + 1)
+            assert int(open(cache).read().split()[1]) == shape
+            assert s.step(1e-5, 1.0, 2)["steps_done"] == 2
