@@ -245,8 +245,10 @@ int nbg_get_body_in(nbg_ctx *ctx, int64_t sim, int64_t id, nbg_soa *host, int32_
  * nbg_save_state: *size receives the snapshot's bytes; with buf NULL that is
  * all it does (a size query).  A cap below the size returns NBG_E_OVERFLOW.
  * nbg_load_state replaces the context's bodies, collections, staged adds,
- * counters and options with the snapshot's.  The layout is described in
- * nbg_api.cu; values are in the machine's byte order.
+ * counters and options with the snapshot's.  The kernel shape stays the
+ * snapshot's: where a symmetric one's j partials do not fit, the next cycle
+ * fails with NBG_E_CUDA (NBG_OPT_MIX_SHAPE sets another).  The layout is
+ * described in nbg_api.cu; values are in the machine's byte order.
  */
 int nbg_save_state(nbg_ctx *ctx, void *buf, int64_t cap, int64_t *size);
 int nbg_load_state(nbg_ctx *ctx, const void *buf, int64_t size);

@@ -67,7 +67,7 @@ struct nbg_ctx {
     /* collection of each staged add, in the order of cb.adds: grouped by
      * collection, arrival order within one (the order k_append_adds reads) */
     std::vector<int> add_sim;
-    int shape_given = 0; /* the mixed kernel's shape was set or tuned (1), restored from a snapshot (2) */
+    bool shape_given = false; /* the mixed kernel's shape was set, tuned or restored from a snapshot */
     unsigned long long device_bytes = 0;
     bool timing = false;
     nbg_timing tacc{};
@@ -476,12 +476,13 @@ static int ensure_jpart(nbg_ctx *ctx, ll need)
     return NBG_OK;
 }
 
-/* the same for a running cycle: a shape that was not asked for gives way to
- * the one-sided kernel where its j partials do not fit */
+/* the same for a running cycle: a shape that the rule chose gives way to
+ * the one-sided kernel where its j partials do not fit.  One that was set, tuned
+ * or restored does not: a resumed run has the results it would have had. */
 static int grow_jpart(nbg_ctx *ctx, ll need)
 {
     const int rc = ensure_jpart(ctx, need);
-    if (rc == NBG_OK || ctx->shape_given == 1) return rc;
+    if (rc == NBG_OK || ctx->shape_given) return rc;
     cudaGetLastError();
     return select_variant(ctx, NBG_MIX_ONE_SIDED);
 }
@@ -1510,7 +1511,7 @@ int nbg_load_state(nbg_ctx *ctx, const void *buf, int64_t size)
     ctx->precision = H.precision;
     if ((rc = nbg_set_option(ctx, NBG_OPT_BARNES_HUT, H.barnes_hut)) != NBG_OK) return rc;
     if (H.mix_variant != ctx->cb.mix_variant && (rc = select_variant(ctx, H.mix_variant)) != NBG_OK) return rc;
-    ctx->shape_given = 2;
+    ctx->shape_given = true;
     ctx->pending_adds = 0;
     ctx->add_sim.clear();
     if ((rc = ensure_cap(ctx, H.n + H.pending_adds + 1, 0)) != NBG_OK) return rc;
@@ -1973,7 +1974,7 @@ int nbg_autotune(nbg_ctx *ctx, const char *cache_path, int *variant, double *bes
         }
     }
     if ((rc = select_variant(ctx, best)) != NBG_OK) return rc;
-    ctx->shape_given = 1;
+    ctx->shape_given = true;
     if (!nbg_mix_is_sym(best)) drop_jpart(ctx);
     if (variant) *variant = best;
     if (best_ms) *best_ms = best_t;
@@ -2119,7 +2120,7 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value)
         return NBG_OK;
     case NBG_OPT_MIX_SHAPE:
         if (value < 0 || value >= NBG_MIX_VARIANTS) return fail(ctx, NBG_E_ARG, "unknown kernel shape");
-        ctx->shape_given = 1;
+        ctx->shape_given = true;
         return select_variant(ctx, (int)value);
     case NBG_OPT_BH_SHAPE:
         if (value < 0 || value > 2) return fail(ctx, NBG_E_ARG, "Barnes-Hut walk shape must be 0..2");

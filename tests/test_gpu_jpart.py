@@ -2,6 +2,7 @@
 whatever shape a context of another form has, and given back when the default
 shape of a load is one-sided.  The failure hook stands in for a device without
 room for them."""
+import numpy as np
 import pytest
 
 from nbodygo_gb300 import _abi as A
@@ -71,3 +72,29 @@ def test_autotune_passes_over_a_shape_without_room(n, tmp_path):
             assert shape not in (A.MIX_SYM, A.MIX_SYM + 1)
             assert int(open(cache).read().split()[1]) == shape
             assert s.step(1e-5, 1.0, 2)["steps_done"] == 2
+
+
+def test_a_restored_shape_is_kept_or_refused():
+    """A resumed run continues bit for bit or not at all; a shape that the
+    rule chose gives way."""
+    b = W.uniform_ball(98304)
+    with Simulation("mixed", seed=2) as s, Simulation("mixed") as t:
+        s.set_bodies(b)
+        s.step(1e-5, 1.0, 1)
+        snap = s.save_state()
+        s.step(1e-5, 1.0, 2)
+        t.set_option(A.OPT_TEST_FAIL_JPART, 1)
+        t.load_state(snap)
+        for call in (t.force_pass, lambda: t.step(1e-5, 1.0, 2)):
+            with pytest.raises(NbgError):
+                call()
+        t.load_state(snap)
+        t.set_option(A.OPT_TEST_FAIL_JPART, 0)
+        t.step(1e-5, 1.0, 2)
+        want, got = s.state(), t.state()
+        for f in ("x", "vx", "fy"):
+            assert np.array_equal(got[f], want[f]), f
+    with Simulation("mixed", seed=2) as s:
+        s.set_option(A.OPT_TEST_FAIL_JPART, 1)
+        s.set_bodies(b)
+        assert s.step(1e-5, 1.0, 2)["steps_done"] == 2
