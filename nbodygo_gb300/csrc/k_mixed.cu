@@ -362,11 +362,13 @@ __device__ __forceinline__ float touch_distance(float amax, float r, float R, fl
 /* the near-pair threshold on r^2 of a body with largest re-centred coordinate
  * amax and radius r (or of several, given the largest of each) against bodies
  * of radius at most R; t is its threshold against r_max, which it never
- * exceeds */
+ * exceeds.  Above zero, so that a body's own pair is near: for a body without
+ * a radius on its tile's origin the square underflows in a system smaller than
+ * 6e-10. */
 __device__ __forceinline__ float near_threshold(float amax, float r, float R, float xmax, float kappa, float t)
 {
     const float b = fmaxf(touch_distance(amax, r, R, xmax), kappa * amax * (1.0f + 0x1p-17f));
-    return fminf(t, b * b * (1.0f + 0x1p-20f));
+    return fminf(t, fmaxf(b * b * (1.0f + 0x1p-20f), 0x1p-126f));
 }
 
 __global__ void __launch_bounds__(TILES_BLOCK) k_mix_reach(DevCtl *ctl, SimSegs seg, const float4 *__restrict__ jlo,

@@ -1,0 +1,38 @@
+"""The ends of the near-pair thresholds' range, formed in FP32 against the other
+block's (k_pair_sym) or the tiles' in reach (k_mix_reach) largest radius."""
+import numpy as np
+import pytest
+
+from nbodygo_gb300 import _abi as A
+from nbodygo_gb300 import workloads as W
+from nbodygo_gb300.api import Simulation
+
+from helpers import assert_events_identical, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def run(prec, b, shape, capacity=0, sims=None):
+    with Simulation(prec, capacity=capacity, seed=3) as s:
+        if prec == "mixed":
+            s.set_option(A.OPT_MIX_SHAPE, shape)
+        s.set_collections([b] + (sims or []))
+        f = np.array(s.force_pass())[:, :len(b["x"])]
+        s.step(0.0, 1.0, 1)
+        return f, s.events()
+
+
+@pytest.mark.parametrize("n,shape,capacity", [(513, A.MIX_SYM, 0), (1025, A.MIX_SYM + 1, 0), (257, 2, 40000),
+                                              (513, 0, 40000)])
+def test_a_tiny_system_of_points(n, shape, capacity):
+    """A ball of radius 1e-10 without radii whose last tile is one body on its
+    own origin, at a position that FP32 holds exactly (no low part).  Beside
+    it, for the one-sided shapes, a collection with a larger radius."""
+    b = W.uniform_ball(n, seed=7, R=1e-10, radius=0.0)
+    for c in "xyz":
+        b[c][:] = b[c].astype(np.float32)
+    other = W.uniform_ball(n, seed=8, R=1e-10, radius=1e-20)
+    sims = [other] if capacity else None
+    f, _ = run("mixed", b, shape, capacity, sims)
+    g, _ = run("fp64", b, shape, 0, sims)
+    assert np.all(np.isfinite(f)) and rel_l2(f, g) <= 1e-6
