@@ -1237,7 +1237,9 @@ k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const
                 const float4 cj = tile_c[seg.mtile_off[sim] + bb];
                 const float ex = cj.x - c.x, ey = cj.y - c.y, ez = cj.z - c.z;
                 const float gap = sqrtf(ex * ex + ey * ey + ez * ez) * (1.0f - 0x1p-18f) - c.w - cj.w;
-                far = gap > 0.f && gap * gap > near_threshold(ra.x, ra.y, R, xmax, kappa, 3.0e38f) * (1.0f + 0x1p-10f);
+                /* no other bound: past FP32's range neither is far */
+                const float reach2 = near_threshold(ra.x, ra.y, R, xmax, kappa, __int_as_float(0x7f800000));
+                far = gap > 0.f && gap * gap > reach2 * (1.0f + 0x1p-10f);
             }
             float thr[SYM_KI];
             if (!far) {

@@ -36,3 +36,17 @@ def test_a_tiny_system_of_points(n, shape, capacity):
     f, _ = run("mixed", b, shape, capacity, sims)
     g, _ = run("fp64", b, shape, 0, sims)
     assert np.all(np.isfinite(f)) and rel_l2(f, g) <= 1e-6
+
+
+@pytest.mark.parametrize("shape", [0, 2, A.MIX_SYM, A.MIX_SYM + 1])
+@pytest.mark.parametrize("gap", [1.75e19, 1.8e19])
+def test_blocks_at_the_end_of_fp32s_range(shape, gap):
+    """Two blocks so far apart that the squared distance is just below FP32's
+    largest value, and two bodies whose radii reach from one to the other."""
+    b = W.uniform_ball(1024, seed=9, R=1e6, radius=1.0, behavior=A.ELASTIC)
+    b["x"][512:] += gap
+    b["radius"][100], b["radius"][700] = 1.0e19, 0.95e19
+    _, ev = run("mixed", b, shape)
+    _, want = run("fp64", b, shape)
+    assert len(want) > 0
+    assert_events_identical(ev, want)
