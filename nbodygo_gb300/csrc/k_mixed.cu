@@ -1053,12 +1053,18 @@ __device__ __forceinline__ float sym_r2(float xj, float yj, float zj, float nxi,
 
 /* A warp's near pairs of one unit, as (own, other) indices in two blocks, with
  * each own body's pairs in a run.  drain() evaluates 32 at a time, one a lane
- * (candidate_pair: FP64), and hands each own body's sum over the batch, in
- * list order, to add(own, x, y, z).  The whole warp calls every member. */
+ * (candidate_pair: FP64), and hands each own body's sum over its run to
+ * add(own, x, y, z), once: a run that goes on past a batch is carried in FP64
+ * to the next, or to finish().  The whole warp calls every member. */
 #define SYM_LIST 64
+#define SYM_NONE 0xffffu
 struct SymNear {
     unsigned *list; /* shared: own << 16 | other */
-    int cnt;
+    int cnt = 0;
+    unsigned open = SYM_NONE; /* the last run's body, and its sum so far (the same in every lane) */
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+
+    __device__ __forceinline__ explicit SymNear(unsigned *l) : list(l) {}
 
     template <class ADD>
     __device__ __forceinline__ void drain(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
@@ -1093,9 +1099,34 @@ struct SymNear {
                     sz += uz;
                 }
             }
-            if (first) add((int)own, sx, sy, sz);
+            const unsigned own_first = __shfl_sync(FULL_MASK, own, 0);
+            if (lane == 0 && open != SYM_NONE) {
+                if (own_first == open) {
+                    sx = ox + sx;
+                    sy = oy + sy;
+                    sz = oz + sz;
+                } else {
+                    add((int)open, ox, oy, oz);
+                }
+            }
+            const int in_batch = cnt - b < 32 ? cnt - b : 32;
+            const int last = __ffs(__shfl_sync(FULL_MASK, run, in_batch - 1)) - 1; /* the last run's first lane */
+            if (first && lane != last) add((int)own, sx, sy, sz);
+            open = __shfl_sync(FULL_MASK, own, last);
+            ox = __shfl_sync(FULL_MASK, sx, last);
+            oy = __shfl_sync(FULL_MASK, sy, last);
+            oz = __shfl_sync(FULL_MASK, sz, last);
         }
         cnt = 0;
+        __syncwarp();
+    }
+
+    template <class ADD>
+    __device__ __forceinline__ void finish(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap,
+                                           const unsigned *__restrict__ perm, ll own0, ll oth0, ADD add)
+    {
+        drain(A, ctl, ev_keys, ev_cap, perm, own0, oth0, add);
+        if ((threadIdx.x & 31) == 0 && open != SYM_NONE) add((int)open, ox, oy, oz);
         __syncwarp();
     }
 
@@ -1347,7 +1378,7 @@ k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const
             /* exact pass, i side: the warp looks over block b for each of its
              * flagged i-bodies in turn, 32 j at a time */
             if (!far && __any_sync(FULL_MASK, nearmask != 0)) {
-                SymNear near = {s_list[w], 0};
+                SymNear near(s_list[w]);
                 auto add = [&](int own, double ux, double uy, double uz) {
                     fold64(sfold[0][own], sfold[1][own], ux);
                     fold64(sfold[2][own], sfold[3][own], uy);
@@ -1376,7 +1407,7 @@ k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const
                         }
                     }
                 }
-                near.drain(A, ctl, ev_keys, ev_cap, perm, ibase, jb, add);
+                near.finish(A, ctl, ev_keys, ev_cap, perm, ibase, jb, add);
             }
             if (diag) continue; /* a diagonal unit has no j slot */
             __syncthreads(); /* jacc and jnear complete */
@@ -1400,7 +1431,7 @@ k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const
             /* exact pass, j side: for each j that met a near pair, block a */
             __syncthreads(); /* the sums are written */
             {
-                SymNear near = {s_list[w], 0};
+                SymNear near(s_list[w]);
                 auto add = [&](int own, double ux, double uy, double uz) {
                     jo[own] = (float)((double)jo[own] + ux);
                     jo[SYM_B + own] = (float)((double)jo[SYM_B + own] + uy);
@@ -1427,7 +1458,7 @@ k_pair_sym(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, const
                         }
                     }
                 }
-                near.drain(A, ctl, ev_keys, ev_cap, perm, jb, ibase, add);
+                near.finish(A, ctl, ev_keys, ev_cap, perm, jb, ibase, add);
             }
         }
         /* this chunk's share of row a's i sums: slot g + chunk */
