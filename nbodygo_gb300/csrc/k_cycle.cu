@@ -89,6 +89,7 @@ __device__ static void begin_cycle(DevCtl *ctl, const SimSegs &seg, int slots, i
         seg.keep[s] = 0;
         seg.frag[s] = 0;
         seg.xmax_bits[s] = 0;
+        seg.heavy[s] = 0;
     }
     block_scan_array(ns, [&](int s) { return (off[s + 1] - off[s] + 63) / 64; }, seg.tile_off);
     const ll mtiles = block_scan_array(

@@ -71,7 +71,10 @@ __device__ __forceinline__ bool is_special(double x, double y, double z, double 
     return !(fabs(x) <= NBG_DBL_MAX && fabs(y) <= NBG_DBL_MAX && fabs(z) <= NBG_DBL_MAX) || r != r;
 }
 
-/* ---- per-cycle reductions: r_max, |x|_max, m_scale ------------------------ */
+/* ---- per-cycle reductions: r_max, |x|_max, m_scale, the heaviest bodies ---- */
+
+/* |m| rounded to FP32, for comparison; a NaN counts as none */
+__device__ __forceinline__ unsigned mass_bits(double m) { return m == m ? __float_as_uint(fabsf((float)m)) : 0u; }
 
 __global__ void k_mix_reduce(BodyArrays A, DevCtl *ctl, SimSegs seg)
 {
@@ -80,11 +83,13 @@ __global__ void k_mix_reduce(BodyArrays A, DevCtl *ctl, SimSegs seg)
     const ll n = ctl->n;
     float rmax = 0.f, xmax = 0.f;
     double mmax = 0.0;
+    ull heavy = 0;
     const ll stride = (ll)gridDim.x * blockDim.x;
     /* warp-uniform trip count: every lane takes part in the per-sim reduction */
     for (ll base = (ll)blockIdx.x * blockDim.x; base < n; base += stride) {
         const ll k = base + threadIdx.x;
         float xk = 0.f;
+        unsigned mk = 0;
         int sim = -1;
         if (k < n) {
             const double x = A.x[k], y = A.y[k], z = A.z[k], r = A.rad[k];
@@ -92,22 +97,37 @@ __global__ void k_mix_reduce(BodyArrays A, DevCtl *ctl, SimSegs seg)
                 rmax = fmaxf(rmax, (float)fmax(r, 0.0));
                 xk = (float)fmax(fabs(x), fmax(fabs(y), fabs(z)));
                 xmax = fmaxf(xmax, xk);
-                if ((A.flags[k] & NBG_LIVE_MASK) == NBG_F_EXISTS) mmax = fmax(mmax, fabs(A.m[k]));
                 sim = nbg_sim_of(seg.off, seg.nsims, k);
+                if ((A.flags[k] & NBG_LIVE_MASK) == NBG_F_EXISTS) {
+                    mmax = fmax(mmax, fabs(A.m[k]));
+                    if (seg.off[sim + 1] - seg.off[sim] <= NBG_HEAVY_MAX_N) mk = mass_bits(A.m[k]);
+                }
             }
         }
         if (seg.nsims > 1) {
             const unsigned peers = __match_any_sync(FULL_MASK, sim);
             const unsigned mx = __reduce_max_sync(peers, __float_as_uint(xk * (1.0f + 0x1p-20f)));
-            if (sim >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicMax(&seg.xmax_bits[sim], mx);
+            const bool first = sim >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1;
+            if (first) atomicMax(&seg.xmax_bits[sim], mx);
+            if (__any_sync(FULL_MASK, mk != 0)) {
+                const unsigned mm = __reduce_max_sync(peers, mk);
+                const unsigned id = __reduce_max_sync(peers, mk == mm ? ~(unsigned)k : 0u);
+                if (first && mm) atomicMax((unsigned long long *)&seg.heavy[sim], nbg_heavy_key(mm, ~id));
+            }
+        } else if (mk) {
+            const ull key = nbg_heavy_key(mk, (unsigned)k);
+            heavy = key > heavy ? key : heavy;
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
         rmax = fmaxf(rmax, __shfl_xor_sync(FULL_MASK, rmax, o));
         xmax = fmaxf(xmax, __shfl_xor_sync(FULL_MASK, xmax, o));
         mmax = fmax(mmax, __shfl_xor_sync(FULL_MASK, mmax, o));
+        const ull other = __shfl_xor_sync(FULL_MASK, heavy, o);
+        heavy = other > heavy ? other : heavy;
     }
     if ((threadIdx.x & 31) == 0) {
+        if (heavy) atomicMax((unsigned long long *)&seg.heavy[0], heavy);
         /* rounding up keeps both bounds conservative */
         atomicMax(&ctl->rmax_bits, __float_as_uint(rmax * (1.0f + 0x1p-20f)));
         atomicMax(&ctl->xmax_bits, __float_as_uint(xmax * (1.0f + 0x1p-20f)));
@@ -130,12 +150,17 @@ __device__ __forceinline__ void pack_body(const BodyArrays &A, ll k, double ms, 
     const float xh = (float)x, yh = (float)y, zh = (float)z;
     const float xl = (float)(x - (double)xh), yl = (float)(y - (double)yh), zl = (float)(z - (double)zh);
     const bool live = (A.flags[k] & NBG_LIVE_MASK) == NBG_F_EXISTS;
-    const float m = live ? (float)(A.m[k] / ms) : 0.f;
+    const float m = live ? (float)(A.m[k] / ms) + 0.f : 0.f; /* never -0 */
     h = make_float4(xh, yh, zh, m);
     l = make_float4(xl, yl, zl, (float)r);
 }
 
 __device__ __forceinline__ bool packed_special(const float4 &lo) { return lo.x != lo.x; }
+
+/* packed mass of a collection's heaviest body where k_mix_out adds its pull
+ * (NBG_HEAVY_MAX_N): it pulls nothing in the pair kernel */
+#define HEAVY_MASS (-0.0f)
+__device__ __forceinline__ bool packed_heavy(const float4 &hi) { return __float_as_uint(hi.w) == 0x80000000u; }
 
 /* ---- the pair kernel ----------------------------------------------------- */
 
@@ -151,33 +176,42 @@ __device__ static int detect_event_mixed(unsigned bi, unsigned bj, double ri, do
     return -1;
 }
 
-/* A pair inside the candidate bound (body indices i, j): decide overlap and
- * collision in FP64 with the reference's expressions (no contraction:
- * explicit _rn intrinsics), return the force term if the pair does not
- * overlap (m_scale-normalised acceleration units), record the event. */
-__device__ static void candidate_pair(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap, ll i, ll j,
-                                      double inv_ms, double &tx, double &ty, double &tz)
+/* The force term of a pair (body indices i, j) in FP64, unless the bodies
+ * overlap, which is decided with the reference's expressions (no contraction:
+ * explicit _rn intrinsics); scale times the mass of j, so 1 / m_scale gives
+ * m_scale-normalised acceleration units. */
+__device__ __forceinline__ void exact_term(const BodyArrays &A, ll i, ll j, double scale, double &dist, double &rr,
+                                           double &tx, double &ty, double &tz)
 {
     tx = ty = tz = 0.0;
-    const unsigned fi = A.flags[i], fj = A.flags[j];
     const double xi = A.x[i], yi = A.y[i], zi = A.z[i], ri = A.rad[i];
     const double dx = __dsub_rn(A.x[j], xi);
     const double dy = __dsub_rn(A.y[j], yi);
     const double dz = __dsub_rn(A.z[j], zi);
-    const double dist = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-    const double rj = A.rad[j];
-    const double rr = __dadd_rn(ri, rj);
-    const bool coll_i = (fi & NBG_F_COLLIDED) != 0;
-    const bool live_j = (fj & NBG_LIVE_MASK) == NBG_F_EXISTS;
+    dist = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+    rr = __dadd_rn(ri, A.rad[j]);
+    const bool coll_i = (A.flags[i] & NBG_F_COLLIDED) != 0;
+    const bool live_j = (A.flags[j] & NBG_LIVE_MASK) == NBG_F_EXISTS;
     if (live_j && (coll_i || dist > rr)) {
-        const double w = (A.m[j] * inv_ms) / (dist * dist * dist);
+        const double w = (A.m[j] * scale) / (dist * dist * dist);
         tx = w * dx;
         ty = w * dy;
         tz = w * dz;
     }
+}
+
+/* A pair inside the candidate bound: its exact term, and the event of an
+ * overlap. */
+__device__ static void candidate_pair(const BodyArrays &A, DevCtl *ctl, ull *ev_keys, ll ev_cap, ll i, ll j,
+                                      double inv_ms, double &tx, double &ty, double &tz)
+{
+    double dist, rr;
+    exact_term(A, i, j, inv_ms, dist, rr, tx, ty, tz);
+    const unsigned fi = A.flags[i], fj = A.flags[j];
+    const bool coll_i = (fi & NBG_F_COLLIDED) != 0;
     const bool live_i = (fi & NBG_LIVE_MASK) == NBG_F_EXISTS;
     if (live_i && !coll_i && dist <= rr) {
-        int type = detect_event_mixed(NBG_BEHAVIOR(fi), NBG_BEHAVIOR(fj), ri, rj, dist);
+        int type = detect_event_mixed(NBG_BEHAVIOR(fi), NBG_BEHAVIOR(fj), A.rad[i], A.rad[j], dist);
         if (type >= 0) {
             ll slot = (ll)atomicAdd((unsigned long long *)&ctl->ev_count, 1ull);
             if (slot < ev_cap) ev_keys[slot] = ((ull)i << 32) | ((ull)j << 2) | (ull)type;
@@ -241,7 +275,7 @@ __device__ __forceinline__ double near_kappa_of(const DevCtl *ctl, ll n, int iti
 __global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl *ctl, SimSegs seg,
                                                            const unsigned *__restrict__ perm, float4 *jhi, float4 *jlo,
                                                            float4 *tile_c, float2 *tile_r, float4 *iprep,
-                                                           int2 *tile_rng, int itile)
+                                                           int2 *tile_rng, int itile, int one_sided)
 {
     __shared__ float red[6][TILES_BLOCK / 32];
     __shared__ float4 s_c;
@@ -259,6 +293,7 @@ __global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl 
         const ll t = tile - seg.mtile_off[sim];
         const ll base = s0 + t * itile;
         const ll n = s1 < base + itile ? s1 : base + itile;
+        const ull heavy = one_sided ? seg.heavy[sim] : 0ull;
         float4 h[TILES_ITEMS], l[TILES_ITEMS];
         float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
 #pragma unroll
@@ -266,6 +301,7 @@ __global__ void __launch_bounds__(TILES_BLOCK) k_mix_tiles(BodyArrays A, DevCtl 
             const ll p = base + q * TILES_BLOCK + tid;
             if (p >= n) continue;
             pack_body(A, (ll)perm[p], ms, h[q], l[q]);
+            if (heavy && perm[p] == nbg_heavy_index(heavy)) h[q].w = HEAVY_MASS;
             jhi[p] = h[q];
             jlo[p] = l[q];
             if (packed_special(l[q])) continue;
@@ -444,6 +480,7 @@ __device__ __forceinline__ void near_pair(const BodyArrays &A, DevCtl *ctl, ull 
         if (!(ms > 0.0)) ms = 1.0;
         double qx, qy, qz;
         candidate_pair(A, ctl, ev_keys, ev_cap, (ll)perm[p], (ll)perm[q], 1.0 / ms, qx, qy, qz);
+        if (packed_heavy(hj)) return;
         fold64(t.hx, t.lx, qx);
         fold64(t.hy, t.ly, qy);
         fold64(t.hz, t.lz, qz);
@@ -908,6 +945,32 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
  * beside the pairs took 546 us a cycle there with 24,320 chunks, now 190 us. */
 #define OUT_SLICES 8
 #define OUT_BODIES 32
+
+/* exact_term where heavy_pull does not hold */
+__device__ __noinline__ static double heavy_pull_exact(const BodyArrays &A, ll i, ll j, int c)
+{
+    double dist, rr, tx, ty, tz;
+    exact_term(A, i, j, 1.0, dist, rr, tx, ty, tz);
+    return c == 0 ? tx : c == 1 ? ty : tz;
+}
+
+/* Component c of the heaviest body's (j) pull on body i at (x, y, z) with
+ * radius r, m_j d / |d|^3: FP64, the reciprocal root from the SFU's by one
+ * Newton step (relative error 2^-43), 20 operations of the FP64 pipe where the
+ * exact term's root and division take 60.  Overlaps, and distances that FP32
+ * does not hold, take the exact term. */
+__device__ __forceinline__ double heavy_pull(const BodyArrays &A, ll i, ll j, double x, double y, double z, double r,
+                                             int c)
+{
+    const double dx = A.x[j] - x, dy = A.y[j] - y, dz = A.z[j] - z;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const float q = (float)r2, rr = (float)(r + A.rad[j]);
+    if (!(q > 1e-30f && q < 1e30f && rr >= 0.f && q > rr * rr * (1.0f + 0x1p-10f))) return heavy_pull_exact(A, i, j, c);
+    double v = (double)rsqrt_sfu(q);
+    v = v * (1.5 - 0.5 * r2 * (v * v));
+    return A.m[j] * (v * v * v) * (c == 0 ? dx : c == 1 ? dy : dz);
+}
+
 __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A, DevCtl *ctl, SimSegs seg,
                                                                    const unsigned *perm, const double *part,
                                                                    const int2 *tile_rng, int itile)
@@ -927,6 +990,7 @@ __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A
         const int li = (int)(gr - g * per) * OUT_BODIES + col;
         const int sim = nbg_sim_of(seg.mtile_off, seg.nsims, g);
         const ll s0 = seg.off[sim], n = seg.off[sim + 1];
+        const ull heavy = seg.heavy[sim];
         const ll t = g - seg.mtile_off[sim];
         if (s0 + t * itile + li - col >= n) continue; /* no body in this group (uniform) */
         int2 rng;
@@ -969,10 +1033,13 @@ __global__ void __launch_bounds__(OUT_SLICES *OUT_BODIES) k_mix_out(BodyArrays A
                      * terms NaN */
                     const bool has_nan = x != x || y != y || z != z || r != r;
                     v = has_nan ? 0.0 : nbg_nan();
+                } else if (heavy && nbg_heavy_index(heavy) != (unsigned)i) {
+                    v += NBG_G * A.m[i] * heavy_pull(A, i, (ll)nbg_heavy_index(heavy), x, y, z, r, row);
                 }
                 (row == 0 ? A.fx : row == 1 ? A.fy : A.fz)[i] = v;
             }
         }
+        __syncwarp();
         __syncthreads(); /* red and range are rewritten by the next group */
     }
 }
@@ -1647,7 +1714,8 @@ void nbg_launch_mixed_prep(const CycleBufs &cb, DevCtl *ctl, cudaStream_t st)
     k_mix_tiles<<<(int)tiles, TILES_BLOCK, 0, st>>>(cb.a, ctl, cb.seg, cb.perm, cb.jhi, cb.jlo, cb.tile_c,
                                                     mix_reach(cb) || nbg_mix_is_sym(cb.mix_variant) ? cb.tile_r : nullptr,
                                                     cb.iprep,
-                                                    nbg_mix_is_sym(cb.mix_variant) ? nullptr : cb.tile_rng, itile);
+                                                    nbg_mix_is_sym(cb.mix_variant) ? nullptr : cb.tile_rng, itile,
+                                                    !nbg_mix_is_sym(cb.mix_variant));
     if (mix_reach(cb))
         k_mix_reach<<<(int)tiles, TILES_BLOCK, 0, st>>>(ctl, cb.seg, cb.jlo, cb.tile_c, cb.tile_r, cb.iprep,
                                                         itile);

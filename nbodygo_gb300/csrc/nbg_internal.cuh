@@ -133,6 +133,25 @@ __device__ __forceinline__ void nbg_sort_decide(DevCtl *ctl)
 #define NBG_NEAR_KAPPA_DEFAULT 0.05f
 /* collections of at most this many bodies use twice the near-pair factor */
 #define NBG_NEAR_SMALL_N 2048
+/* In a collection of at most this many bodies the one-sided kernels leave the
+ * heaviest body's pull to k_mix_out, which adds it in FP64.  One body, a star,
+ * may carry nearly all of every other's force, and then the FP32 error of that
+ * one term is the body's, most of it the rounding of the offset from the tile's
+ * origin; in larger collections the tiles are smaller next to the distances.
+ * Force error of disks of 500 / 1,000 / 2,000 / 3,000 bodies around a star, the
+ * star's own left out (L2, mean of 80): 1.48 / 1.84 / 1.95 / 1.76e-7 with the
+ * star in the pair kernel, 1e-14 so (1.28 / 1.35 / 1.54 / 1.55e-7 with tiles of 512
+ * along a Z-order curve; from 4,000 bodies on the present tiles are better).  A
+ * near-pair factor of 0.25 gives 1.3e-7 and costs 30 to 70% of such a cycle; this,
+ * nothing that shows in the cycle of 2,501 Plummer bodies. */
+#define NBG_HEAVY_MAX_N 4096
+/* seg.heavy: |mass| as FP32 bits, then the complement of the index, so that
+ * the largest is the heaviest body, and among equals the first */
+__host__ __device__ __forceinline__ ull nbg_heavy_key(unsigned mass_bits, unsigned index)
+{
+    return mass_bits ? (ull)mass_bits << 32 | (unsigned)~index : 0ull;
+}
+__host__ __device__ __forceinline__ unsigned nbg_heavy_index(ull key) { return ~(unsigned)key; }
 
 /* A collection may hold several independent simulations stored one after
  * another: sim s occupies bodies [off[s], off[s+1]) and bodies of different
@@ -153,11 +172,12 @@ struct SimSegs {
     ll *keep_start;  /* [nsims+1] */
     ll *new_off;     /* [nsims+1] layout after Cycle */
     unsigned *xmax_bits; /* [nsims] mixed: |x| max of sim s (Hilbert grid) */
+    ull *heavy;          /* [nsims] mixed: sim s's heaviest body (NBG_HEAVY_MAX_N), 0 = none */
 };
 
 /* bytes of the SimSegs arrays for nsims sims (one allocation, carved by
- * nbg_seg_carve: 11 ll arrays and 2 32-bit arrays of nsims + 1) */
-#define NBG_SEG_BYTES(ns) ((size_t)((ns) + 1) * 8 * 11 + (size_t)((ns) + 1) * 4 * 2 + 256)
+ * nbg_seg_carve: 12 64-bit arrays and 2 32-bit arrays of nsims + 1) */
+#define NBG_SEG_BYTES(ns) ((size_t)((ns) + 1) * 8 * 12 + (size_t)((ns) + 1) * 4 * 2 + 256)
 
 static inline SimSegs nbg_seg_carve(void *base, int nsims)
 {
@@ -176,7 +196,8 @@ static inline SimSegs nbg_seg_carve(void *base, int nsims)
     s.hadd_start = p + 8 * m;
     s.keep_start = p + 9 * m;
     s.new_off = p + 10 * m;
-    s.xmax_bits = (unsigned *)(p + 11 * m) + m; /* the first 32-bit array is spare */
+    s.heavy = (ull *)(p + 11 * m);
+    s.xmax_bits = (unsigned *)(p + 12 * m) + m; /* the first 32-bit array is spare */
     return s;
 }
 
