@@ -907,16 +907,16 @@ __device__ static __noinline__ double lane_atan2(double y, double x)
 __device__ static __noinline__ double lane_poly(double r, bool c)
 {
     const double z = r * r;
-    double p = c ? -0x1.0ce396db7f853p-70 : 0x1.71b8ef6dcf572p-66;
-    p = (c ? 0x1.e542ba4020225p-62 : -0x1.2f49b46814157p-57) + z * p;
-    p = (c ? -0x1.6827863b97d97p-53 : 0x1.952c77030ad4ap-49) + z * p;
-    p = (c ? 0x1.ae7f3e733b81fp-45 : -0x1.ae7f3e733b81fp-41) + z * p;
-    p = (c ? -0x1.93974a8c07c9dp-37 : 0x1.6124613a86d09p-33) + z * p;
-    p = (c ? 0x1.1eed8eff8d898p-29 : -0x1.ae64567f544e4p-26) + z * p;
-    p = (c ? -0x1.27e4fb7789f5cp-22 : 0x1.71de3a556c734p-19) + z * p;
-    p = (c ? 0x1.a01a01a01a01ap-16 : -0x1.a01a01a01a01ap-13) + z * p;
-    p = (c ? -0x1.6c16c16c16c17p-10 : 0x1.1111111111111p-7) + z * p;
-    p = (c ? 0x1.5555555555555p-5 : -0x1.5555555555555p-3) + z * p;
+    double p = c ? NBG_C11 : NBG_S10;
+    p = (c ? NBG_C10 : NBG_S9) + z * p;
+    p = (c ? NBG_C9 : NBG_S8) + z * p;
+    p = (c ? NBG_C8 : NBG_S7) + z * p;
+    p = (c ? NBG_C7 : NBG_S6) + z * p;
+    p = (c ? NBG_C6 : NBG_S5) + z * p;
+    p = (c ? NBG_C5 : NBG_S4) + z * p;
+    p = (c ? NBG_C4 : NBG_S3) + z * p;
+    p = (c ? NBG_C3 : NBG_S2) + z * p;
+    p = (c ? NBG_C2 : NBG_S1) + z * p;
     const double m = (c ? z : r) * z * p; /* the term that the polynomial makes */
     if (!c) return r + m;
     const double hz = 0.5 * z;

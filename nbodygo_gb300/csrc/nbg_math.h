@@ -75,20 +75,43 @@ NBG_FN double nbg_nan(void)
 NBG_FN int nbg_isinf(double x) { return fabs(x) > NBG_DBL_MAX; }
 NBG_FN int nbg_isfinite(double x) { return fabs(x) <= NBG_DBL_MAX; }
 
+/* Taylor coefficients of sin (S10 of x^21 down to S1 of x^3) and cos (C11 of
+ * x^22 down to C2 of x^4), for the polynomials here and k_cycle.cu's by lane. */
+#define NBG_S10 0x1.71b8ef6dcf572p-66
+#define NBG_S9 -0x1.2f49b46814157p-57
+#define NBG_S8 0x1.952c77030ad4ap-49
+#define NBG_S7 -0x1.ae7f3e733b81fp-41
+#define NBG_S6 0x1.6124613a86d09p-33
+#define NBG_S5 -0x1.ae64567f544e4p-26
+#define NBG_S4 0x1.71de3a556c734p-19
+#define NBG_S3 -0x1.a01a01a01a01ap-13
+#define NBG_S2 0x1.1111111111111p-7
+#define NBG_S1 -0x1.5555555555555p-3
+#define NBG_C11 -0x1.0ce396db7f853p-70
+#define NBG_C10 0x1.e542ba4020225p-62
+#define NBG_C9 -0x1.6827863b97d97p-53
+#define NBG_C8 0x1.ae7f3e733b81fp-45
+#define NBG_C7 -0x1.93974a8c07c9dp-37
+#define NBG_C6 0x1.1eed8eff8d898p-29
+#define NBG_C5 -0x1.27e4fb7789f5cp-22
+#define NBG_C4 0x1.a01a01a01a01ap-16
+#define NBG_C3 -0x1.6c16c16c16c17p-10
+#define NBG_C2 0x1.5555555555555p-5
+
 /* sin(r) for |r| <= ~pi/4: r + r^3 * P(r^2), Taylor coefficients 1/(2k+1)!. */
 NBG_FN double nbg_sin_poly(double r)
 {
     double z = r * r;
-    double p = 0x1.71b8ef6dcf572p-66;
-    p = -0x1.2f49b46814157p-57 + z * p;
-    p = 0x1.952c77030ad4ap-49 + z * p;
-    p = -0x1.ae7f3e733b81fp-41 + z * p;
-    p = 0x1.6124613a86d09p-33 + z * p;
-    p = -0x1.ae64567f544e4p-26 + z * p;
-    p = 0x1.71de3a556c734p-19 + z * p;
-    p = -0x1.a01a01a01a01ap-13 + z * p;
-    p = 0x1.1111111111111p-7 + z * p;
-    p = -0x1.5555555555555p-3 + z * p;
+    double p = NBG_S10;
+    p = NBG_S9 + z * p;
+    p = NBG_S8 + z * p;
+    p = NBG_S7 + z * p;
+    p = NBG_S6 + z * p;
+    p = NBG_S5 + z * p;
+    p = NBG_S4 + z * p;
+    p = NBG_S3 + z * p;
+    p = NBG_S2 + z * p;
+    p = NBG_S1 + z * p;
     return r + (r * z) * p;
 }
 
@@ -96,16 +119,16 @@ NBG_FN double nbg_sin_poly(double r)
 NBG_FN double nbg_cos_poly(double r)
 {
     double z = r * r;
-    double q = -0x1.0ce396db7f853p-70;
-    q = 0x1.e542ba4020225p-62 + z * q;
-    q = -0x1.6827863b97d97p-53 + z * q;
-    q = 0x1.ae7f3e733b81fp-45 + z * q;
-    q = -0x1.93974a8c07c9dp-37 + z * q;
-    q = 0x1.1eed8eff8d898p-29 + z * q;
-    q = -0x1.27e4fb7789f5cp-22 + z * q;
-    q = 0x1.a01a01a01a01ap-16 + z * q;
-    q = -0x1.6c16c16c16c17p-10 + z * q;
-    q = 0x1.5555555555555p-5 + z * q;
+    double q = NBG_C11;
+    q = NBG_C10 + z * q;
+    q = NBG_C9 + z * q;
+    q = NBG_C8 + z * q;
+    q = NBG_C7 + z * q;
+    q = NBG_C6 + z * q;
+    q = NBG_C5 + z * q;
+    q = NBG_C4 + z * q;
+    q = NBG_C3 + z * q;
+    q = NBG_C2 + z * q;
     double hz = 0.5 * z;
     double w = 1.0 - hz;
     return w + (((1.0 - w) - hz) + (z * z) * q);
