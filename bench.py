@@ -98,7 +98,7 @@ def parse():
     ap.add_argument("--chunks", type=int, default=None,
                     help="mixed: most chunks the pair work is cut into (library default 32 per resident CTA)")
     ap.add_argument("--p64-split-max", type=int, default=None,
-                    help="plain FP64: largest capacity for the split pair pass (library default 65536)")
+                    help="accepted, no effect (one plain FP64 pair pass serves every size)")
     ap.add_argument("--sort-interval", type=int, default=None,
                     help="mixed: cycles between spatial sorts of the i-tiles (library default 4)")
     ap.add_argument("--drift-cycles", type=int, default=0,

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_keep_count(BodyArrays A, Dev
 
 /* The cycle's start of a collection of one scan tile's capacity: k_begin and
  * k_frag_count by one block.  Launches of a few microseconds each are most of
- * a small collection's cycle: with 8 launches in place of 45 the mixed cycle of
+ * a small collection's cycle: with 10 launches in place of 45 the mixed cycle of
  * 2,501 bodies takes 103 us in place of 161, with 6 in place of 14 the plain
  * cycle of 1,000 bodies 101 in place of 110. */
 __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_begin_small(BodyArrays A, DevCtl *ctl, SimSegs seg, int slots,
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_events_small(BodyArrays A, B
 }
 
 /* ------------------------------------------------------------------------ */
-/* K5: collision resolution, one thread, newest event first                 */
+/* K5: collision resolution, newest event first, a thread or a warp to one  */
 /* ------------------------------------------------------------------------ */
 
 struct ElasticOut {
@@ -1524,8 +1524,9 @@ __global__ void __launch_bounds__(NBG_SCAN_BLOCK) k_compact(BodyArrays A, BodyAr
  * (fragments, host adds) follow its kept bodies.  A sim's sorted positions
  * cover the same range as its indices, so the stable compaction over
  * positions uses the per-sim offsets of the body compaction.  Three steps:
- * kept positions per block, their block offsets (k_scan_blocks mode 2), and
- * the scatter into the scratch order; k_order_copy then installs it. */
+ * kept positions per block and, by the last block, their offsets
+ * (scan_blocks mode 2), the scatter into the scratch order, and its
+ * installation (order_copy). */
 __device__ static void order_blocksum(const DevCtl *ctl, const unsigned *perm, const unsigned *remap, ll blk,
                                       ll *blk_sum)
 {

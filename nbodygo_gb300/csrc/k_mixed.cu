@@ -936,7 +936,8 @@ k_pair_mixed(const __grid_constant__ BodyArrays A, DevCtl *ctl, SimSegs seg, con
 }
 
 /* f = (G m_i m_scale) * the sum of the chunks' shares of body p's i-tile,
- * written to body perm[p].  A CTA takes 32 bodies of one tile: the chunks
+ * and the heaviest body's pull (NBG_HEAVY_MAX_N), written to body perm[p].  A CTA
+ * takes 32 bodies of one tile: the chunks
  * that share the tile are cut into OUT_SLICES runs, one per row of 32
  * threads, each row adds its run in chunk order, and the rows' sums are added
  * in row order, so the result is the same on every run.  Small collections
@@ -1620,8 +1621,8 @@ __global__ void k_sym_out(BodyArrays A, DevCtl *ctl, SimSegs seg, const unsigned
  * two tile buffers filled from registers loaded a tile ahead; 3: sums in
  * shared memory and two tile buffers re-centred from raw tiles that bulk
  * copies bring into shared memory two tiles ahead.  Shapes 15 and 16 are
- * the symmetric kernel's.  Variant 0 is the default; the autotuner
- * (nbg_autotune) measures the others. */
+ * the symmetric kernel's.  nbg_default_shape chooses among 2, 6 and 15; the
+ * autotuner (nbg_autotune) measures them all. */
 #define MIX_VARIANTS(X)              \
     X(0, 0, 128, 4, 256, 2, 3)       \
     X(1, 0, 128, 4, 256, 1, 3)       \

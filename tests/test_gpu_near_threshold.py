@@ -8,6 +8,7 @@ from nbodygo_gb300 import workloads as W
 from nbodygo_gb300.api import Simulation
 
 from helpers import assert_events_identical, rel_l2
+from test_gpu_near_reach import crowded_disk
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +51,15 @@ def test_blocks_at_the_end_of_fp32s_range(shape, gap):
     _, want = run("fp64", b, shape)
     assert len(want) > 0
     assert_events_identical(ev, want)
+
+
+@pytest.mark.parametrize("shape", [0, 2])
+def test_large_bodies_without_thresholds_by_tile(shape):
+    """A capacity below the one from which k_mix_reach runs: every threshold
+    is against the largest radius of all."""
+    b = crowded_disk(16001)
+    f, ev = run("mixed", b, shape, 16384)
+    g, want = run("fp64", b, shape, 16384)
+    assert len(want) > 60
+    assert_events_identical(ev, want)
+    assert rel_l2(f[:, 1:], g[:, 1:]) <= 1e-6
