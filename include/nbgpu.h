@@ -422,8 +422,10 @@ int nbg_get_timing(nbg_ctx *ctx, nbg_timing *t);
    is left with no bodies (one empty collection, no staged adds); it stays
    usable, and the next load allocates again.  The hook clears itself. */
 #define NBG_OPT_TEST_FAIL_GROWTH 15
-/* test hook for the symmetric kernel's j partials: while 1, they do not
-   grow, as on a device without room for them; 0 (default) turns it off. */
+/* test hook for the mixed pair kernels' buffers: while bit 0 is set, the
+   symmetric kernel's j partials do not grow, and while bit 1 is, the partial
+   sums of a new kernel shape do not, as on a device without room for them; 0
+   (default) turns it off. */
 #define NBG_OPT_TEST_FAIL_JPART 16
 #define NBG_OPT_NEAR_PPM 5   /* mixed: pairs closer than (value * 1e-6) x the i-body's
                                 distance from its tile origin take the near-pair

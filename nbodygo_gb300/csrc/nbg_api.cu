@@ -95,6 +95,7 @@ struct nbg_ctx {
     int ev_radix_auto = 0; /* automatic choice for the next call */
     bool test_fail_growth = false; /* NBG_OPT_TEST_FAIL_GROWTH: the next growth fails */
     bool test_fail_jpart = false;  /* NBG_OPT_TEST_FAIL_JPART: the j partials do not grow */
+    bool test_fail_part = false;   /* likewise the partial sums */
     cudaEvent_t win[2] = {nullptr, nullptr}; /* the last two launches in flight */
 };
 
@@ -397,6 +398,7 @@ static int ensure_part(nbg_ctx *ctx, ll need)
     cudaFree(ctx->cb.part);
     ctx->cb.part = nullptr;
     ctx->cb.part_doubles = 0;
+    if (ctx->test_fail_part) return fail(ctx, NBG_E_CUDA, "partial sums: out of memory (test hook)");
     CK(cudaMalloc((void **)&ctx->cb.part, (size_t)need * sizeof(double)));
     ctx->cb.part_doubles = need;
     invalidate_graph(ctx);
@@ -1021,7 +1023,12 @@ int nbg_set_collections(nbg_ctx *ctx, int64_t nsims, const int64_t *counts, cons
     if (reshaped) invalidate_graph(ctx);
     if (!ctx->shape_given) {
         const int v = nbg_default_shape((int)nsims, (const ll *)counts, ctx->device_bytes);
-        if (v != ctx->cb.mix_variant && (rc = select_variant(ctx, v)) != NBG_OK) return rc;
+        if (v != ctx->cb.mix_variant && (rc = select_variant(ctx, v)) != NBG_OK) {
+            /* the arrays hold the new bodies, the control block the old count */
+            lose_bodies(ctx);
+            ctx->err += " (the context now holds no bodies)";
+            return rc;
+        }
         if (!nbg_mix_is_sym(v)) drop_jpart(ctx);
     }
     k_set_loaded<<<1, 1, 0, ctx->st>>>(ctx->ctl, n);
@@ -2160,8 +2167,9 @@ int nbg_set_option(nbg_ctx *ctx, int key, int64_t value)
         ctx->test_fail_growth = value != 0;
         return NBG_OK;
     case NBG_OPT_TEST_FAIL_JPART:
-        if (value < 0 || value > 1) return fail(ctx, NBG_E_ARG, "j-partial failure hook must be 0 or 1");
-        ctx->test_fail_jpart = value != 0;
+        if (value < 0 || value > 3) return fail(ctx, NBG_E_ARG, "j-partial failure hook must be 0..3");
+        ctx->test_fail_jpart = (value & 1) != 0;
+        ctx->test_fail_part = (value & 2) != 0;
         return NBG_OK;
     case NBG_OPT_STEP_DEADLINE_MS:
         if (value < 0 || value > ((ll)1 << 40)) return fail(ctx, NBG_E_ARG, "deadline must be 0..2^40 ms");

@@ -98,3 +98,24 @@ def test_a_restored_shape_is_kept_or_refused():
         s.set_option(A.OPT_TEST_FAIL_JPART, 1)
         s.set_bodies(b)
         assert s.step(1e-5, 1.0, 2)["steps_done"] == 2
+
+
+def test_a_load_whose_shape_has_no_room_leaves_an_empty_context():
+    """The default shape of the new collection needs larger partial sums: if
+    they do not fit, the load fails and no old count stands beside new bodies."""
+    small, large = W.uniform_ball(3000), W.uniform_ball(98304)
+    with Simulation("mixed", capacity=98305, seed=6) as s, Simulation("mixed", capacity=98305, seed=6) as t:
+        s.set_bodies(small)
+        s.step(1e-5, 1.0, 1)
+        s.set_option(A.OPT_TEST_FAIL_JPART, 2)
+        with pytest.raises(NbgError):
+            s.set_bodies(large)
+        assert s.count() == 0 and len(s.state()["x"]) == 0
+        s.set_option(A.OPT_TEST_FAIL_JPART, 0)
+        assert s.step(1e-5, 1.0, 2)["n_bodies"] == 0
+        for c in (s, t):
+            c.set_bodies(large)
+            c.step(1e-5, 1.0, 2)
+        got, want = s.state(), t.state()
+        for f in ("x", "vx", "fy"):
+            assert np.array_equal(got[f], want[f]), f
